@@ -369,8 +369,31 @@ __global__ void reduce_partials_kernel(const double *__restrict__ partials, int 
     }
 }
 
+// The same for a few outputs of many rows: a CTA per output.
+__global__ void __launch_bounds__(256) reduce_rows_kernel(const double *__restrict__ partials, int nblocks, int m,
+                                                          double *__restrict__ out)
+{
+    __shared__ double red[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += 256) s += partials[(int64_t)b * m + blockIdx.x];
+    s = warp_sum(s);
+    if (lane == 0) red[warp] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0.0;
+        for (int q = 0; q < 8; ++q) s += red[q];
+        out[blockIdx.x] = s;
+    }
+}
+
 int launch_reduce(const double *partials, int nblocks, int m, double *out, cudaStream_t st)
 {
+    if (m <= 8 && nblocks > 64) {
+        reduce_rows_kernel<<<m, 256, 0, st>>>(partials, nblocks, m, out);
+        ED_CHECK_LAUNCH();
+        return ED_OK;
+    }
     int threads = 256, per = threads / 32;
     int blocks = (m + per - 1) / per;
     if (blocks > 1024) blocks = 1024;

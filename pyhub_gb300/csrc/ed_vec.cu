@@ -11,6 +11,8 @@
 // products in FP32 before the FP64 stage; see multidot_kernel.)
 #include "ed_common.cuh"
 
+#include <algorithm>
+
 namespace ed {
 
 int launch_reduce(const double *partials, int nblocks, int m, double *out, cudaStream_t st);
@@ -19,94 +21,181 @@ static constexpr int kVecThreads = 256;
 static constexpr int kEPT = 16;                      // elements per thread per chunk
 static constexpr int kChunk = kVecThreads * kEPT;    // 4096 elements
 static constexpr int kMaxBlocks = 1024;
+static constexpr int kMaxNormRows = 2 * kMaxBlocks;  // partial norms that the smallest scratch holds
+static constexpr int kVecResident = 4;               // CTAs per SM that a vector pass aims at
 
+// Four consecutive elements p[i..i+3] (zeros past n); p is 16-byte aligned and i a multiple of 4.
 template <typename T>
-__device__ __forceinline__ void load_chunk(T (&r)[kEPT], const T *__restrict__ p, int64_t base, int64_t n)
+__device__ __forceinline__ void load4(T *r, const T *__restrict__ p, int64_t i, int64_t n)
 {
-    // thread t owns elements base + t*4 + k*1024 + j (j<4), k < kEPT/4: float4 / double2x2 friendly
-#pragma unroll
-    for (int k = 0; k < kEPT / 4; ++k) {
-        const int64_t i = base + (int64_t)k * (kVecThreads * 4) + threadIdx.x * 4;
-        if (i + 3 < n) {
-            if constexpr (sizeof(T) == 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(p + i));
-                r[4 * k] = v.x; r[4 * k + 1] = v.y; r[4 * k + 2] = v.z; r[4 * k + 3] = v.w;
-            } else {
-                const double2 v0 = __ldg(reinterpret_cast<const double2 *>(p + i));
-                const double2 v1 = __ldg(reinterpret_cast<const double2 *>(p + i + 2));
-                r[4 * k] = v0.x; r[4 * k + 1] = v0.y; r[4 * k + 2] = v1.x; r[4 * k + 3] = v1.y;
-            }
+    if (i + 3 < n) {
+        if constexpr (sizeof(T) == 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(p + i));
+            r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
         } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) r[4 * k + j] = (i + j < n) ? __ldg(p + i + j) : (T)0;
+            const double2 v0 = __ldg(reinterpret_cast<const double2 *>(p + i));
+            const double2 v1 = __ldg(reinterpret_cast<const double2 *>(p + i + 2));
+            r[0] = v0.x; r[1] = v0.y; r[2] = v1.x; r[3] = v1.y;
         }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = (i + j < n) ? __ldg(p + i + j) : (T)0;
     }
 }
 
-// partials[block][j] (j < nvec) = sum over the block's chunks of <V_j, w>,
+// EPT elements of a thread: base + t*4 + k*4*NT + j (j < 4), k < EPT/4, in a CTA of NT threads.
+template <typename T, int EPT, int NT>
+__device__ __forceinline__ void load_chunk(T (&r)[EPT], const T *__restrict__ p, int64_t base, int64_t n)
+{
+#pragma unroll
+    for (int k = 0; k < EPT / 4; ++k) load4<T>(r + 4 * k, p, base + (int64_t)k * (NT * 4) + threadIdx.x * 4, n);
+}
+
+// FP32: partials[block][j] (j < nvec) = sum over the block's chunks of <V_j, w>,
 // partials[block][nvec + j] the same with z (when z != NULL).
-// FP32 vectors: each warp forms its 512 products per chunk and reduces them in
+// Each warp forms its 512 products per chunk and reduces them in
 // FP32 (shuffles); only that warp partial is promoted and added in FP64, so
 // the FP64 work is one add per 512 elements and vector.  For random-sign
 // data the FP32 stage contributes an absolute error ~eps32 |V_j||w|/sqrt(n).
-template <typename T>
-__global__ void __launch_bounds__(kVecThreads) multidot_kernel(int64_t n, const T *__restrict__ V, int64_t ldv,
-                                                               int nvec, const T *__restrict__ w,
-                                                               const T *__restrict__ z,
-                                                               double *__restrict__ partials)
+// Bound by HBM once the chunks fill the chip.  A vector shorter than that (fewer chunks than
+// kVecResident CTAs per SM) splits the basis over blockIdx.y, jper vectors each, so that its pass
+// is a few vectors deep instead of all of them (100 vectors of 63,488: 72 -> 19 us; of 853,872:
+// 117 -> 74 us; 11.8 M and more: unchanged, 6.6-6.9 TB/s).
+__global__ void __launch_bounds__(kVecThreads, kVecResident) multidot32_kernel(int64_t n, const float *__restrict__ V, int64_t ldv,
+                                                                 int nvec, int jper, const float *__restrict__ w,
+                                                                 const float *__restrict__ z,
+                                                                 double *__restrict__ partials)
 {
-    extern __shared__ double acc[];  // [8 warps][m]
-    const int m = z ? 2 * nvec : nvec;
+    extern __shared__ double acc[];  // [8 warps][mj]
+    const int j0 = blockIdx.y * jper, nj = min(jper, nvec - j0);
+    const int m = z ? 2 * nvec : nvec, mj = z ? 2 * nj : nj;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int j = threadIdx.x; j < 8 * m; j += blockDim.x) acc[j] = 0.0;
+    for (int j = threadIdx.x; j < 8 * mj; j += blockDim.x) acc[j] = 0.0;
     __syncthreads();
     const int64_t nchunks = (n + kChunk - 1) / kChunk;
     for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         const int64_t base = ch * kChunk;
-        T rw[kEPT], rz[kEPT];
-        load_chunk<T>(rw, w, base, n);
-        if (z) load_chunk<T>(rz, z, base, n);
+        float rw[kEPT], rz[kEPT];
+        load_chunk<float, kEPT, kVecThreads>(rw, w, base, n);
+        if (z) load_chunk<float, kEPT, kVecThreads>(rz, z, base, n);
 #pragma unroll 2
-        for (int j = 0; j < nvec; ++j) {
-            T rv[kEPT];
-            load_chunk<T>(rv, V + (int64_t)j * ldv, base, n);
-            T pw = 0, pz = 0;
+        for (int j = 0; j < nj; ++j) {
+            float rv[kEPT];
+            load_chunk<float, kEPT, kVecThreads>(rv, V + (int64_t)(j0 + j) * ldv, base, n);
+            float pw = 0, pz = 0;
 #pragma unroll
             for (int k = 0; k < kEPT; ++k) pw += rv[k] * rw[k];
             if (z) {
 #pragma unroll
                 for (int k = 0; k < kEPT; ++k) pz += rv[k] * rz[k];
             }
-            if constexpr (sizeof(T) == 4) {
-                pw = warp_sumf(pw);
-                if (z) pz = warp_sumf(pz);
-                if (lane == 0) {
-                    acc[warp * m + j] += (double)pw;
-                    if (z) acc[warp * m + nvec + j] += (double)pz;
-                }
-            } else {
-                const double sw = warp_sum((double)pw);
-                const double sz = z ? warp_sum((double)pz) : 0.0;
-                if (lane == 0) {
-                    acc[warp * m + j] += sw;
-                    if (z) acc[warp * m + nvec + j] += sz;
-                }
+            pw = warp_sumf(pw);
+            if (z) pz = warp_sumf(pz);
+            if (lane == 0) {
+                acc[warp * mj + j] += (double)pw;
+                if (z) acc[warp * mj + nj + j] += (double)pz;
             }
         }
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+    for (int j = threadIdx.x; j < mj; j += blockDim.x) {
         double s = 0.0;
-        for (int q = 0; q < 8; ++q) s += acc[q * m + j];
-        partials[(int64_t)blockIdx.x * m + j] = s;
+        for (int q = 0; q < 8; ++q) s += acc[q * mj + j];
+        partials[(int64_t)blockIdx.x * m + (j < nj ? j0 + j : nvec + j0 + j - nj)] = s;
+    }
+}
+
+// FP64, same partials.  An FP64 instruction costs 64 FP32 ones on this chip, so the pass is bound by
+// the FP64 pipe (two FMA per basis element) and spends it on nothing else: a CTA owns kJ64 vectors
+// and one range of elements, every thread keeps its 2*kJ64 sums in registers over the whole range,
+// and lanes are summed once at its end (the pass that summed lanes after every 16 elements took 11
+// FP64 instructions per 8 here).  w and z are read again for every kJ64 vectors, from L2.
+static constexpr int kJ64 = 8;
+static constexpr int kStep64 = kVecThreads * 2;   // elements of one iteration: a 16-byte load per thread
+
+__device__ __forceinline__ double2 load2(const double *__restrict__ p, int64_t i, int64_t n)
+{
+    if (i + 1 < n) return __ldg(reinterpret_cast<const double2 *>(p + i));
+    return make_double2(i < n ? __ldg(p + i) : 0.0, 0.0);
+}
+
+// Sums of N values over the 32 lanes (N a power of two <= 32): each exchange halves the values a
+// lane holds, so N sums cost about N additions instead of 5 N.  Value q ends in v[0] of lane
+// q * (32 / N) (and its copies).
+template <int N>
+__device__ __forceinline__ void warp_sum_many(double (&v)[N])
+{
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool hi = (lane & o) != 0;
+#pragma unroll
+        for (int q = 0; q < N / 2; ++q) {
+            if (q >= h) break;
+            const double mine = hi ? v[q + h] : v[q], other = hi ? v[q] : v[q + h];
+            v[q] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+        }
+    }
+    for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+}
+
+template <bool Z>
+__global__ void __launch_bounds__(kVecThreads, 2) multidot64_kernel(int64_t n, const double *__restrict__ V,
+                                                                    int64_t ldv, int nvec,
+                                                                    const double *__restrict__ w,
+                                                                    const double *__restrict__ z,
+                                                                    double *__restrict__ partials)
+{
+    constexpr int NS = Z ? 2 * kJ64 : kJ64;
+    __shared__ double red[kVecThreads / 32][NS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ng = gridDim.y;
+    const int j0 = (int)((int64_t)nvec * blockIdx.y / ng), nj = (int)((int64_t)nvec * (blockIdx.y + 1) / ng) - j0;
+    const int64_t steps = (n + kStep64 - 1) / kStep64;
+    const int64_t s0 = steps * blockIdx.x / gridDim.x, s1 = steps * (blockIdx.x + 1) / gridDim.x;
+    double acc[NS];
+#pragma unroll
+    for (int q = 0; q < NS; ++q) acc[q] = 0.0;
+    const double *Vj = V + (int64_t)j0 * ldv;
+    for (int64_t st = s0; st < s1; ++st) {
+        const int64_t i = st * kStep64 + threadIdx.x * 2;
+        double2 v[kJ64];
+#pragma unroll
+        for (int j = 0; j < kJ64; ++j)
+            if (j < nj) v[j] = load2(Vj + (int64_t)j * ldv, i, n);
+        const double2 a = load2(w, i, n);
+        double2 b;
+        if constexpr (Z) b = load2(z, i, n);
+#pragma unroll
+        for (int j = 0; j < kJ64; ++j) {
+            if (j >= nj) break;
+            acc[j] = fma(v[j].x, a.x, acc[j]);
+            if constexpr (Z) acc[kJ64 + j] = fma(v[j].x, b.x, acc[kJ64 + j]);
+            acc[j] = fma(v[j].y, a.y, acc[j]);
+            if constexpr (Z) acc[kJ64 + j] = fma(v[j].y, b.y, acc[kJ64 + j]);
+        }
+    }
+    warp_sum_many<NS>(acc);
+    if (lane % (32 / NS) == 0) red[warp][lane / (32 / NS)] = acc[0];
+    __syncthreads();
+    const int q = threadIdx.x, j = q % kJ64;
+    if (q < NS && j < nj) {
+        double s = 0.0;
+        for (int k = 0; k < kVecThreads / 32; ++k) s += red[k][q];
+        partials[(int64_t)blockIdx.x * (Z ? 2 * nvec : nvec) + (q < kJ64 ? 0 : nvec) + j0 + j] = s;
     }
 }
 
 // out = ws w - sum_j coef_j V_j (w may be NULL; ws = wscale[0], a device
 // scalar, or 1 when wscale is NULL), optional partial <out,out>.
 // Accumulation type A: FP32 for an FP32 basis with FP32 output, FP64 otherwise.
-template <typename T, typename O, typename A>
-__global__ void __launch_bounds__(kVecThreads) update_kernel(int64_t n, const T *__restrict__ V, int64_t ldv,
+// EPT elements per thread, NT threads: 16 x 256 streams long vectors at the HBM rate (FP64: the FP64
+// pipe's), 4 x 128 spreads shorter ones evenly over the SMs (FP64, 50 vectors of 853,872: 125 ->
+// 97 us; from about 2.5 M elements on the 16-element form is as fast or faster: FP32, 4 M: 131 us
+// against 146).
+template <typename T, typename O, typename A, int EPT, int NT>
+__global__ void __launch_bounds__(NT) update_kernel(int64_t n, const T *__restrict__ V, int64_t ldv,
                                                              int nvec, const double *__restrict__ coef,
                                                              const double *__restrict__ wscale, const O *w, O *out,
                                                              double *__restrict__ partials)
@@ -118,32 +207,39 @@ __global__ void __launch_bounds__(kVecThreads) update_kernel(int64_t n, const T 
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double nrm = 0.0;
-    const int64_t nchunks = (n + kChunk - 1) / kChunk;
+    constexpr int64_t chunk = (int64_t)NT * EPT;
+    const int64_t nchunks = (n + chunk - 1) / chunk;
     for (int64_t ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-        const int64_t base = ch * kChunk;
-        A r[kEPT];
+        const int64_t base = ch * chunk;
+        A r[EPT];
         if (w) {
-            O rw[kEPT];
-            load_chunk<O>(rw, w, base, n);
+            O rw[EPT];
+            load_chunk<O, EPT, NT>(rw, w, base, n);
 #pragma unroll
-            for (int k = 0; k < kEPT; ++k) r[k] = ws * (A)rw[k];
+            for (int k = 0; k < EPT; ++k) r[k] = ws * (A)rw[k];
         } else {
 #pragma unroll
-            for (int k = 0; k < kEPT; ++k) r[k] = (A)0;
+            for (int k = 0; k < EPT; ++k) r[k] = (A)0;
         }
-        for (int j = 0; j < nvec; ++j) {
-            T rv[kEPT];
-            load_chunk<T>(rv, V + (int64_t)j * ldv, base, n);
+        auto subtract = [&](int j) {
+            T rv[EPT];
+            load_chunk<T, EPT, NT>(rv, V + (int64_t)j * ldv, base, n);
             const A c = cs[j];
 #pragma unroll
-            for (int k = 0; k < kEPT; ++k) r[k] -= c * (A)rv[k];
+            for (int k = 0; k < EPT; ++k) r[k] -= c * (A)rv[k];
+        };
+        if constexpr (EPT == 4) {
+#pragma unroll 4
+            for (int j = 0; j < nvec; ++j) subtract(j);
+        } else {
+            for (int j = 0; j < nvec; ++j) subtract(j);
         }
-        O ro[kEPT];
+        O ro[EPT];
 #pragma unroll
-        for (int k = 0; k < kEPT; ++k) ro[k] = (O)r[k];
+        for (int k = 0; k < EPT; ++k) ro[k] = (O)r[k];
 #pragma unroll
-        for (int k = 0; k < kEPT / 4; ++k) {
-            const int64_t i = base + (int64_t)k * (kVecThreads * 4) + threadIdx.x * 4;
+        for (int k = 0; k < EPT / 4; ++k) {
+            const int64_t i = base + (int64_t)k * (NT * 4) + threadIdx.x * 4;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 if (i + j < n) out[i + j] = ro[4 * k + j];
@@ -152,16 +248,70 @@ __global__ void __launch_bounds__(kVecThreads) update_kernel(int64_t n, const T 
             if constexpr (sizeof(O) == 4) {
                 float p = 0.f;
 #pragma unroll
-                for (int k = 0; k < kEPT; ++k) p += ro[k] * ro[k];
+                for (int k = 0; k < EPT; ++k) p += ro[k] * ro[k];
                 nrm += (double)p;
             } else {
 #pragma unroll
-                for (int k = 0; k < kEPT; ++k) nrm += (double)ro[k] * (double)ro[k];
+                for (int k = 0; k < EPT; ++k) nrm += (double)ro[k] * (double)ro[k];
             }
         }
     }
     if (partials) {
-        __shared__ double red[8];
+        __shared__ double red[NT / 32];
+        nrm = warp_sum(nrm);
+        if (lane == 0) red[warp] = nrm;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double s = 0.0;
+            for (int q = 0; q < NT / 32; ++q) s += red[q];
+            partials[blockIdx.x] = s;
+        }
+    }
+}
+
+// The same for short vectors, where the chain of nvec loads is the time: a CTA's eight warps take
+// every eighth vector of one 128-element tile each, and their sums meet in shared memory
+// (FP64, 50 vectors of 4,928: 65 -> 14 us; of 63,488: 61 -> 18 us, most of it the two launches).
+static constexpr int kSplitTile = 128;
+
+template <typename T, typename O, typename A>
+__global__ void __launch_bounds__(kVecThreads) update_split_kernel(int64_t n, const T *__restrict__ V, int64_t ldv,
+                                                                   int nvec, const double *__restrict__ coef,
+                                                                   const double *__restrict__ wscale, const O *w,
+                                                                   O *out, double *__restrict__ partials)
+{
+    __shared__ __align__(16) A sums[8][kSplitTile];
+    __shared__ double red[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const A ws = wscale ? (A)wscale[0] : (A)1;
+    const int64_t ntiles = (n + kSplitTile - 1) / kSplitTile;
+    double nrm = 0.0;
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int64_t i = tile * kSplitTile + lane * 4;
+        A r[4] = {0, 0, 0, 0};
+#pragma unroll 4
+        for (int j = warp; j < nvec; j += 8) {
+            T rv[4];
+            load4<T>(rv, V + (int64_t)j * ldv, i, n);
+            const A c = (A)__ldg(coef + j);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[k] += c * (A)rv[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sums[warp][lane * 4 + k] = r[k];
+        __syncthreads();
+        const int64_t e = tile * kSplitTile + threadIdx.x;
+        if (threadIdx.x < kSplitTile && e < n) {
+            A s = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) s += sums[q][threadIdx.x];
+            const O o = (O)((w ? ws * (A)w[e] : (A)0) - s);
+            out[e] = o;
+            nrm += (double)o * (double)o;
+        }
+        __syncthreads();
+    }
+    if (partials) {
         nrm = warp_sum(nrm);
         if (lane == 0) red[warp] = nrm;
         __syncthreads();
@@ -173,13 +323,69 @@ __global__ void __launch_bounds__(kVecThreads) update_kernel(int64_t n, const T 
     }
 }
 
-static int grid_for(int64_t n)
+static int64_t vec_ctas() { return std::min<int64_t>((int64_t)num_sms() * kVecResident, kMaxBlocks); }
+
+// Partial rows of the multi-dot's grid (z or not) in *rows; the partials hold rows * m doubles.
+static int launch_multidot(cudaStream_t st, int dtype, int64_t n, const void *V, int64_t ldv, int nvec, const void *w,
+                           const void *z, double *part, int *rows)
 {
-    int64_t nchunks = (n + kChunk - 1) / kChunk;
-    int64_t cap = (int64_t)num_sms() * 4;
-    if (cap > kMaxBlocks) cap = kMaxBlocks;
-    if (nchunks < cap) cap = nchunks;
-    return (int)(cap < 1 ? 1 : cap);
+    const int64_t ctas = vec_ctas();
+    if (dtype == ED_F32) {
+        const int64_t nchunks = (n + kChunk - 1) / kChunk;
+        const int gx = (int)std::max<int64_t>(1, std::min(nchunks, ctas));
+        // one pass over all vectors once the chunks alone fill the chip (w and z are read once);
+        // below that, groups of at least 4 vectors per CTA row
+        int ng = (int)std::min<int64_t>((nvec + 3) / 4, std::max<int64_t>(1, ctas / gx));
+        const int jper = (nvec + ng - 1) / ng;
+        ng = (nvec + jper - 1) / jper;
+        const size_t smem = sizeof(double) * 8 * (size_t)jper * (z ? 2 : 1);
+        if (smem > 48 * 1024)
+            ED_CHECK_CUDA(cudaFuncSetAttribute(multidot32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem));
+        multidot32_kernel<<<dim3((unsigned)gx, (unsigned)ng), kVecThreads, smem, st>>>(
+            n, static_cast<const float *>(V), ldv, nvec, jper, static_cast<const float *>(w),
+            static_cast<const float *>(z), part);
+        *rows = gx;
+    } else {
+        const int64_t steps = (n + kStep64 - 1) / kStep64;
+        // groups of 5 to kJ64 vectors, as even as they come: the CTAs with the largest group end the pass
+        int ng = (nvec + kJ64 - 1) / kJ64;
+        for (int g = ng + 1; g <= (nvec + 4) / 5; ++g)
+            if ((int64_t)((nvec + g - 1) / g) * g < (int64_t)((nvec + ng - 1) / ng) * ng) ng = g;
+        const int gx = (int)std::max<int64_t>(1, std::min(steps, ctas / ng));   // whole waves: one CTA more costs a wave
+        const dim3 grid((unsigned)gx, (unsigned)ng);
+        const double *Vd = static_cast<const double *>(V), *wd = static_cast<const double *>(w),
+                     *zd = static_cast<const double *>(z);
+        if (z) multidot64_kernel<true><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
+        else multidot64_kernel<false><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
+        *rows = gx;
+    }
+    ED_CHECK_LAUNCH();
+    return ED_OK;
+}
+
+template <typename T, typename O, typename A>
+static int launch_update(cudaStream_t st, int64_t n, const T *V, int64_t ldv, int nvec, const double *coef,
+                         const double *wscale, const O *w, O *out, double *part, int *rows)
+{
+    const int64_t ctas = vec_ctas();
+    const size_t smem = sizeof(double) * (size_t)(nvec > 0 ? nvec : 1);
+    const int64_t tiles = (n + kSplitTile - 1) / kSplitTile;
+    // up to four tiles per CTA of the split form; then 4 elements per thread until the 16-element
+    // chunks fill every resident CTA
+    if (tiles <= 4 * ctas) {
+        *rows = (int)std::min(tiles, ctas);
+        update_split_kernel<T, O, A><<<*rows, kVecThreads, 0, st>>>(n, V, ldv, nvec, coef, wscale, w, out, part);
+    } else if ((n + kChunk - 1) / kChunk < ctas) {
+        *rows = (int)std::min<int64_t>((n + 511) / 512, kMaxNormRows);
+        update_kernel<T, O, A, 4, 128><<<*rows, 128, smem, st>>>(n, V, ldv, nvec, coef, wscale, w, out, part);
+    } else {
+        *rows = (int)std::min<int64_t>((n + kChunk - 1) / kChunk, ctas);
+        update_kernel<T, O, A, kEPT, kVecThreads><<<*rows, kVecThreads, smem, st>>>(n, V, ldv, nvec, coef, wscale, w,
+                                                                                    out, part);
+    }
+    ED_CHECK_LAUNCH();
+    return ED_OK;
 }
 
 }  // namespace ed
@@ -210,21 +416,11 @@ extern "C" int ed_multidot(void *stream, int dtype, int64_t n, const void *V, in
     const size_t smem = sizeof(double) * 8 * (size_t)m;
     ED_REQUIRE(smem <= 200 * 1024, "nvec=%d too large for one pass", nvec);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int grid = grid_for(n);
     double *part = static_cast<double *>(scratch);
-    if (dtype == ED_F32) {
-        ED_CHECK_CUDA(cudaFuncSetAttribute(multidot_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        multidot_kernel<float><<<grid, kVecThreads, smem, st>>>(n, static_cast<const float *>(V), ldv, nvec,
-                                                               static_cast<const float *>(w),
-                                                               static_cast<const float *>(z), part);
-    } else {
-        ED_CHECK_CUDA(cudaFuncSetAttribute(multidot_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        multidot_kernel<double><<<grid, kVecThreads, smem, st>>>(n, static_cast<const double *>(V), ldv, nvec,
-                                                                static_cast<const double *>(w),
-                                                                static_cast<const double *>(z), part);
-    }
-    ED_CHECK_LAUNCH();
-    return launch_reduce(part, grid, m, out, st);
+    int rows = 0;
+    const int rc = launch_multidot(st, dtype, n, V, ldv, nvec, w, z, part, &rows);
+    if (rc) return rc;
+    return launch_reduce(part, rows, m, out, st);
 }
 
 extern "C" int ed_update_wscaled(void *stream, int dtype, int out_dtype, int64_t n, const void *V, int64_t ldv,
@@ -251,28 +447,25 @@ extern "C" int ed_update_wscaled(void *stream, int dtype, int out_dtype, int64_t
     }
     if (n == 0) return ED_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int grid = grid_for(n);
     double *part = norm2 ? static_cast<double *>(scratch) : nullptr;
-    const size_t smem = sizeof(double) * (size_t)(nvec > 0 ? nvec : 1);
-    if (dtype == ED_F32 && out_dtype == ED_F32) {
-        update_kernel<float, float, float><<<grid, kVecThreads, smem, st>>>(
-            n, static_cast<const float *>(V), ldv, nvec, coef, wscale, static_cast<const float *>(w),
-            static_cast<float *>(out), part);
-    } else if (dtype == ED_F32 && out_dtype == ED_F64) {
-        update_kernel<float, double, double><<<grid, kVecThreads, smem, st>>>(
-            n, static_cast<const float *>(V), ldv, nvec, coef, wscale, static_cast<const double *>(w),
-            static_cast<double *>(out), part);
-    } else if (dtype == ED_F64 && out_dtype == ED_F64) {
-        update_kernel<double, double, double><<<grid, kVecThreads, smem, st>>>(
-            n, static_cast<const double *>(V), ldv, nvec, coef, wscale, static_cast<const double *>(w),
-            static_cast<double *>(out), part);
-    } else {
-        update_kernel<double, float, double><<<grid, kVecThreads, smem, st>>>(
-            n, static_cast<const double *>(V), ldv, nvec, coef, wscale, static_cast<const float *>(w),
-            static_cast<float *>(out), part);
-    }
-    ED_CHECK_LAUNCH();
-    if (norm2) return launch_reduce(part, grid, 1, norm2, st);
+    int rows = 0, rc;
+    if (dtype == ED_F32 && out_dtype == ED_F32)
+        rc = launch_update<float, float, float>(st, n, static_cast<const float *>(V), ldv, nvec, coef, wscale,
+                                                static_cast<const float *>(w), static_cast<float *>(out), part, &rows);
+    else if (dtype == ED_F32 && out_dtype == ED_F64)
+        rc = launch_update<float, double, double>(st, n, static_cast<const float *>(V), ldv, nvec, coef, wscale,
+                                                  static_cast<const double *>(w), static_cast<double *>(out), part,
+                                                  &rows);
+    else if (dtype == ED_F64 && out_dtype == ED_F64)
+        rc = launch_update<double, double, double>(st, n, static_cast<const double *>(V), ldv, nvec, coef, wscale,
+                                                   static_cast<const double *>(w), static_cast<double *>(out), part,
+                                                   &rows);
+    else
+        rc = launch_update<double, float, double>(st, n, static_cast<const double *>(V), ldv, nvec, coef, wscale,
+                                                  static_cast<const float *>(w), static_cast<float *>(out), part,
+                                                  &rows);
+    if (rc) return rc;
+    if (norm2) return launch_reduce(part, rows, 1, norm2, st);
     return ED_OK;
 }
 
@@ -367,24 +560,14 @@ extern "C" int ed_multidot_noalloc(void *stream, int dtype, int64_t n, const voi
                    (!z || (reinterpret_cast<uintptr_t>(z) % 16) == 0) && ((ldv * esz) % 16) == 0,
                "V, w, z and the vector stride must be 16-byte aligned");
     const int m = z ? 2 * nvec : nvec;
-    const int grid = grid_for(n);
-    if ((int64_t)grid * m > kNoAllocDoubles) {
-        set_error("%d blocks x %d sums exceed the fixed scratch of %lld doubles", grid, m, (long long)kNoAllocDoubles);
-        return ED_ERR_RANGE;
-    }
+    // a grid has at most kMaxBlocks partial rows
+    static_assert((int64_t)kMaxBlocks * 2 * kNoAllocMaxNvec <= kNoAllocDoubles, "partials exceed the fixed scratch");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     double *part = nullptr;
-    const int rc = noalloc_partials(st, &part);
+    int rc = noalloc_partials(st, &part);
     if (rc) return rc;
-    const size_t smem = sizeof(double) * 8 * (size_t)m;  // at most 8 KiB: no opt-in needed
-    if (dtype == ED_F32)
-        multidot_kernel<float><<<grid, kVecThreads, smem, st>>>(n, static_cast<const float *>(V), ldv, nvec,
-                                                               static_cast<const float *>(w),
-                                                               static_cast<const float *>(z), part);
-    else
-        multidot_kernel<double><<<grid, kVecThreads, smem, st>>>(n, static_cast<const double *>(V), ldv, nvec,
-                                                                static_cast<const double *>(w),
-                                                                static_cast<const double *>(z), part);
-    ED_CHECK_LAUNCH();
-    return launch_reduce(part, grid, m, out, st);
+    int rows = 0;
+    rc = launch_multidot(st, dtype, n, V, ldv, nvec, w, z, part, &rows);
+    if (rc) return rc;
+    return launch_reduce(part, rows, m, out, st);
 }
