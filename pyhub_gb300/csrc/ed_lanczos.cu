@@ -19,54 +19,27 @@
 // explicit inverse is as accurate as the triangular solves it replaces.
 #include "ed_common.cuh"
 
+#include <cooperative_groups.h>
+
 namespace ed {
 
-constexpr int kCoefThreads = 512;
-constexpr int kLanczosMax = 8192;   // largest step count a state can hold
+namespace cg = cooperative_groups;
+
+constexpr int kCoefThreads = 256;
+constexpr int kCoefCtas = 8;         // one thread-block cluster
+constexpr int kLanczosMax = 8192;    // largest step count a state can hold
 
 // State layout (FP64): [0] stop code, [1] largest |G - I| entry seen,
 // [2 .. 2+mmax] scales s_j, then Linv as (mmax+1) x (mmax+1) row-major, then
-// four work vectors of mmax+1 entries (Gram row, projections, Linv g, Linv c).
+// four spare vectors of mmax+1 entries.
 __host__ __device__ inline int64_t lz_linv_off(int mmax) { return 3 + (int64_t)mmax; }
 __host__ __device__ inline int64_t lz_work_off(int mmax) { return lz_linv_off(mmax) + (int64_t)(mmax + 1) * (mmax + 1); }
 
-__device__ __forceinline__ double block_sum_d(double v, double *red)
-{
-    v = warp_sum(v);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x < 32) {
-        t = (lane < (int)(blockDim.x >> 5)) ? red[lane] : 0.0;
-        t = warp_sum(t);
-        if (lane == 0) red[0] = t;
-    }
-    __syncthreads();
-    t = red[0];
-    __syncthreads();
-    return t;
-}
+// Rows of Linv that a CTA of the cluster owns, i = kCoefCtas p + rank: p below this (32 rows at a time).
+__host__ __device__ inline int coef_rows(int k) { return (k + 32 * kCoefCtas - 1) / (32 * kCoefCtas) * 32; }
+__host__ __device__ inline size_t coef_smem(int k) { return sizeof(double) * (2 * (size_t)(k + 1) + 2 * (size_t)coef_rows(k)); }
 
-__device__ __forceinline__ double block_max_d(double v, double *red)
-{
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x < 32) {
-        t = (lane < (int)(blockDim.x >> 5)) ? red[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) t = fmax(t, __shfl_xor_sync(0xffffffffu, t, o));
-        if (lane == 0) red[0] = t;
-    }
-    __syncthreads();
-    t = red[0];
-    __syncthreads();
-    return t;
-}
-
-// One CTA.  Part 1 (every call, k >= 1): beta_{k-1} and s_k from nrm, with
+// One cluster of kCoefCtas CTAs.  Part 1 (every call, k >= 1): beta_{k-1} and s_k from nrm, with
 // the breakdown test of the host loop (beta <= 1e-13 max(1, |alpha|)).
 // Part 1 is idempotent: a second call for the same k with the same nrm writes
 // the same beta_{k-1} and s_k.  The host's look-ahead relies on it (a run that
@@ -76,109 +49,172 @@ __device__ __forceinline__ double block_max_d(double v, double *red)
 // when u_k is numerically dependent on the basis.  Once stopped, coef is
 // written as zeros (and s stays 0), so the vectors that follow are zero and
 // finite until the host sees the stop code.
-__global__ void __launch_bounds__(kCoefThreads) lanczos_coef_kernel(int k, int mmax, const double *__restrict__ dots,
-                                                                    const double *__restrict__ nrm,
-                                                                    double *__restrict__ state,
-                                                                    double *__restrict__ coef,
-                                                                    double *__restrict__ alpha,
-                                                                    double *__restrict__ beta)
+//
+// What bounds it: latency.  A dependent FP64 operation takes tens of clocks here, a square root or a
+// quotient hundreds, and one SM does 2 FP64 multiply-adds per clock (k^2 / 2 per product with Linv).
+// Linv is therefore read twice instead of four times (g and c go through the row pass together, l
+// and z through the column pass: the new row's product with c is (c_k - l.z) / lam), its rows are
+// dealt over the CTAs of a cluster, whose sums meet once in distributed shared memory, and the
+// chain holds no sum over a whole CTA and no quotient.  One CTA with four passes took 12.2,
+// 19.2, 33.6 and 72.4 us at k = 10, 40, 100 and 200 (launch included); this form 7.9, 9.2, 10.8 and 13.9.
+__global__ void __cluster_dims__(kCoefCtas, 1, 1) __launch_bounds__(kCoefThreads)
+    lanczos_coef_kernel(int k, int mmax, const double *__restrict__ dots, const double *__restrict__ nrm, double *state,
+                        double *__restrict__ coef, double *__restrict__ alpha, double *__restrict__ beta)
 {
-    __shared__ double red[32];
-    __shared__ int stop;
+    extern __shared__ double dyn[];
+    __shared__ double head[2];                       // s_k, stop code
+    __shared__ double part[2][kCoefThreads / 32];    // per warp: l.l and l.z over the CTA's rows
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), t = threadIdx.x, lane = t & 31;
     double *s = state + 2;
-    double *Linv = state + lz_linv_off(mmax);
-    const int64_t ldl = mmax + 1;
-    double *g = state + lz_work_off(mmax);   // [k+1] Gram row
-    double *c = g + ldl;                     // [k+1] projections
-    double *l = c + ldl;                     // [k]   Linv g
-    double *z = l + ldl;                     // [k+1] Linv c
-    if (threadIdx.x == 0) {
-        if (k >= 1 && state[0] == 0.0) {
-            const double nb = nrm[0];
-            const double bk = sqrt(fmax(nb, 0.0));
+    if (dots == nullptr && rank != 0) return;
+    if (t == 0) {
+        double stop = state[0], sk = s[k];
+        if (k >= 1 && stop == 0.0) {
+            const double nb = nrm[0], pos = fmax(nb, 0.0);
+            const double bk = sqrt(pos);
             if (!isfinite(nb)) {
-                state[0] = -(double)k;
-                s[k] = 0.0;
+                stop = -(double)k;
+                sk = 0.0;
             } else {
-                beta[k - 1] = bk;
+                if (rank == 0) beta[k - 1] = bk;
                 if (bk <= 1e-13 * fmax(1.0, fabs(alpha[k - 1]))) {
-                    state[0] = (double)k;
-                    s[k] = 0.0;
+                    stop = (double)k;
+                    sk = 0.0;
                 } else {
-                    s[k] = 1.0 / bk;
+                    sk = rsqrt(pos);
                 }
             }
         }
-        stop = (state[0] != 0.0) ? 1 : 0;
+        head[0] = sk;
+        head[1] = stop;
     }
     __syncthreads();
-    if (dots == nullptr) return;
-    if (stop) {
-        for (int j = threadIdx.x; j <= k; j += blockDim.x) coef[j] = 0.0;
+    const double sk = head[0], stop = head[1];
+    if (dots == nullptr || stop != 0.0) {
+        if (dots != nullptr) cluster.sync();   // every CTA has read the state before rank 0 writes it
+        if (rank != 0) return;
+        if (t == 0) {
+            s[k] = sk;
+            if (stop != 0.0) state[0] = stop;
+        }
+        if (dots != nullptr)
+            for (int j = t; j <= k; j += kCoefThreads) coef[j] = 0.0;
         return;
     }
-    const double sk = s[k];
-    for (int j = threadIdx.x; j <= k; j += blockDim.x) {
-        const double sj = s[j];
-        g[j] = sj * sk * dots[k + 1 + j];
-        c[j] = sj * sk * dots[j];
+    double *Linv = state + lz_linv_off(mmax);
+    const int64_t ldl = mmax + 1;
+    double *g = dyn, *c = g + (k + 1);       // Gram row and projections; then this CTA's column sums
+    double *l = c + (k + 1), *z = l + coef_rows(k);   // Linv g and Linv c on the CTA's rows
+    long long off = 0;     // bits of the largest |G - I| entry: non-negative doubles order as integers
+    for (int j = t; j <= k; j += kCoefThreads) {
+        const double f = (j == k ? sk : s[j]) * sk;
+        const double gj = f * dots[k + 1 + j];
+        g[j] = gj;
+        c[j] = f * dots[j];
+        off = max(off, __double_as_longlong(fabs(j == k ? gj - 1.0 : gj)));
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    // l = Linv[0:k][0:k] g[0:k]  (lower triangular, one warp per row)
-    for (int i = warp; i < k; i += nwarps) {
-        const double *row = Linv + (int64_t)i * ldl;
-        double t = 0.0;
-        for (int j = lane; j <= i; j += 32) t += row[j] * g[j];
-        t = warp_sum(t);
-        if (lane == 0) l[i] = t;
+    const double gk = g[k], ck = c[k];
+    // l = Linv[0:k][0:k] g, z = Linv[0:k][0:k] c on the CTA's rows: 8 lanes per row
+    const int sub = t >> 3, l8 = t & 7;
+    double ll = 0.0, lz = 0.0;
+    for (int p = sub; p < coef_rows(k); p += 32) {
+        const int i = p * kCoefCtas + rank;
+        double tg = 0.0, tc = 0.0;
+        if (i < k) {
+            const double *row = Linv + (int64_t)i * ldl;
+#pragma unroll 4
+            for (int j = l8; j <= i; j += 8) {
+                const double v = row[j];
+                tg = fma(v, g[j], tg);
+                tc = fma(v, c[j], tc);
+            }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            tg += __shfl_xor_sync(0xffffffffu, tg, o);
+            tc += __shfl_xor_sync(0xffffffffu, tc, o);
+        }
+        if (l8 == 0) {
+            l[p] = tg;
+            z[p] = tc;
+        }
+        ll = fma(tg, tg, ll);
+        lz = fma(tg, tc, lz);
     }
-    __syncthreads();
-    double ll = 0.0, off = 0.0;
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        ll += l[i] * l[i];
-        off = fmax(off, fabs(g[i]));
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {      // the eight lanes of a row hold the same sums
+        ll += __shfl_xor_sync(0xffffffffu, ll, o);
+        lz += __shfl_xor_sync(0xffffffffu, lz, o);
     }
-    if (threadIdx.x == 0) off = fmax(off, fabs(g[k] - 1.0));
-    ll = block_sum_d(ll, red);
-    off = block_max_d(off, red);
+    if (lane == 0) {
+        part[0][t >> 5] = ll;
+        part[1][t >> 5] = lz;
+    }
+    __syncthreads();       // l and z are written, g and c are read
+    // column sums over the CTA's rows
+    for (int j = t; j < k; j += kCoefThreads) {
+        double a = 0.0, b = 0.0;
+#pragma unroll 4
+        for (int p = (max(j - rank, 0) + kCoefCtas - 1) / kCoefCtas; p * kCoefCtas + rank < k; ++p) {
+            const double v = Linv[(int64_t)(p * kCoefCtas + rank) * ldl + j];
+            a = fma(v, l[p], a);
+            b = fma(v, z[p], b);
+        }
+        g[j] = a;
+        c[j] = b;
+    }
+    cluster.sync();
+    // l.l and l.z over the cluster, by every warp: kCoefCtas x 8 warps' sums, two per lane
+    {
+        constexpr int NW = kCoefThreads / 32;
+        static_assert(kCoefCtas * NW == 64, "two partial sums per lane");
+        const double *p0 = cluster.map_shared_rank(&part[0][0], lane / NW);
+        const double *p1 = cluster.map_shared_rank(&part[0][0], lane / NW + 32 / NW);
+        ll = warp_sum(p0[lane % NW] + p1[lane % NW]);
+        lz = warp_sum(p0[NW + lane % NW] + p1[NW + lane % NW]);
+    }
     // a healthy step has lam^2 = g_k - |l|^2 within rounding of 1; below g_k / 2 the stored
     // vector lies mostly inside the span of the basis (a Krylov space exhausted to rounding
     // noise): the run stops with k steps, before the inverse factor would blow up
-    if (k >= 1 && !(g[k] - ll >= 0.5 * g[k])) {
-        for (int j = threadIdx.x; j <= k; j += blockDim.x) coef[j] = 0.0;
-        if (threadIdx.x == 0) state[0] = (double)k;
-        return;
+    if (k >= 1 && !(gk - ll >= 0.5 * gk)) {
+        if (rank == 0) {
+            for (int j = t; j <= k; j += kCoefThreads) coef[j] = 0.0;
+            if (t == 0) {
+                s[k] = sk;
+                state[0] = (double)k;
+            }
+        }
+    } else {
+        // new row k of Linv: -(l^T Linv[0:k][0:k]) / lam, then 1 / lam; z_k = <row k, c>;
+        // y = Linv^T z, coef_j = y_j s_j: each CTA a share of the columns
+        const double ilam = rsqrt(fmax(gk - ll, 1e-300));
+        const double zk = (ck - lz) * ilam;
+        double *rowk = Linv + (int64_t)k * ldl;
+        for (int j = rank * kCoefThreads + t; j < k; j += kCoefCtas * kCoefThreads) {
+            double a = 0.0, b = 0.0;
+#pragma unroll
+            for (int r = 0; r < kCoefCtas; ++r) {
+                const double *rg = cluster.map_shared_rank(g, r);
+                a += rg[j];
+                b += rg[k + 1 + j];
+            }
+            const double v = -a * ilam;
+            rowk[j] = v;
+            coef[j] = fma(zk, v, b) * s[j];
+        }
+        if (rank == 0) {
+            if (off) atomicMax(reinterpret_cast<unsigned long long *>(state + 1), (unsigned long long)off);
+            if (t == 0) {
+                s[k] = sk;
+                rowk[k] = ilam;
+                coef[k] = zk * ilam * sk;
+                alpha[k] = ck;
+            }
+        }
     }
-    const double lam = sqrt(fmax(g[k] - ll, 1e-300));
-    // new row k of Linv: -(l^T Linv[0:k][0:k]) / lam, then 1 / lam
-    double *rowk = Linv + (int64_t)k * ldl;
-    for (int j = threadIdx.x; j < k; j += blockDim.x) {
-        double t = 0.0;
-        for (int i = j; i < k; ++i) t += l[i] * Linv[(int64_t)i * ldl + j];
-        rowk[j] = -t / lam;
-    }
-    if (threadIdx.x == 0) {
-        rowk[k] = 1.0 / lam;
-        state[1] = fmax(state[1], off);
-    }
-    __syncthreads();
-    // z = Linv[0:k+1][0:k+1] c
-    for (int i = warp; i <= k; i += nwarps) {
-        const double *row = Linv + (int64_t)i * ldl;
-        double t = 0.0;
-        for (int j = lane; j <= i; j += 32) t += row[j] * c[j];
-        t = warp_sum(t);
-        if (lane == 0) z[i] = t;
-    }
-    __syncthreads();
-    // y = Linv^T z, coef_j = y_j s_j
-    for (int j = threadIdx.x; j <= k; j += blockDim.x) {
-        double t = 0.0;
-        for (int i = j; i <= k; ++i) t += Linv[(int64_t)i * ldl + j] * z[i];
-        coef[j] = t * s[j];
-    }
-    if (threadIdx.x == 0) alpha[k] = c[k];
+    cluster.sync();        // no CTA leaves while its shared memory is read
 }
 
 }  // namespace ed
@@ -201,7 +237,11 @@ extern "C" int ed_lanczos_coef(void *stream, int k, int mmax, const double *dots
     ED_REQUIRE(k == 0 || nrm != nullptr, "nrm is NULL");
     ED_REQUIRE(dots == nullptr || (coef != nullptr && k < mmax), "coef is NULL or step %d has no next vector", k);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    lanczos_coef_kernel<<<1, kCoefThreads, 0, st>>>(k, mmax, dots, nrm, state, coef, alpha, beta);
+    const size_t smem = coef_smem(k);
+    if (smem > 48 * 1024)
+        ED_CHECK_CUDA(cudaFuncSetAttribute(lanczos_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)coef_smem(kLanczosMax)));
+    lanczos_coef_kernel<<<kCoefCtas, kCoefThreads, smem, st>>>(k, mmax, dots, nrm, state, coef, alpha, beta);
     ED_CHECK_LAUNCH();
     return ED_OK;
 }
