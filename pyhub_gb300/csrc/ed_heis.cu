@@ -666,120 +666,201 @@ __global__ void __launch_bounds__(256) heis_slab_kernel(const T *__restrict__ x,
 //   q[p][0] = J!=K: sum over states I with J up, K down of (-1)^(J+K) bra[I'] ket[I]
 //             (I' = I with J and K swapped);  J==K: 0.5 sum bra ket
 //   q[p][1] = sum bra ket Sz_J Sz_K
-// The per-pair kernel forms only the transverse (flip) sums q0 of J != K:
-// CTAs are (row range, chunk of kRdmP pairs); each thread keeps the chunk's
-// sums in registers over all its rows, so one pass over the vector serves
-// kRdmP pairs.  The diagonal sums (q1 of every pair, q0 of J == K) come from
-// heis_rdm_diag_kernel, factorised: with s_j = +1 / -1 for site j+1 up /
-// down and b = bra*ket, sum b s_J s_K is sum_col C(col) s_J s_K for two A
-// sites, sum_row W(row) s_J s_K for two B sites and sum_col s_J T_K(col) for
-// an A site J and a B site K, where per class m of rows C(col) = sum_row b,
-// T_K(col) = sum_row b s_K(row) and W(row) = sum_col b: ~nB FP64 operations
-// per element for every pair at once.
+// Everything here is bound by the FP64 pipe (2 FMA per clock and SM), so the kernels enumerate the
+// states that take part instead of testing all of them: a test leaves the other lanes' FP64 slots
+// empty (26% of the states take part in a flip).  When bra is ket, q[(J,K)] and q[(K,J)] hold the
+// same products (I <-> I') and are formed once.
+//   * heis_rdm_flip_kernel: a warp owns one task over one chunk of rows.  Two A sites: the columns
+//     with J up, K down are the patterns of the other sites with one hole less, two bits inserted;
+//     lanes over those columns, each applied to all the chunk's rows of that class.  Two B sites:
+//     whole rows against their swapped rows.  An A site J and every B site asked for with it: the
+//     columns with J fixed against one other row per B site, so an element of ket is loaded once
+//     for all of them.
+//   * heis_rdm_diag_kernel: the Sz Sz sums with an A site, factorised through column sums.
+//   * heis_rdm_rows_kernel: those of two B sites, from row sums.
+// 4x6, FP64, all pairs: 6.29 ms with every ordered pair tested state by state and 31 FP64
+// operations per element of the diagonal sums; 0.79 ms in this form (flips 0.58, diagonal 0.17, rows 0.04).
 
-constexpr int kRdmP = 8;
-constexpr int kRdmThreads = 256;
+constexpr int kRdmTasks = kMaxSites * kMaxSites;
+constexpr int kRdmChunks = 512;
 
 struct HsRdmArgs {
-    int nA, npairs;
-    int64_t nrows;
+    int nA, nB, npairs;
     int64_t col_base[kMaxHalf + 2], ncol[kMaxHalf + 1];
     const uint32_t *col_pat, *row_pat;
-    const int32_t *rankA, *row_m, *rowidx;
+    const int32_t *rankA, *rowidx, *rows_of_m;
     const int64_t *row_off;
-    int16_t pj[kMaxSites * kMaxSites], pk[kMaxSites * kMaxSites];   // hole-bit positions (site-1)
-    // the diagonal pass: rows grouped by m, and its tiles per m (columns x row ranges)
-    const int32_t *rows_of_m;
     int64_t row_base[kMaxHalf + 2];
-    int tile_base[kMaxHalf + 2], nry[kMaxHalf + 1];
+    int16_t pj[kRdmTasks], pk[kRdmTasks];   // the distinct pairs: hole-bit positions (site-1)
+    int16_t map[kRdmTasks];                 // distinct pair of each pair of the caller's list
+    // flip tasks: nab pairs (A site, orientation) first, then one per pair of two A or two B sites
+    int nab, ntask, nbb;
+    int8_t ab_site[2 * kMaxHalf], ab_bit[2 * kMaxHalf];
+    uint32_t ab_mask[2 * kMaxHalf];         // B sites asked for
+    int16_t ab_pair[2 * kMaxHalf][kMaxHalf];
+    int16_t task_pair[kRdmTasks], bb_pair[kRdmTasks];
+    // rows in rows_of_m order are cut into chunks of about equal numbers of states
+    int chunk0[kRdmChunks + 1];
+    int tile_base[kMaxHalf + 2], nry[kMaxHalf + 1];   // tiles of the diagonal pass per class m
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kRdmThreads) heis_rdm_row_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
-                                                                   const HsRdmArgs a, double *__restrict__ partials)
+constexpr int kRdmThreads = 256;
+
+__device__ __forceinline__ uint32_t insert_bit(uint32_t h, int pos, uint32_t bit)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *xs = reinterpret_cast<T *>(smem_raw);   // the bra row
-    const int p0 = blockIdx.y * kRdmP;
-    const int np = min(kRdmP, a.npairs - p0);
-    const int nA = a.nA;
-    double acc0[kRdmP], acc1[kRdmP];
+    const uint32_t low = (1u << pos) - 1u;
+    return (h & low) | ((h & ~low) << 1) | (bit << pos);
+}
+
+// acc + b k in FP64; FP32 vectors form the product in FP32, as their sums over a row always have
+template <typename T> __device__ __forceinline__ void mul_add(double &acc, T b, T k)
+{
+    if constexpr (sizeof(T) == 8) acc = fma(b, k, acc);
+    else acc += (double)(b * k);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kRdmThreads) heis_rdm_flip_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
+                                                                    const HsRdmArgs a, int mlo, int mhi,
+                                                                    double *__restrict__ partials)
+{
+    const int lane = threadIdx.x & 31;
+    const int task = blockIdx.x * (kRdmThreads / 32) + (threadIdx.x >> 5), chunk = blockIdx.y;
+    if (task >= a.ntask) return;
+    double *out = partials + (int64_t)chunk * a.npairs * 2;
+    const int64_t p0 = a.chunk0[chunk], p1 = a.chunk0[chunk + 1];
+    if (task < a.nab) {
+        const int J = a.ab_site[task];
+        const uint32_t bit = (uint32_t)a.ab_bit[task], mask = a.ab_mask[task];
+        double acc[kMaxHalf];
 #pragma unroll
-    for (int q = 0; q < kRdmP; ++q) acc0[q] = acc1[q] = 0.0;
-    for (int64_t row = blockIdx.x; row < a.nrows; row += gridDim.x) {
-        const uint32_t hb = __ldg(a.row_pat + row);
-        const int m = __ldg(a.row_m + row);
-        const int64_t off = __ldg(a.row_off + row);
-        const int len = (int)a.ncol[m];
-        const int64_t cbase = a.col_base[m];
-        __syncthreads();
-        for (int c = threadIdx.x; c < len; c += blockDim.x) xs[c] = bra[off + c];
-        __syncthreads();
-        // per-row facts of every pair: source row offset of the swapped state (or -1)
-        int64_t soff[kRdmP];
+        for (int k = 0; k < kMaxHalf; ++k) acc[k] = 0.0;
+        for (int m = mlo; m <= mhi; ++m) {
+            const int64_t ra = max(p0, a.row_base[m]), rb = min(p1, a.row_base[m + 1]);
+            if (ra >= rb || m < (int)bit) continue;
+            // the patterns of the other nA - 1 A sites with m - bit holes are the first of their class
+            const int hm = m - (int)bit;
+            if (hm > a.nA - 1) continue;
+            int64_t ne = 1;
+            for (int i = 1; i <= hm; ++i) ne = ne * (a.nA - 1 - hm + i) / i;
+            for (int64_t r = ra; r < rb; ++r) {
+                const int32_t row = __ldg(a.rows_of_m + r);
+                const uint32_t hb = __ldg(a.row_pat + row);
+                const uint32_t need = mask & (bit ? ~hb : hb);
+                if (!need) continue;
+                const T *kr = ket + __ldg(a.row_off + row);
+                int64_t my_off = 0;
+                if ((need >> lane) & 1u) my_off = __ldg(a.row_off + __ldg(a.rowidx + (hb ^ (1u << lane))));
+                for (int64_t e0 = 0; e0 < ne; e0 += 32) {
+                    const int64_t e = e0 + lane;
+                    const bool ok = e < ne;
+                    const uint32_t base = __ldg(a.col_pat + a.col_base[hm] + (ok ? e : 0));
+                    const uint32_t h = insert_bit(base, J, bit);
+                    const int c = __ldg(a.rankA + h), c2 = __ldg(a.rankA + (h ^ (1u << J)));
+                    const T kv = ok ? __ldg(kr + c) : (T)0;
 #pragma unroll
-        for (int q = 0; q < kRdmP; ++q) {
-            soff[q] = -1;
-            if (q >= np) continue;
-            const int J = a.pj[p0 + q], K = a.pk[p0 + q];
-            uint32_t mb = 0;
-            if (J >= nA) mb |= 1u << (J - nA);
-            if (K >= nA) mb |= 1u << (K - nA);
-            if (mb) {
-                const int32_t r2 = __ldg(a.rowidx + (hb ^ mb));
-                if (r2 >= 0) soff[q] = __ldg(a.row_off + r2);
-            } else {
-                soff[q] = off;
+                    for (int k = 0; k < kMaxHalf; ++k) {
+                        if ((need >> k) & 1u) {
+                            const int64_t o2 = __shfl_sync(0xffffffffu, my_off, k);
+                            mul_add<T>(acc[k], __ldg(bra + o2 + c2), kv);
+                        }
+                    }
+                }
             }
         }
-        T r0[kRdmP], r1[kRdmP];
 #pragma unroll
-        for (int q = 0; q < kRdmP; ++q) r0[q] = r1[q] = 0;
-        for (int c = threadIdx.x; c < len; c += blockDim.x) {
-            const uint32_t ha = __ldg(a.col_pat + cbase + c);
-            const uint64_t h = (uint64_t)ha | ((uint64_t)hb << nA);   // bit j: site j+1 is down
-            const T kv = __ldg(ket + off + c);
-#pragma unroll
-            for (int q = 0; q < kRdmP; ++q) {
-                if (q >= np) break;
-                const int J = a.pj[p0 + q], K = a.pk[p0 + q];
-                const int dJ = (int)((h >> J) & 1u), dK = (int)((h >> K) & 1u);
-                if (J == K || dJ || !dK || soff[q] < 0) continue;   // a flip needs J up, K down
-                // the swapped state: A part and B part of h ^ (bit J | bit K)
-                uint32_t ma = 0;
-                if (J < nA) ma |= 1u << J;
-                if (K < nA) ma |= 1u << K;
-                const int cs = ma ? __ldg(a.rankA + (ha ^ ma)) : c;
-                const T bv = (soff[q] == off) ? xs[cs] : __ldg(bra + soff[q] + cs);
-                // sign (-1)^((J+1)+(K+1)) folded into the FMA's operand: one operation per flip
-                r0[q] = ((J + K) & 1) ? fma(-bv, kv, r0[q]) : fma(bv, kv, r0[q]);
+        for (int k = 0; k < kMaxHalf; ++k) {
+            if (!((mask >> k) & 1u)) continue;
+            const double s = warp_sum(acc[k]);
+            if (lane == 0) out[2 * a.ab_pair[task][k]] = ((J + k + a.nA) & 1) ? -s : s;
+        }
+        return;
+    }
+    const int p = a.task_pair[task - a.nab];
+    const int J = a.pj[p], K = a.pk[p];
+    double acc = 0.0;
+    if (J < a.nA) {     // two A sites
+        const int lo = min(J, K), hi = max(J, K);
+        const uint32_t mask = (1u << J) | (1u << K);
+        for (int m = max(mlo, 1); m <= mhi; ++m) {
+            const int64_t ra = max(p0, a.row_base[m]), rb = min(p1, a.row_base[m + 1]);
+            if (ra >= rb || m - 1 > a.nA - 2) continue;
+            int64_t ne = 1;
+            for (int i = 1; i <= m - 1; ++i) ne = ne * (a.nA - 2 - (m - 1) + i) / i;
+            for (int64_t e = lane; e < ne; e += 32) {
+                const uint32_t base = __ldg(a.col_pat + a.col_base[m - 1] + e);
+                const uint32_t h = insert_bit(insert_bit(base, lo, lo == K), hi, hi == K);   // J up, K down
+                const int c = __ldg(a.rankA + h), c2 = __ldg(a.rankA + (h ^ mask));
+#pragma unroll 4
+                for (int64_t r = ra; r < rb; ++r) {
+                    const int64_t off = __ldg(a.row_off + __ldg(a.rows_of_m + r));
+                    mul_add<T>(acc, __ldg(bra + off + c2), __ldg(ket + off + c));
+                }
             }
         }
-#pragma unroll
-        for (int q = 0; q < kRdmP; ++q) {
-            acc0[q] += (double)r0[q];
-            acc1[q] += (double)r1[q];
+    } else {            // two B sites
+        const uint32_t bJ = 1u << (J - a.nA), bK = 1u << (K - a.nA);
+        for (int m = mlo; m <= mhi; ++m) {
+            const int64_t ra = max(p0, a.row_base[m]), rb = min(p1, a.row_base[m + 1]);
+            const int len = (int)a.ncol[m];
+            for (int64_t r = ra; r < rb; ++r) {
+                const int32_t row = __ldg(a.rows_of_m + r);
+                const uint32_t hb = __ldg(a.row_pat + row);
+                if ((hb & bJ) || !(hb & bK)) continue;
+                const T *kr = ket + __ldg(a.row_off + row);
+                const T *br = bra + __ldg(a.row_off + __ldg(a.rowidx + (hb ^ bJ ^ bK)));
+#pragma unroll 4
+                for (int c = lane; c < len; c += 32) mul_add<T>(acc, __ldg(br + c), __ldg(kr + c));
+            }
         }
     }
-    __shared__ double red[kRdmThreads / 32][kRdmP][2];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int q = 0; q < kRdmP; ++q) {
-        const double w0 = warp_sum(acc0[q]), w1 = warp_sum(acc1[q]);
-        if (lane == 0) {
-            red[warp][q][0] = w0;
-            red[warp][q][1] = w1;
+    acc = warp_sum(acc);
+    if (lane == 0) out[2 * p] = ((J + K) & 1) ? -acc : acc;
+}
+
+// Sz Sz of two B sites: with W(row) = sum over the row of b = bra ket, sum_row W s_J s_K.  A warp per
+// row (one FMA per element), the row's W then goes to every pair's sum (lanes over pairs).
+template <typename T>
+__global__ void __launch_bounds__(kRdmThreads) heis_rdm_rows_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
+                                                                    const HsRdmArgs a, int mlo, int mhi,
+                                                                    double *__restrict__ partials)
+{
+    extern __shared__ double accs[];   // [8 warps][nbb]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = blockIdx.x;
+    double *mine = accs + warp * a.nbb;
+    for (int q = lane; q < a.nbb; q += 32) mine[q] = 0.0;
+    const int64_t p0 = a.chunk0[chunk], p1 = a.chunk0[chunk + 1];
+    for (int m = mlo; m <= mhi; ++m) {
+        const int64_t ra = max(p0, a.row_base[m]), rb = min(p1, a.row_base[m + 1]);
+        const int len = (int)a.ncol[m];
+        for (int64_t r = ra + warp; r < rb; r += kRdmThreads / 32) {
+            const int32_t row = __ldg(a.rows_of_m + r);
+            const uint32_t hb = __ldg(a.row_pat + row);
+            const int64_t off = __ldg(a.row_off + row);
+            double w = 0.0;
+#pragma unroll 4
+            for (int c = lane; c < len; c += 32) w = fma((double)__ldg(bra + off + c), (double)__ldg(ket + off + c), w);
+            w = warp_sum(w);
+            for (int q = lane; q < a.nbb; q += 32) {
+                const int p = a.bb_pair[q];
+                mine[q] += (((hb >> (a.pj[p] - a.nA)) ^ (hb >> (a.pk[p] - a.nA))) & 1u) ? -w : w;
+            }
         }
     }
     __syncthreads();
-    if (threadIdx.x < 2 * np) {
-        const int q = threadIdx.x >> 1, k = threadIdx.x & 1;
+    for (int q = threadIdx.x; q < a.nbb; q += kRdmThreads) {
         double t = 0.0;
-        for (int w = 0; w < kRdmThreads / 32; ++w) t += red[w][q][k];
-        partials[((int64_t)blockIdx.x * a.npairs + p0 + q) * 2 + k] = t;
+        for (int w = 0; w < kRdmThreads / 32; ++w) t += accs[w * a.nbb + q];
+        partials[((int64_t)chunk * a.npairs + a.bb_pair[q]) * 2 + 1] = 0.25 * t;
     }
 }
 
+// The other diagonal sums: with s_j = +1 / -1 for site j+1 up / down, sum b s_J s_K is
+// sum_col C(col) s_J s_K for two A sites and sum_col s_J T_K(col) for an A site J and a B site K, where
+// per class m of rows C(col) = sum_row b and T_K(col) = sum_row b s_K(row) = C - 2 (sum over the rows
+// with K down).  A thread owns a column; rows come in ascending pattern order, so the low half of the
+// B sites costs an addition only where the bit is set (uniform over the CTA) and the high half one
+// addition per run of equal high bits: about 2 + nB/4 FP64 operations per element.
 constexpr int kHdThreads = 256;
 
 template <typename T>
@@ -790,8 +871,7 @@ __global__ void __launch_bounds__(kHdThreads) heis_rdm_diag_kernel(const T *__re
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *Ts = reinterpret_cast<double *>(smem_raw);   // [kMaxHalf][kHdThreads]
     double *Cs = Ts + kMaxHalf * kHdThreads;              // [kHdThreads]
-    double *accW = Cs + kHdThreads;                       // [npairs]
-    __shared__ double red[kHdThreads / 32];
+    constexpr int LO = kMaxHalf / 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int m = mlo;
     while (m < mhi && blockIdx.x >= a.tile_base[m + 1]) ++m;
@@ -802,68 +882,91 @@ __global__ void __launch_bounds__(kHdThreads) heis_rdm_diag_kernel(const T *__re
     const bool act = col < a.ncol[m];
     const int64_t nr_m = a.row_base[m + 1] - a.row_base[m];
     const int64_t q0r = nr_m * ry / nry, q1r = nr_m * (ry + 1) / nry;
-    const int nA = a.nA;
-    for (int q = threadIdx.x; q < a.npairs; q += blockDim.x) accW[q] = 0.0;
-    double C = 0.0, Tk[kMaxHalf];
+    const int nA = a.nA, lo = a.nB / 2;     // B bits [0, lo) bit by bit, [lo, nB) per run
+    double C = 0.0, S = 0.0, Tl[LO], Th[LO];
 #pragma unroll
-    for (int k = 0; k < kMaxHalf; ++k) Tk[k] = 0.0;
-    for (int64_t rr = q0r; rr < q1r; ++rr) {
-        const int32_t row = __ldg(a.rows_of_m + a.row_base[m] + rr);
-        const uint32_t hb = __ldg(a.row_pat + row);
-        const int64_t off = __ldg(a.row_off + row);
-        const double b = act ? (double)__ldg(bra + off + col) * (double)__ldg(ket + off + col) : 0.0;
-        C += b;
+    for (int k = 0; k < LO; ++k) Tl[k] = Th[k] = 0.0;
+    uint32_t run = 0;
+    auto flush = [&]() {
 #pragma unroll
-        for (int k = 0; k < kMaxHalf; ++k) Tk[k] += ((hb >> k) & 1u) ? -b : b;
-        double w = warp_sum(b);
-        __syncthreads();
-        if (lane == 0) red[warp] = w;
-        __syncthreads();
-        w = 0.0;
+        for (int k = 0; k < LO; ++k)
+            if ((run >> k) & 1u) Th[k] += S;
+        C += S;
+        S = 0.0;
+    };
+    const int32_t *rows = a.rows_of_m + a.row_base[m];
+    for (int64_t r0 = q0r; r0 < q1r; r0 += 4) {
+        double b[4];
+        uint32_t hb[4];
 #pragma unroll
-        for (int q = 0; q < kHdThreads / 32; ++q) w += red[q];
-        for (int q = threadIdx.x; q < a.npairs; q += blockDim.x) {
-            const int J = a.pj[q], K = a.pk[q];
-            if (J >= nA && K >= nA && J != K) {
-                const int sJ = ((hb >> (J - nA)) & 1u) ? -1 : 1, sK = ((hb >> (K - nA)) & 1u) ? -1 : 1;
-                accW[q] += (sJ * sK > 0) ? w : -w;
+        for (int i = 0; i < 4; ++i) {       // four rows' loads in flight
+            const bool in = r0 + i < q1r;
+            const int32_t row = __ldg(rows + (in ? r0 + i : q1r - 1));
+            hb[i] = __ldg(a.row_pat + row);
+            const int64_t at = __ldg(a.row_off + row) + col;
+            b[i] = (in && act) ? (double)__ldg(bra + at) * (double)__ldg(ket + at) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if ((hb[i] >> lo) != run) {
+                flush();
+                run = hb[i] >> lo;
             }
+            S += b[i];
+#pragma unroll
+            for (int k = 0; k < LO; ++k)
+                if (k < lo && ((hb[i] >> k) & 1u)) Tl[k] += b[i];
         }
     }
+    flush();
 #pragma unroll
-    for (int k = 0; k < kMaxHalf; ++k) Ts[k * kHdThreads + threadIdx.x] = Tk[k];
+    for (int k = 0; k < LO; ++k) {
+        if (k < lo) Ts[k * kHdThreads + threadIdx.x] = C - 2.0 * Tl[k];
+        if (lo + k < a.nB) Ts[(lo + k) * kHdThreads + threadIdx.x] = C - 2.0 * Th[k];
+    }
     Cs[threadIdx.x] = C;
     __syncthreads();
+    // sums over the tile's columns (a column past the class holds zeros): lanes over columns
+    constexpr int NC = kHdThreads / 32;
+    uint32_t ha[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i)
+        ha[i] = __ldg(a.col_pat + a.col_base[m] + min((int64_t)cx * kHdThreads + i * 32 + lane, a.ncol[m] - 1));
     for (int q = warp; q < a.npairs; q += kHdThreads / 32) {
         const int J = a.pj[q], K = a.pk[q];
+        if (J >= nA && K >= nA && J != K) continue;      // heis_rdm_rows_kernel
+        const bool cross = (J < nA) != (K < nA);
+        const int ja = J < nA ? J : K;
+        const double *v = cross ? Ts + ((J < nA ? K : J) - nA) * kHdThreads : Cs;
+        const int kA = (J == K || cross) ? 31 : K;       // bit 31 of a pattern is clear
+        const int jA = (J == K) ? 31 : ja;
         double s1 = 0.0;
-        for (int t = lane; t < kHdThreads; t += 32) {
-            const int64_t cc = (int64_t)cx * kHdThreads + t;
-            if (cc >= a.ncol[m]) continue;
-            const uint32_t ha = __ldg(a.col_pat + a.col_base[m] + cc);
-            if (J == K) {
-                s1 += Cs[t];
-            } else if (J < nA && K < nA) {
-                const bool neg = (((ha >> J) ^ (ha >> K)) & 1u) != 0;
-                s1 += neg ? -Cs[t] : Cs[t];
-            } else if (J < nA || K < nA) {
-                const int ja = J < nA ? J : K, kb = (J < nA ? K : J) - nA;
-                const double tv = Ts[kb * kHdThreads + t];
-                s1 += ((ha >> ja) & 1u) ? -tv : tv;
-            }
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            const double tv = v[i * 32 + lane];
+            s1 += (((ha[i] >> jA) ^ (ha[i] >> kA)) & 1u) ? -tv : tv;
         }
         s1 = warp_sum(s1);
         if (lane == 0) {
             double *o = partials + ((int64_t)blockIdx.x * a.npairs + q) * 2;
-            if (J == K) {
-                o[0] = 0.5 * s1;
-                o[1] = 0.25 * s1;
-            } else {
-                o[0] = 0.0;
-                o[1] = 0.25 * ((J >= nA && K >= nA) ? accW[q] : s1);
-            }
+            if (J == K) o[0] = 0.5 * s1;
+            o[1] = 0.25 * s1;
         }
     }
+}
+
+// out[p][k] = sum over the partial rows of the distinct pair of p
+__global__ void __launch_bounds__(256) heis_rdm_reduce_kernel(const double *__restrict__ partials, int nrows,
+                                                              const HsRdmArgs a, int nout, double *__restrict__ out)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int j = blockIdx.x * 8 + warp;
+    if (j >= 2 * nout) return;
+    const int q = 2 * a.map[j >> 1] + (j & 1);
+    double s = 0.0;
+    for (int b = lane; b < nrows; b += 32) s += partials[(int64_t)b * 2 * a.npairs + q];
+    s = warp_sum(s);
+    if (lane == 0) out[j] = s;
 }
 
 template <typename T>
@@ -871,28 +974,62 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
                                const int32_t *pairs, double *out, double *scratch, int max_blocks)
 {
     const HeisStruct &h = *s->hs;
-    HsRdmArgs a;
-    a.nA = h.nA;
-    a.npairs = npairs;
-    a.nrows = h.nrows;
-    for (int m = 0; m <= kMaxHalf + 1; ++m) {
-        a.col_base[m] = h.col_base[m];
-        if (m <= kMaxHalf) a.ncol[m] = h.ncol[m];
-    }
-    a.col_pat = h.col_pat; a.row_pat = h.row_pat;
-    a.rankA = h.rankA; a.row_m = h.row_m; a.rowidx = h.rowidx; a.row_off = h.row_off;
-    for (int p = 0; p < npairs; ++p) {
-        a.pj[p] = (int16_t)(pairs[2 * p] - 1);
-        a.pk[p] = (int16_t)(pairs[2 * p + 1] - 1);
-    }
     if (h.nB > kMaxHalf) {
         set_error("B half of %d sites (at most %d)", h.nB, kMaxHalf);
         return ED_ERR_RANGE;
     }
+    HsRdmArgs a;
+    a.nA = h.nA;
+    a.nB = h.nB;
+    for (int m = 0; m <= kMaxHalf + 1; ++m) {
+        a.col_base[m] = h.col_base[m];
+        a.row_base[m] = h.row_base[m];
+        if (m <= kMaxHalf) a.ncol[m] = h.ncol[m];
+    }
+    a.col_pat = h.col_pat; a.row_pat = h.row_pat;
+    a.rankA = h.rankA; a.rowidx = h.rowidx; a.row_off = h.row_off;
     a.rows_of_m = h.rows_of_m;
-    for (int m = 0; m <= kMaxHalf + 1; ++m) a.row_base[m] = h.row_base[m];
-    // diagonal tiles: per class m, 256-column tiles times row ranges, about max_blocks in all
+    // distinct pairs (unordered when bra is ket) and the tasks they give
+    int16_t seen[kMaxSites][kMaxSites];
+    std::memset(seen, -1, sizeof(seen));
+    int16_t ab_task[kMaxHalf][2];
+    std::memset(ab_task, -1, sizeof(ab_task));
+    a.npairs = a.nab = a.nbb = 0;
+    int nother = 0;
+    const bool same = (bra == ket);
+    for (int p = 0; p < npairs; ++p) {
+        int J = pairs[2 * p] - 1, K = pairs[2 * p + 1] - 1;
+        if (same && J > K) std::swap(J, K);
+        if (seen[J][K] < 0) {
+            const int q = a.npairs++;
+            seen[J][K] = (int16_t)q;
+            a.pj[q] = (int16_t)J;
+            a.pk[q] = (int16_t)K;
+            const bool ja = J < h.nA, ka = K < h.nA;
+            if (J != K && ja != ka) {
+                const int site = ja ? J : K, bit = ja ? 0 : 1, kb = (ja ? K : J) - h.nA;   // J up: bit 0 at an A site J
+                if (ab_task[site][bit] < 0) {
+                    const int t = a.nab++;
+                    ab_task[site][bit] = (int16_t)t;
+                    a.ab_site[t] = (int8_t)site;
+                    a.ab_bit[t] = (int8_t)bit;
+                    a.ab_mask[t] = 0;
+                }
+                const int t = ab_task[site][bit];
+                a.ab_mask[t] |= 1u << kb;
+                a.ab_pair[t][kb] = (int16_t)q;
+            } else if (J != K) {
+                a.task_pair[nother++] = (int16_t)q;
+                if (!ja) a.bb_pair[a.nbb++] = (int16_t)q;
+            }
+        }
+        a.map[p] = seen[J][K];
+    }
+    a.ntask = a.nab + nother;
+    // diagonal tiles: per class m, 256-column tiles times row ranges, about one per SM (a tile's sums over
+    // the pairs cost more than its rows)
     const int64_t dim = s->dim;
+    const int want_tiles = std::min(num_sms(), max_blocks);
     int ntiles = 0;
     for (int m = 0; m <= kMaxHalf + 1; ++m) a.tile_base[m] = 0;
     for (int m = h.mlo; m <= h.mhi; ++m) {
@@ -900,30 +1037,55 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
         const int64_t nr_m = h.row_base[m + 1] - h.row_base[m];
         const int ncx = (int)((h.ncol[m] + kHdThreads - 1) / kHdThreads);
         const double share = dim > 0 ? (double)(h.ncol[m] * nr_m) / (double)dim : 0.0;
-        int nry = (int)std::max<double>(1.0, std::floor(share * max_blocks / std::max(ncx, 1)));
+        int nry = (int)std::max<double>(1.0, std::floor(share * want_tiles / std::max(ncx, 1)));
         nry = (int)std::min<int64_t>(std::max<int64_t>(nr_m, 1), nry);
         a.nry[m] = nry;
         ntiles += ncx * nry;
     }
     a.tile_base[h.mhi + 1] = ntiles;
-    const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(h.nrows, max_blocks));
-    if (gx + ntiles > 3 * max_blocks) {
-        set_error("spin-correlation pass needs %d partial rows (scratch holds %d)", gx + ntiles, 3 * max_blocks);
+    // row chunks: rows [0, nrows) of rows_of_m, cut where the states before them pass i/nch of all
+    const int nch = (int)std::max<int64_t>(1, std::min<int64_t>({h.nrows, kRdmChunks, 3 * max_blocks - ntiles}));
+    if (nch + ntiles > 3 * max_blocks) {
+        set_error("spin-correlation pass needs %d partial rows (scratch holds %d)", nch + ntiles, 3 * max_blocks);
         return ED_ERR_RANGE;
     }
-    // flips (q0 of J != K) into partial rows [0, gx), diagonal sums into [gx, gx + ntiles)
-    const size_t smem = (size_t)std::max<int64_t>(h.max_len, 1) * sizeof(T);
-    ED_CHECK_CUDA(cudaFuncSetAttribute(heis_rdm_row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const dim3 grid((unsigned)gx, (unsigned)((npairs + kRdmP - 1) / kRdmP));
-    heis_rdm_row_kernel<T><<<grid, kRdmThreads, smem, st>>>(bra, ket, a, scratch);
-    ED_CHECK_LAUNCH();
-    const size_t smemd = (size_t)(kMaxHalf + 1) * kHdThreads * sizeof(double) + (size_t)npairs * sizeof(double);
-    ED_CHECK_CUDA(cudaFuncSetAttribute(heis_rdm_diag_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smemd));
+    {
+        int m = h.mlo;
+        int64_t before = 0;     // states of the classes below m
+        for (int i = 0; i <= nch; ++i) {
+            const int64_t want = (int64_t)((double)dim * i / nch);
+            while (m < h.mhi && before + h.ncol[m] * (h.row_base[m + 1] - h.row_base[m]) <= want) {
+                before += h.ncol[m] * (h.row_base[m + 1] - h.row_base[m]);
+                ++m;
+            }
+            const int64_t r = h.row_base[m] + (want - before) / std::max<int64_t>(h.ncol[m], 1);
+            a.chunk0[i] = (int)std::min<int64_t>(i == nch ? h.nrows : r, h.nrows);
+        }
+        a.chunk0[0] = 0;
+    }
+    // partial rows [0, nch): flips and two-B-site sums of each chunk; [nch, nch + ntiles): the tiles
+    ED_CHECK_CUDA(cudaMemsetAsync(scratch, 0, sizeof(double) * 2 * (size_t)a.npairs * (nch + ntiles), st));
+    if (a.ntask > 0) {
+        constexpr int W = kRdmThreads / 32;
+        heis_rdm_flip_kernel<T><<<dim3((unsigned)((a.ntask + W - 1) / W), (unsigned)nch), kRdmThreads, 0, st>>>(
+            bra, ket, a, h.mlo, h.mhi, scratch);
+        ED_CHECK_LAUNCH();
+    }
+    if (a.nbb > 0) {
+        const size_t smemr = (size_t)(kRdmThreads / 32) * a.nbb * sizeof(double);
+        if (smemr > 48 * 1024)
+            ED_CHECK_CUDA(cudaFuncSetAttribute(heis_rdm_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smemr));
+        heis_rdm_rows_kernel<T><<<nch, kRdmThreads, smemr, st>>>(bra, ket, a, h.mlo, h.mhi, scratch);
+        ED_CHECK_LAUNCH();
+    }
+    const size_t smemd = (size_t)(kMaxHalf + 1) * kHdThreads * sizeof(double);
     heis_rdm_diag_kernel<T><<<ntiles, kHdThreads, smemd, st>>>(bra, ket, a, h.mlo, h.mhi,
-                                                                scratch + (int64_t)gx * 2 * npairs);
+                                                               scratch + (int64_t)nch * 2 * a.npairs);
     ED_CHECK_LAUNCH();
-    return launch_reduce(scratch, gx + ntiles, 2 * npairs, out, st);
+    heis_rdm_reduce_kernel<<<(2 * npairs + 7) / 8, 256, 0, st>>>(scratch, nch + ntiles, a, npairs, out);
+    ED_CHECK_LAUNCH();
+    return ED_OK;
 }
 
 int heis_struct_rdm(ed_sector *s, cudaStream_t st, int dtype, const void *bra, const void *ket, int npairs,
