@@ -670,16 +670,17 @@ __global__ void __launch_bounds__(256) heis_slab_kernel(const T *__restrict__ x,
 // states that take part instead of testing all of them: a test leaves the other lanes' FP64 slots
 // empty (26% of the states take part in a flip).  When bra is ket, q[(J,K)] and q[(K,J)] hold the
 // same products (I <-> I') and are formed once.
-//   * heis_rdm_flip_kernel: a warp owns one task over one chunk of rows.  Two A sites: the columns
+//   * rdm_flips: a warp owns one task over one chunk of rows.  Two A sites: the columns
 //     with J up, K down are the patterns of the other sites with one hole less, two bits inserted;
 //     lanes over those columns, each applied to all the chunk's rows of that class.  Two B sites:
 //     whole rows against their swapped rows.  An A site J and every B site asked for with it: the
 //     columns with J fixed against one other row per B site, so an element of ket is loaded once
 //     for all of them.
-//   * heis_rdm_diag_kernel: the Sz Sz sums with an A site, factorised through column sums.
-//   * heis_rdm_rows_kernel: those of two B sites, from row sums.
-// 4x6, FP64, all pairs: 6.29 ms with every ordered pair tested state by state and 31 FP64
-// operations per element of the diagonal sums; 0.79 ms in this form (flips 0.58, diagonal 0.17, rows 0.04).
+//   * rdm_diag_tile: the Sz Sz sums with an A site, factorised through column sums.
+//   * rdm_rows: those of two B sites, from row sums.
+// The three run as one launch.  All pairs of 24 sites, FP64, whole call: 6.38 ms with every ordered
+// pair tested state by state and 31 FP64 operations per element of the diagonal sums, 0.78 ms in
+// this form; 8 sites 69 -> 68 us, 16 sites 371 -> 128 us.
 
 constexpr int kRdmTasks = kMaxSites * kMaxSites;
 constexpr int kRdmChunks = 512;
@@ -691,8 +692,7 @@ struct HsRdmArgs {
     const int32_t *rankA, *rowidx, *rows_of_m;
     const int64_t *row_off;
     int64_t row_base[kMaxHalf + 2];
-    int16_t pj[kRdmTasks], pk[kRdmTasks];   // the distinct pairs: hole-bit positions (site-1)
-    int16_t map[kRdmTasks];                 // distinct pair of each pair of the caller's list
+    int8_t pj[kRdmTasks], pk[kRdmTasks];    // the distinct pairs: hole-bit positions (site-1)
     // flip tasks: nab pairs (A site, orientation) first, then one per pair of two A or two B sites
     int nab, ntask, nbb;
     int8_t ab_site[2 * kMaxHalf], ab_bit[2 * kMaxHalf];
@@ -720,12 +720,10 @@ template <typename T> __device__ __forceinline__ void mul_add(double &acc, T b, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kRdmThreads) heis_rdm_flip_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
-                                                                    const HsRdmArgs a, int mlo, int mhi,
-                                                                    double *__restrict__ partials)
+__device__ __forceinline__ void rdm_flips(const T *__restrict__ bra, const T *__restrict__ ket, const HsRdmArgs &a,
+                                          int mlo, int mhi, int task, int chunk, double *__restrict__ partials)
 {
     const int lane = threadIdx.x & 31;
-    const int task = blockIdx.x * (kRdmThreads / 32) + (threadIdx.x >> 5), chunk = blockIdx.y;
     if (task >= a.ntask) return;
     double *out = partials + (int64_t)chunk * a.npairs * 2;
     const int64_t p0 = a.chunk0[chunk], p1 = a.chunk0[chunk + 1];
@@ -821,12 +819,11 @@ __global__ void __launch_bounds__(kRdmThreads) heis_rdm_flip_kernel(const T *__r
 // Sz Sz of two B sites: with W(row) = sum over the row of b = bra ket, sum_row W s_J s_K.  A warp per
 // row (one FMA per element), the row's W then goes to every pair's sum (lanes over pairs).
 template <typename T>
-__global__ void __launch_bounds__(kRdmThreads) heis_rdm_rows_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
-                                                                    const HsRdmArgs a, int mlo, int mhi,
-                                                                    double *__restrict__ partials)
+__device__ __forceinline__ void rdm_rows(const T *__restrict__ bra, const T *__restrict__ ket, const HsRdmArgs &a,
+                                         int mlo, int mhi, int chunk, double *accs, double *__restrict__ partials)
 {
-    extern __shared__ double accs[];   // [8 warps][nbb]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = blockIdx.x;
+    // accs: [8 warps][nbb]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double *mine = accs + warp * a.nbb;
     for (int q = lane; q < a.nbb; q += 32) mine[q] = 0.0;
     const int64_t p0 = a.chunk0[chunk], p1 = a.chunk0[chunk + 1];
@@ -861,22 +858,20 @@ __global__ void __launch_bounds__(kRdmThreads) heis_rdm_rows_kernel(const T *__r
 // with K down).  A thread owns a column; rows come in ascending pattern order, so the low half of the
 // B sites costs an addition only where the bit is set (uniform over the CTA) and the high half one
 // addition per run of equal high bits: about 2 + nB/4 FP64 operations per element.
-constexpr int kHdThreads = 256;
+constexpr int kHdThreads = kRdmThreads;
 
 template <typename T>
-__global__ void __launch_bounds__(kHdThreads) heis_rdm_diag_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
-                                                                   const HsRdmArgs a, int mlo, int mhi,
-                                                                   double *__restrict__ partials)
+__device__ __forceinline__ void rdm_diag_tile(const T *__restrict__ bra, const T *__restrict__ ket, const HsRdmArgs &a,
+                                              int mlo, int mhi, int tile, double *Ts, double *__restrict__ partials)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *Ts = reinterpret_cast<double *>(smem_raw);   // [kMaxHalf][kHdThreads]
-    double *Cs = Ts + kMaxHalf * kHdThreads;              // [kHdThreads]
+    // Ts: [nB][kHdThreads], then Cs
+    double *Cs = Ts + a.nB * kHdThreads;
     constexpr int LO = kMaxHalf / 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int m = mlo;
-    while (m < mhi && blockIdx.x >= a.tile_base[m + 1]) ++m;
+    while (m < mhi && tile >= a.tile_base[m + 1]) ++m;
     const int ncx = (int)((a.ncol[m] + kHdThreads - 1) / kHdThreads);
-    const int local = blockIdx.x - a.tile_base[m];
+    const int local = tile - a.tile_base[m];
     const int cx = local % ncx, ry = local / ncx, nry = a.nry[m];
     const int64_t col = (int64_t)cx * kHdThreads + threadIdx.x;
     const bool act = col < a.ncol[m];
@@ -934,7 +929,7 @@ __global__ void __launch_bounds__(kHdThreads) heis_rdm_diag_kernel(const T *__re
         ha[i] = __ldg(a.col_pat + a.col_base[m] + min((int64_t)cx * kHdThreads + i * 32 + lane, a.ncol[m] - 1));
     for (int q = warp; q < a.npairs; q += kHdThreads / 32) {
         const int J = a.pj[q], K = a.pk[q];
-        if (J >= nA && K >= nA && J != K) continue;      // heis_rdm_rows_kernel
+        if (J >= nA && K >= nA && J != K) continue;      // rdm_rows
         const bool cross = (J < nA) != (K < nA);
         const int ja = J < nA ? J : K;
         const double *v = cross ? Ts + ((J < nA ? K : J) - nA) * kHdThreads : Cs;
@@ -948,23 +943,53 @@ __global__ void __launch_bounds__(kHdThreads) heis_rdm_diag_kernel(const T *__re
         }
         s1 = warp_sum(s1);
         if (lane == 0) {
-            double *o = partials + ((int64_t)blockIdx.x * a.npairs + q) * 2;
+            double *o = partials + ((int64_t)tile * a.npairs + q) * 2;
             if (J == K) o[0] = 0.5 * s1;
             o[1] = 0.25 * s1;
         }
     }
 }
 
+// One launch: the diagonal tiles, then the row chunks, then the flips (tasks of one chunk side by side).
+template <typename T>
+__global__ void __launch_bounds__(kRdmThreads) heis_rdm_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
+                                                               const __grid_constant__ HsRdmArgs a, int mlo, int mhi,
+                                                               int ntiles, int nch, double *__restrict__ partials)
+{
+    extern __shared__ __align__(16) double smem_d[];
+    int b = blockIdx.x;
+    if (b < ntiles) {
+        rdm_diag_tile<T>(bra, ket, a, mlo, mhi, b, smem_d, partials + (int64_t)nch * 2 * a.npairs);
+        return;
+    }
+    b -= ntiles;
+    if (a.nbb > 0) {
+        if (b < nch) {
+            rdm_rows<T>(bra, ket, a, mlo, mhi, b, smem_d, partials);
+            return;
+        }
+        b -= nch;
+    }
+    constexpr int W = kRdmThreads / 32;
+    const int ng = (a.ntask + W - 1) / W;
+    rdm_flips<T>(bra, ket, a, mlo, mhi, (b % ng) * W + (threadIdx.x >> 5), b / ng, partials);
+}
+
 // out[p][k] = sum over the partial rows of the distinct pair of p
-__global__ void __launch_bounds__(256) heis_rdm_reduce_kernel(const double *__restrict__ partials, int nrows,
-                                                              const HsRdmArgs a, int nout, double *__restrict__ out)
+struct HsRdmMap {
+    int16_t pair[kRdmTasks];
+};
+
+__global__ void __launch_bounds__(256) heis_rdm_reduce_kernel(const double *__restrict__ partials, int nrows, int npairs,
+                                                              const __grid_constant__ HsRdmMap map, int nout,
+                                                              double *__restrict__ out)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = blockIdx.x * 8 + warp;
     if (j >= 2 * nout) return;
-    const int q = 2 * a.map[j >> 1] + (j & 1);
+    const int q = 2 * map.pair[j >> 1] + (j & 1);
     double s = 0.0;
-    for (int b = lane; b < nrows; b += 32) s += partials[(int64_t)b * 2 * a.npairs + q];
+    for (int b = lane; b < nrows; b += 32) s += partials[(int64_t)b * 2 * npairs + q];
     s = warp_sum(s);
     if (lane == 0) out[j] = s;
 }
@@ -979,6 +1004,7 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
         return ED_ERR_RANGE;
     }
     HsRdmArgs a;
+    HsRdmMap map;     // distinct pair of each pair of the caller's list
     a.nA = h.nA;
     a.nB = h.nB;
     for (int m = 0; m <= kMaxHalf + 1; ++m) {
@@ -1003,8 +1029,8 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
         if (seen[J][K] < 0) {
             const int q = a.npairs++;
             seen[J][K] = (int16_t)q;
-            a.pj[q] = (int16_t)J;
-            a.pk[q] = (int16_t)K;
+            a.pj[q] = (int8_t)J;
+            a.pk[q] = (int8_t)K;
             const bool ja = J < h.nA, ka = K < h.nA;
             if (J != K && ja != ka) {
                 const int site = ja ? J : K, bit = ja ? 0 : 1, kb = (ja ? K : J) - h.nA;   // J up: bit 0 at an A site J
@@ -1023,7 +1049,7 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
                 if (!ja) a.bb_pair[a.nbb++] = (int16_t)q;
             }
         }
-        a.map[p] = seen[J][K];
+        map.pair[p] = seen[J][K];
     }
     a.ntask = a.nab + nother;
     // diagonal tiles: per class m, 256-column tiles times row ranges, about one per SM (a tile's sums over
@@ -1065,25 +1091,14 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
     }
     // partial rows [0, nch): flips and two-B-site sums of each chunk; [nch, nch + ntiles): the tiles
     ED_CHECK_CUDA(cudaMemsetAsync(scratch, 0, sizeof(double) * 2 * (size_t)a.npairs * (nch + ntiles), st));
-    if (a.ntask > 0) {
-        constexpr int W = kRdmThreads / 32;
-        heis_rdm_flip_kernel<T><<<dim3((unsigned)((a.ntask + W - 1) / W), (unsigned)nch), kRdmThreads, 0, st>>>(
-            bra, ket, a, h.mlo, h.mhi, scratch);
-        ED_CHECK_LAUNCH();
-    }
-    if (a.nbb > 0) {
-        const size_t smemr = (size_t)(kRdmThreads / 32) * a.nbb * sizeof(double);
-        if (smemr > 48 * 1024)
-            ED_CHECK_CUDA(cudaFuncSetAttribute(heis_rdm_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smemr));
-        heis_rdm_rows_kernel<T><<<nch, kRdmThreads, smemr, st>>>(bra, ket, a, h.mlo, h.mhi, scratch);
-        ED_CHECK_LAUNCH();
-    }
-    const size_t smemd = (size_t)(kMaxHalf + 1) * kHdThreads * sizeof(double);
-    heis_rdm_diag_kernel<T><<<ntiles, kHdThreads, smemd, st>>>(bra, ket, a, h.mlo, h.mhi,
-                                                               scratch + (int64_t)nch * 2 * a.npairs);
+    constexpr int W = kRdmThreads / 32;
+    const size_t smem = sizeof(double) * std::max((size_t)(h.nB + 1) * kHdThreads, (size_t)W * a.nbb);
+    if (smem > 48 * 1024)
+        ED_CHECK_CUDA(cudaFuncSetAttribute(heis_rdm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int nblk = ntiles + (a.nbb > 0 ? nch : 0) + (a.ntask + W - 1) / W * nch;
+    heis_rdm_kernel<T><<<nblk, kRdmThreads, smem, st>>>(bra, ket, a, h.mlo, h.mhi, ntiles, nch, scratch);
     ED_CHECK_LAUNCH();
-    heis_rdm_reduce_kernel<<<(2 * npairs + 7) / 8, 256, 0, st>>>(scratch, nch + ntiles, a, npairs, out);
+    heis_rdm_reduce_kernel<<<(2 * npairs + 7) / 8, 256, 0, st>>>(scratch, nch + ntiles, a.npairs, map, npairs, out);
     ED_CHECK_LAUNCH();
     return ED_OK;
 }
