@@ -228,6 +228,12 @@ int ed_gf_start_sites(const ed_sector *src, const ed_sector *dst, void *stream, 
 int64_t ed_lanczos_step_scratch_bytes(const ed_sector *s, int mmax);
 int ed_lanczos_step(ed_sector *s, void *stream, int dtype, int64_t ld, void *V, int64_t ldv, int k, int mmax,
                     void *w, double *state, double *alpha, double *beta, void *scratch, int64_t scratch_bytes);
+/* Steps k0 .. k1-1 of the same loop in one call (0 <= k0 < k1 <= mmax); the same vectors and scalars as
+ * k1-k0 calls of ed_lanczos_step.  ||u_k1||^2 is in the scratch at double 2(mmax+1), where a closing
+ * ed_lanczos_coef (dots = NULL) may read it. */
+int ed_lanczos_steps(ed_sector *s, void *stream, int dtype, int64_t ld, void *V, int64_t ldv, int k0, int k1,
+                     int mmax, void *w, double *state, double *alpha, double *beta, void *scratch,
+                     int64_t scratch_bytes);
 /* The reduced quantities of one state as the reference stores them: Hubbard
  * gamma (host [2][N][N], up then down, symmetric), docc (host [N], NI of
  * TWO_RDM) and sisj (host [N][N], J_SPIN) from the pairs K <= J mirrored

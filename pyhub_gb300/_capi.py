@@ -30,6 +30,7 @@ _SIGS = {
     "ed_sector_destroy": (_I, [_P]),
     "ed_lanczos_step_scratch_bytes": (_I64, [_P, _I]),
     "ed_lanczos_step": (_I, [_P, _P, _I, _I64, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _I64]),
+    "ed_lanczos_steps": (_I, [_P, _P, _I, _I64, _P, _I64, _I, _I, _I, _P, _P, _P, _P, _P, _I64]),
     "ed_rdm1_scratch_bytes": (_I64, [_P]),
     "ed_rdm1": (_I, [_P, _P, _I, _I64, _P, _P, _P, _P, _P, _I64]),
     "ed_hf_grad": (_I, [_P, _P, _I, _I64, _P, _I, _P, _P, _P, _P, _P, _I64]),
@@ -287,6 +288,15 @@ class Sector:
             self._h, _stream(stream), dtype_code(V.dtype), int(ld), _ptr(V), int(V.stride(0)), int(k), int(mmax),
             _ptr(w), _ptr(state), _ptr(alpha), _ptr(beta), _ptr(scratch),
             int(scratch.numel() * scratch.element_size())))
+
+    def lanczos_steps(self, V, k0: int, k1: int, mmax: int, w, state, alpha, beta, scratch, ld: int | None = None,
+                      stream=None):
+        """ed_lanczos_steps: steps k0 .. k1-1 as lanczos_step, in one call."""
+        ld = self.ld if ld is None else ld
+        check("ed_lanczos_steps", lib().ed_lanczos_steps(
+            self._h, _stream(stream), dtype_code(V.dtype), int(ld), _ptr(V, int(k1) * int(V.stride(0)) + self.n, "V"),
+            int(V.stride(0)), int(k0), int(k1), int(mmax), _ptr(w, self._need(ld), "w"), _ptr(state), _ptr(alpha),
+            _ptr(beta), _ptr(scratch), int(scratch.numel() * scratch.element_size())))
 
     def lanczos_step_scratch_bytes(self, mmax: int) -> int:
         return int(lib().ed_lanczos_step_scratch_bytes(self._h, int(mmax)))

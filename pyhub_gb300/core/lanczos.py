@@ -41,6 +41,7 @@ import scipy.linalg as sla
 from .. import _capi
 
 NADD = 5
+LOOKAHEAD_SMALL = 1 << 18   # vectors up to this length: a block of steps is enqueued behind a check
 
 
 def _torch():
@@ -249,14 +250,23 @@ def lanczos_full(sec, v0, max_steps: int, dtype=None, rule=None, check_every: in
     V = torch.empty((m + 1, n), dtype=dtype, device=dev)
     w = torch.zeros(n, dtype=dtype, device=dev)
     ws = _Scratch(n, m + 1, dev)
+    # whole blocks of steps go through one library call; the calls of a timed run, and of anything
+    # that only looks like a sector, are made one by one
+    native = timer is None and type(sec) is _capi.Sector
+    if native:
+        sbuf = torch.empty((sec.lanczos_step_scratch_bytes(m) + 7) // 8, dtype=torch.float64, device=dev)
+        ws.nrm = sbuf[2 * (m + 1): 2 * (m + 1) + 2]
+        if sec.kind != _capi.ED_HUBBARD and n > sec.dim:
+            V[:, sec.dim:].zero_()   # the steps work on the dim entries of a Heisenberg vector
     V[0].copy_(v0)
     _capi.multidot(V, 1, V[0], ws.dots, ws.buf)
     n0 = float(ws.dots[0].item())
     if not (n0 > 0.0 and math.isfinite(n0)):
         raise ValueError("start vector has zero or non-finite norm")
-    state = torch.zeros(_capi.lanczos_state_doubles(m), dtype=torch.float64, device=dev)
+    # alpha, beta, then the state: a check's copy is one block
+    dbl = torch.zeros(2 * m + _capi.lanczos_state_doubles(m), dtype=torch.float64, device=dev)
+    ab, state = dbl[: 2 * m].view(2, m), dbl[2 * m:]
     state[2] = 1.0 / math.sqrt(n0)
-    ab = torch.zeros((2, m), dtype=torch.float64, device=dev)   # alpha, beta
     es = V.element_size()
     k_done = 0
     converged = breakdown = False
@@ -272,15 +282,13 @@ def lanczos_full(sec, v0, max_steps: int, dtype=None, rule=None, check_every: in
         """close(k) with the copies left in flight: (k, event, host buffers)."""
         _capi.lanczos_coef(k, m, None, ws.nrm, state, None, ab[0], ab[1])
         cuda = state.is_cuda
-        hs = torch.empty(2, dtype=torch.float64, pin_memory=cuda)
-        hab = torch.empty((2, k), dtype=torch.float64, pin_memory=cuda)
-        hs.copy_(state[:2], non_blocking=cuda)
-        hab.copy_(ab[:, :k], non_blocking=cuda)
+        h = torch.empty(2 * m + 2, dtype=torch.float64, pin_memory=cuda)
+        h.copy_(dbl[: 2 * m + 2], non_blocking=cuda)
         ev = None
         if cuda:
             ev = torch.cuda.Event()
             ev.record()
-        return k, ev, hs, hab
+        return k, ev, h[2 * m:], h[: 2 * m].view(2, m)[:, :k]
 
     def judge(k, stop, alpha, beta):
         """The rule at check k: True to stop there."""
@@ -296,7 +304,36 @@ def lanczos_full(sec, v0, max_steps: int, dtype=None, rule=None, check_every: in
     pending = None
     snap = None      # (k, stop, gram, alpha, beta) of the check the run stopped at
 
-    for k in range(m):
+    # while a check is read, one more step runs; where a step is shorter than the reading, steps up to
+    # the next check (they are cheap, and the GPU would idle)
+    ahead = check_every if sec.n <= LOOKAHEAD_SMALL else 1
+    while native and k_done < m:
+        k1 = m if rule is None else min(m, max(k_done // check_every * check_every + check_every,
+                                               -(-min_steps // check_every) * check_every))
+        if pending is not None:
+            k1 = min(k1, k_done + ahead)
+        sec.lanczos_steps(V, k_done, k1, m, w, state, ab[0], ab[1], sbuf)
+        k_done = k1
+        if pending is not None:
+            kc, ev, hs, hab = pending
+            pending = None
+            ev.synchronize()
+            st_c, g_c = int(hs[0]), float(hs[1])
+            a_c, b_c = hab[0].numpy().copy(), hab[1].numpy().copy()
+            if judge(kc, st_c, a_c, b_c):
+                snap = (kc, st_c, g_c, a_c, b_c)
+                converged = st_c == 0
+                break
+        if rule is not None and k_done % check_every == 0 and k_done >= min_steps:
+            if lookahead and k_done < m:
+                pending = post(k_done)
+                continue
+            stop, gram_off, alpha, beta = close(k_done)
+            if judge(k_done, stop, alpha, beta):
+                snap = (k_done, stop, gram_off, alpha, beta)
+                converged = stop == 0
+                break
+    for k in range(k_done, m if not native else k_done):
         e = timer("hv", 2.0 * sec.dim * es) if timer is not None else None
         sec.hv(V[k], w)
         if e is not None:

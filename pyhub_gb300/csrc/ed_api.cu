@@ -25,47 +25,76 @@ static int64_t rdm1_pairs(const ed_sector *s)
 
 using namespace ed;
 
+// Scratch of a step: [dots 2(mmax+1)][nrm 2][coef mmax+1], the partial norms, then the kernels' partials.
+static int64_t step_head(int mmax)
+{
+    return ((2 * (int64_t)(mmax + 1) + 2 + (mmax + 1)) * (int64_t)sizeof(double) + 255) / 256 * 256;
+}
+
 extern "C" int64_t ed_lanczos_step_scratch_bytes(const ed_sector *s, int mmax)
 {
     if (!s || mmax < 1) return 0;
-    const int64_t head = (2 * (int64_t)(mmax + 1) + 2 + (mmax + 1)) * (int64_t)sizeof(double);
-    return (head + 255) / 256 * 256 + ed_scratch_bytes(s->nsdn * s->nsup, mmax + 1);
+    return step_head(mmax) + (int64_t)kMaxNormRows * (int64_t)sizeof(double) + ed_scratch_bytes(s->nsdn * s->nsup, mmax + 1);
 }
 
-extern "C" int ed_lanczos_step(ed_sector *s, void *stream, int dtype, int64_t ld, void *V, int64_t ldv, int k,
-                               int mmax, void *w, double *state, double *alpha, double *beta, void *scratch,
-                               int64_t scratch_bytes)
+extern "C" int ed_lanczos_steps(ed_sector *s, void *stream, int dtype, int64_t ld, void *V, int64_t ldv, int k0, int k1,
+                                int mmax, void *w, double *state, double *alpha, double *beta, void *scratch,
+                                int64_t scratch_bytes)
 {
     clear_error();
     ED_REQUIRE(s != nullptr, "sector is NULL");
     ED_REQUIRE(V != nullptr && w != nullptr && state != nullptr && alpha != nullptr && beta != nullptr &&
                    scratch != nullptr, "NULL argument");
     ED_REQUIRE(dtype == ED_F32 || dtype == ED_F64, "dtype must be ED_F32 or ED_F64");
-    ED_REQUIRE(mmax >= 1 && mmax <= 8192 && k >= 0 && k < mmax, "step k=%d outside 0..mmax-1 (mmax=%d)", k, mmax);
+    ED_REQUIRE(mmax >= 1 && mmax <= 8192 && k0 >= 0 && k0 < k1 && k1 <= mmax,
+               "steps %d..%d outside 0..mmax-1 (mmax=%d)", k0, k1 - 1, mmax);
     const int64_t need = ed_lanczos_step_scratch_bytes(s, mmax);
     ED_REQUIRE(scratch_bytes >= need, "scratch of %lld bytes is below %lld", (long long)scratch_bytes,
                (long long)need);
     const int64_t n = vec_len(s, ld);
     ED_REQUIRE(ldv >= n, "basis row stride %lld below the vector length %lld", (long long)ldv, (long long)n);
     const size_t esz = (dtype == ED_F32) ? 4 : 8;
-    // scratch: [dots 2(mmax+1)][nrm 2][coef mmax+1] then the kernels' own partials
+    ED_REQUIRE((reinterpret_cast<uintptr_t>(V) % 16) == 0 && (reinterpret_cast<uintptr_t>(w) % 16) == 0 &&
+                   ((ldv * esz) % 16) == 0, "V, w and the vector stride must be 16-byte aligned");
+    ED_REQUIRE(sizeof(double) * 16 * (size_t)k1 <= 200 * 1024, "nvec=%d too large for one pass", k1);
+    if (n == 0) return ED_OK;
     double *dots = static_cast<double *>(scratch);
     double *nrm = dots + 2 * (mmax + 1);
     double *coef = nrm + 2;
-    const int64_t head = ((2 * (int64_t)(mmax + 1) + 2 + (mmax + 1)) * (int64_t)sizeof(double) + 255) / 256 * 256;
-    void *rest = static_cast<unsigned char *>(scratch) + head;
-    const int64_t rest_bytes = scratch_bytes - head;
+    double *npart = reinterpret_cast<double *>(static_cast<unsigned char *>(scratch) + step_head(mmax));
+    double *part = npart + kMaxNormRows;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char *vb = static_cast<unsigned char *>(V);
-    const void *uk = vb + (size_t)k * (size_t)ldv * esz;
-    void *unext = vb + (size_t)(k + 1) * (size_t)ldv * esz;
-    int rc = ed_hv(s, stream, dtype, ld, uk, w, 1.0, nullptr, rest, rest_bytes);
-    if (rc) return rc;
-    rc = ed_multidot(stream, dtype, n, V, ldv, k + 1, w, uk, dots, rest, rest_bytes);
-    if (rc) return rc;
-    rc = ed_lanczos_coef(stream, k, mmax, dots, nrm, state, coef, alpha, beta);
-    if (rc) return rc;
-    return ed_update_wscaled(stream, dtype, dtype, n, V, ldv, k + 1, coef, state + 2 + k, w, unext, nrm, rest,
-                             rest_bytes);
+    const double *nsrc = nrm;    // ||u_k||^2 of the step: summed, or the previous update's partial sums
+    int nrows = 1;
+    for (int k = k0; k < k1; ++k) {
+        const void *uk = vb + (size_t)k * (size_t)ldv * esz;
+        void *unext = vb + (size_t)(k + 1) * (size_t)ldv * esz;
+        int rc = ed_hv(s, stream, dtype, ld, uk, w, 1.0, nullptr, part, ed_scratch_bytes(n, 1));
+        if (rc) return rc;
+        int rows = 0;
+        rc = launch_multidot(st, dtype, n, V, ldv, k + 1, w, uk, part, &rows);
+        if (rc) return rc;
+        // few partial rows (short vectors) are summed by the coefficient kernel itself
+        const bool direct = rows <= kCoefDotRows;
+        if (!direct) {
+            rc = launch_reduce(part, rows, 2 * (k + 1), dots, st);
+            if (rc) return rc;
+        }
+        rc = launch_coef(st, k, mmax, direct ? part : dots, direct ? rows : 1, nsrc, nrows, state, coef, alpha, beta);
+        if (rc) return rc;
+        rc = launch_update_same(st, dtype, n, V, ldv, k + 1, coef, state + 2 + k, w, unext, npart, &nrows);
+        if (rc) return rc;
+        nsrc = npart;
+    }
+    return launch_reduce(npart, nrows, 1, nrm, st);
+}
+
+extern "C" int ed_lanczos_step(ed_sector *s, void *stream, int dtype, int64_t ld, void *V, int64_t ldv, int k,
+                               int mmax, void *w, double *state, double *alpha, double *beta, void *scratch,
+                               int64_t scratch_bytes)
+{
+    return ed_lanczos_steps(s, stream, dtype, ld, V, ldv, k, k + 1, mmax, w, state, alpha, beta, scratch, scratch_bytes);
 }
 
 extern "C" int64_t ed_rdm1_scratch_bytes(const ed_sector *s)

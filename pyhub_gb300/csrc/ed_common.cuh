@@ -151,6 +151,18 @@ int heis_struct_rdm(ed_sector *s, cudaStream_t st, int dtype, const void *bra, c
                     const int32_t *pairs, double *out, double *scratch, int max_blocks);
 int launch_reduce(const double *partials, int nblocks, int m, double *out, cudaStream_t st);
 
+// The passes of a Lanczos step without their reductions (checked by the caller): the multi-dot's
+// partials [rows][2 nvec or nvec] and the update's partial norms [rows].
+constexpr int kMaxNormRows = 2048;
+int launch_multidot(cudaStream_t st, int dtype, int64_t n, const void *V, int64_t ldv, int nvec, const void *w,
+                    const void *z, double *part, int *rows);
+int launch_update_same(cudaStream_t st, int dtype, int64_t n, const void *V, int64_t ldv, int nvec, const double *coef,
+                       const double *wscale, const void *w, void *out, double *part, int *rows);
+// ed_lanczos_coef on sums that are still drows rows of dots (at most kCoefDotRows) and nrows of nrm.
+constexpr int kCoefDotRows = 16;
+int launch_coef(cudaStream_t st, int k, int mmax, const double *dots, int drows, const double *nrm, int nrows,
+                double *state, double *coef, double *alpha, double *beta);
+
 }  // namespace ed
 
 // Product space of the generic operator engine (operators.x,
@@ -219,6 +231,21 @@ __device__ __forceinline__ float warp_sumf(float v)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// Sum of n values by a CTA of 256 threads, in the order of the reduction kernels (red: 8 doubles;
+// valid in thread 0).
+__device__ __forceinline__ double sum_rows_cta(const double *__restrict__ v, int n, int stride, double *red)
+{
+    double s = 0.0;
+    for (int b = threadIdx.x; b < n; b += 256) s += v[(int64_t)b * stride];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0.0;
+    if (threadIdx.x == 0)
+        for (int q = 0; q < 8; ++q) s += red[q];
+    return s;
 }
 
 int num_sms();

@@ -374,17 +374,8 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const double *__restri
                                                           double *__restrict__ out)
 {
     __shared__ double red[8];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += 256) s += partials[(int64_t)b * m + blockIdx.x];
-    s = warp_sum(s);
-    if (lane == 0) red[warp] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s = 0.0;
-        for (int q = 0; q < 8; ++q) s += red[q];
-        out[blockIdx.x] = s;
-    }
+    const double s = sum_rows_cta(partials + blockIdx.x, nblocks, m, red);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 int launch_reduce(const double *partials, int nblocks, int m, double *out, cudaStream_t st)

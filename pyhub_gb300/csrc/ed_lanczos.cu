@@ -39,6 +39,20 @@ __host__ __device__ inline int64_t lz_work_off(int mmax) { return lz_linv_off(mm
 __host__ __device__ inline int coef_rows(int k) { return (k + 32 * kCoefCtas - 1) / (32 * kCoefCtas) * 32; }
 __host__ __device__ inline size_t coef_smem(int k) { return sizeof(double) * (2 * (size_t)(k + 1) + 2 * (size_t)coef_rows(k)); }
 
+// Sum q of the multi-dot, or of its partial rows (the pairing of launch_reduce's warp sum).
+__device__ __forceinline__ double dot_sum(const double *__restrict__ dots, int drows, int m, int q)
+{
+    if (drows == 1) return dots[q];
+    double v[kCoefDotRows];
+#pragma unroll
+    for (int r = 0; r < kCoefDotRows; ++r) v[r] = (r < drows) ? dots[(int64_t)r * m + q] : 0.0;
+#pragma unroll
+    for (int o = kCoefDotRows / 2; o >= 1; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < o; ++r) v[r] += v[r + o];
+    return v[0];
+}
+
 // One cluster of kCoefCtas CTAs.  Part 1 (every call, k >= 1): beta_{k-1} and s_k from nrm, with
 // the breakdown test of the host loop (beta <= 1e-13 max(1, |alpha|)).
 // Part 1 is idempotent: a second call for the same k with the same nrm writes
@@ -58,20 +72,34 @@ __host__ __device__ inline size_t coef_smem(int k) { return sizeof(double) * (2 
 // chain holds no sum over a whole CTA and no quotient.  One CTA with four passes took 12.2,
 // 19.2, 33.6 and 72.4 us at k = 10, 40, 100 and 200 (launch included); this form 7.9, 9.2, 10.8 and 13.9.
 __global__ void __cluster_dims__(kCoefCtas, 1, 1) __launch_bounds__(kCoefThreads)
-    lanczos_coef_kernel(int k, int mmax, const double *__restrict__ dots, const double *__restrict__ nrm, double *state,
-                        double *__restrict__ coef, double *__restrict__ alpha, double *__restrict__ beta)
+    lanczos_coef_kernel(int k, int mmax, const double *__restrict__ dots, int drows, const double *__restrict__ nrm,
+                        int nrows, double *state, double *__restrict__ coef, double *__restrict__ alpha,
+                        double *__restrict__ beta)
 {
     extern __shared__ double dyn[];
+    __shared__ double red[8];
     __shared__ double head[2];                       // s_k, stop code
     __shared__ double part[2][kCoefThreads / 32];    // per warp: l.l and l.z over the CTA's rows
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), t = threadIdx.x, lane = t & 31;
     double *s = state + 2;
     if (dots == nullptr && rank != 0) return;
+    // ||u_k||^2, or its partial sums in the order of launch_reduce
+    double nrm2 = 0.0;
+    if (nrows > 64) {
+        nrm2 = sum_rows_cta(nrm, nrows, 1, red);
+    } else if (nrows > 1) {
+        if (t < 32) {
+            for (int b = t; b < nrows; b += 32) nrm2 += nrm[b];
+            nrm2 = warp_sum(nrm2);
+        }
+    } else if (k >= 1) {
+        nrm2 = nrm[0];
+    }
     if (t == 0) {
         double stop = state[0], sk = s[k];
         if (k >= 1 && stop == 0.0) {
-            const double nb = nrm[0], pos = fmax(nb, 0.0);
+            const double nb = nrm2, pos = fmax(nb, 0.0);
             const double bk = sqrt(pos);
             if (!isfinite(nb)) {
                 stop = -(double)k;
@@ -109,9 +137,9 @@ __global__ void __cluster_dims__(kCoefCtas, 1, 1) __launch_bounds__(kCoefThreads
     long long off = 0;     // bits of the largest |G - I| entry: non-negative doubles order as integers
     for (int j = t; j <= k; j += kCoefThreads) {
         const double f = (j == k ? sk : s[j]) * sk;
-        const double gj = f * dots[k + 1 + j];
+        const double gj = f * dot_sum(dots, drows, 2 * (k + 1), k + 1 + j);
         g[j] = gj;
-        c[j] = f * dots[j];
+        c[j] = f * dot_sum(dots, drows, 2 * (k + 1), j);
         off = max(off, __double_as_longlong(fabs(j == k ? gj - 1.0 : gj)));
     }
     __syncthreads();
@@ -237,11 +265,18 @@ extern "C" int ed_lanczos_coef(void *stream, int k, int mmax, const double *dots
     ED_REQUIRE(k == 0 || nrm != nullptr, "nrm is NULL");
     ED_REQUIRE(dots == nullptr || (coef != nullptr && k < mmax), "coef is NULL or step %d has no next vector", k);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return launch_coef(st, k, mmax, dots, 1, nrm, 1, state, coef, alpha, beta);
+}
+
+int ed::launch_coef(cudaStream_t st, int k, int mmax, const double *dots, int drows, const double *nrm, int nrows,
+                    double *state, double *coef, double *alpha, double *beta)
+{
     const size_t smem = coef_smem(k);
     if (smem > 48 * 1024)
         ED_CHECK_CUDA(cudaFuncSetAttribute(lanczos_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)coef_smem(kLanczosMax)));
-    lanczos_coef_kernel<<<kCoefCtas, kCoefThreads, smem, st>>>(k, mmax, dots, nrm, state, coef, alpha, beta);
+    lanczos_coef_kernel<<<kCoefCtas, kCoefThreads, smem, st>>>(k, mmax, dots, drows, nrm, nrows, state, coef,
+                                                                alpha, beta);
     ED_CHECK_LAUNCH();
     return ED_OK;
 }

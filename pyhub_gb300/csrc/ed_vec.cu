@@ -21,7 +21,7 @@ static constexpr int kVecThreads = 256;
 static constexpr int kEPT = 16;                      // elements per thread per chunk
 static constexpr int kChunk = kVecThreads * kEPT;    // 4096 elements
 static constexpr int kMaxBlocks = 1024;
-static constexpr int kMaxNormRows = 2 * kMaxBlocks;  // partial norms that the smallest scratch holds
+static_assert(kMaxNormRows <= 2 * kMaxBlocks, "the smallest scratch holds 2 * kMaxBlocks partial norms");
 static constexpr int kVecResident = 4;               // CTAs per SM that a vector pass aims at
 
 // Four consecutive elements p[i..i+3] (zeros past n); p is 16-byte aligned and i a multiple of 4.
@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(kVecThreads) update_split_kernel(int64_t n, co
 static int64_t vec_ctas() { return std::min<int64_t>((int64_t)num_sms() * kVecResident, kMaxBlocks); }
 
 // Partial rows of the multi-dot's grid (z or not) in *rows; the partials hold rows * m doubles.
-static int launch_multidot(cudaStream_t st, int dtype, int64_t n, const void *V, int64_t ldv, int nvec, const void *w,
-                           const void *z, double *part, int *rows)
+int launch_multidot(cudaStream_t st, int dtype, int64_t n, const void *V, int64_t ldv, int nvec, const void *w,
+                    const void *z, double *part, int *rows)
 {
     const int64_t ctas = vec_ctas();
     if (dtype == ED_F32) {
@@ -386,6 +386,16 @@ static int launch_update(cudaStream_t st, int64_t n, const T *V, int64_t ldv, in
     }
     ED_CHECK_LAUNCH();
     return ED_OK;
+}
+
+int launch_update_same(cudaStream_t st, int dtype, int64_t n, const void *V, int64_t ldv, int nvec, const double *coef,
+                       const double *wscale, const void *w, void *out, double *part, int *rows)
+{
+    if (dtype == ED_F32)
+        return launch_update<float, float, float>(st, n, static_cast<const float *>(V), ldv, nvec, coef, wscale,
+                                                  static_cast<const float *>(w), static_cast<float *>(out), part, rows);
+    return launch_update<double, double, double>(st, n, static_cast<const double *>(V), ldv, nvec, coef, wscale,
+                                                 static_cast<const double *>(w), static_cast<double *>(out), part, rows);
 }
 
 }  // namespace ed
