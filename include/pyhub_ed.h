@@ -244,6 +244,15 @@ int ed_lanczos_steps(ed_sector *s, void *stream, int dtype, int64_t ld, void *V,
 int64_t ed_rdm1_scratch_bytes(const ed_sector *s);
 int ed_rdm1(ed_sector *s, void *stream, int dtype, int64_t ld, const void *psi, double *gamma, double *docc,
             double *sisj, void *scratch, int64_t scratch_bytes);
+/* MINRES for (H - e0) x = b on the complement of psi (FP64 vectors of row
+ * stride ld, row padding zero): b is projected off psi, every product too, x
+ * is returned off psi.  Stops at residual rtol * |b| or after maxiter
+ * iterations; iters and relres (host) report the count and the residual
+ * reached.  scratch: ed_minres_scratch_bytes, 16-byte aligned.  Synchronises
+ * the stream.  No reference counterpart. */
+int64_t ed_minres_scratch_bytes(const ed_sector *s, int64_t ld);
+int ed_minres(ed_sector *s, void *stream, int64_t ld, const double *psi, double e0, const double *b, double *x,
+              int maxiter, double rtol, int *iters, double *relres, void *scratch, int64_t scratch_bytes);
 /* Hellmann-Feynman gradient of <psi|H|psi> for a Hubbard sector: g_t[b] =
  * dE/dt for bond b (bonds: host int32 [2*nbonds], 1-based, t_ij = t_ji one
  * parameter) = sum_s <c+_is c_js + c+_js c_is>; g_u[i] = <n_i,up n_i,down>;

@@ -31,6 +31,8 @@ _SIGS = {
     "ed_lanczos_step_scratch_bytes": (_I64, [_P, _I]),
     "ed_lanczos_step": (_I, [_P, _P, _I, _I64, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _I64]),
     "ed_lanczos_steps": (_I, [_P, _P, _I, _I64, _P, _I64, _I, _I, _I, _P, _P, _P, _P, _P, _I64]),
+    "ed_minres_scratch_bytes": (_I64, [_P, _I64]),
+    "ed_minres": (_I, [_P, _P, _I64, _P, _D, _P, _P, _I, _D, ctypes.POINTER(_I), ctypes.POINTER(_D), _P, _I64]),
     "ed_rdm1_scratch_bytes": (_I64, [_P]),
     "ed_rdm1": (_I, [_P, _P, _I, _I64, _P, _P, _P, _P, _P, _I64]),
     "ed_hf_grad": (_I, [_P, _P, _I, _I64, _P, _I, _P, _P, _P, _P, _P, _I64]),
@@ -288,6 +290,22 @@ class Sector:
             self._h, _stream(stream), dtype_code(V.dtype), int(ld), _ptr(V), int(V.stride(0)), int(k), int(mmax),
             _ptr(w), _ptr(state), _ptr(alpha), _ptr(beta), _ptr(scratch),
             int(scratch.numel() * scratch.element_size())))
+
+    def minres(self, psi, e0: float, b, maxiter: int, rtol: float, stream=None):
+        """ed_minres: (x, iterations, relative residual) of (H - e0) x = b on the
+        complement of psi (FP64 device vectors in the internal layout)."""
+        import torch
+        if psi.dtype != torch.float64 or b.dtype != torch.float64:
+            raise TypeError("minres works in FP64")
+        nb = int(lib().ed_minres_scratch_bytes(self._h, self.ld))
+        scratch = torch.empty((nb + 7) // 8, dtype=torch.float64, device=psi.device)
+        x = torch.zeros_like(b)
+        it, rr = _I(), _D()
+        need = self.n if self.kind == ED_HUBBARD else self.dim
+        check("ed_minres", lib().ed_minres(self._h, _stream(stream), self.ld, _ptr(psi, need, "psi"), float(e0),
+                                           _ptr(b, need, "b"), _ptr(x, need, "x"), int(maxiter), float(rtol),
+                                           ctypes.byref(it), ctypes.byref(rr), _ptr(scratch), nb))
+        return x, it.value, rr.value
 
     def lanczos_steps(self, V, k0: int, k1: int, mmax: int, w, state, alpha, beta, scratch, ld: int | None = None,
                       stream=None):

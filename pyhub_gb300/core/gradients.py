@@ -153,7 +153,9 @@ def minres(apply, b, psi, maxiter: int = 2000, rtol: float = 1e-10):
     symmetric system (H - E0) x = b with b orthogonal to psi.  Every
     operator application is projected onto the complement of psi, the
     near-null direction of H - E0.  Three-term Lanczos recurrence with Givens
-    rotations of its tridiagonal: work vectors only, no stored basis."""
+    rotations of its tridiagonal: work vectors only, no stored basis.
+    For a sector's own H, Sector.minres runs the same recurrence in fused
+    kernels; this form takes any operator."""
     torch = _torch()
 
     def proj(v):
@@ -217,13 +219,7 @@ def rdm_loss_gradient(params: HubbardParams, sol: Solution, target: dict, maxite
     Apsi = torch.zeros_like(psi)
     _apply_one_body(sol, G, psi, Apsi)
     b = -2.0 * Apsi
-    work = torch.zeros_like(psi)
-
-    def apply(v):
-        sol.sector.hv(v, work)
-        return work - sol.e0 * v
-
-    lam, iters, relres = minres(apply, b, psi, maxiter=maxiter, rtol=rtol)
+    lam, iters, relres = sol.sector.minres(psi, sol.e0, b, maxiter, rtol)
     # dH/dtheta is symmetric, so <lam|dH|psi> = <psi|dH|lam>: one transition pass
     raw, _ = sol.sector.rdm_raw(lam, psi, pairs=params.pairs(), flags=1)
     return L, params.contract(raw), {"minres_iters": iters, "minres_relres": relres}
