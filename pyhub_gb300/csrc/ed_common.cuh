@@ -233,6 +233,14 @@ __device__ __forceinline__ float warp_sumf(float v)
     return v;
 }
 
+// s += v behind a warp-uniform condition: the empty statement keeps the compiler from turning the
+// branch into a select and an unconditional FP64 addition (16 clocks of an SM's FP64 pipe per warp).
+__device__ __forceinline__ void add_branch(double &s, double v)
+{
+    asm volatile("");
+    s += v;
+}
+
 // Sum of n values by a CTA of 256 threads, in the order of the reduction kernels (red: 8 doubles;
 // valid in thread 0).
 __device__ __forceinline__ double sum_rows_cta(const double *__restrict__ v, int n, int stride, double *red)

@@ -890,11 +890,12 @@ __device__ __forceinline__ void rdm_diag_tile(const T *__restrict__ bra, const T
         S = 0.0;
     };
     const int32_t *rows = a.rows_of_m + a.row_base[m];
-    for (int64_t r0 = q0r; r0 < q1r; r0 += 4) {
-        double b[4];
-        uint32_t hb[4];
+    constexpr int G = 4;                    // rows' loads in flight
+    for (int64_t r0 = q0r; r0 < q1r; r0 += G) {
+        double b[G];
+        uint32_t hb[G];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {       // four rows' loads in flight
+        for (int i = 0; i < G; ++i) {
             const bool in = r0 + i < q1r;
             const int32_t row = __ldg(rows + (in ? r0 + i : q1r - 1));
             hb[i] = __ldg(a.row_pat + row);
@@ -902,7 +903,7 @@ __device__ __forceinline__ void rdm_diag_tile(const T *__restrict__ bra, const T
             b[i] = (in && act) ? (double)__ldg(bra + at) * (double)__ldg(ket + at) : 0.0;
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < G; ++i) {
             if ((hb[i] >> lo) != run) {
                 flush();
                 run = hb[i] >> lo;
@@ -910,7 +911,7 @@ __device__ __forceinline__ void rdm_diag_tile(const T *__restrict__ bra, const T
             S += b[i];
 #pragma unroll
             for (int k = 0; k < LO; ++k)
-                if (k < lo && ((hb[i] >> k) & 1u)) Tl[k] += b[i];
+                if (k < lo && ((hb[i] >> k) & 1u)) add_branch(Tl[k], b[i]);
         }
     }
     flush();

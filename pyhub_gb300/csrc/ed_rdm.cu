@@ -23,6 +23,7 @@
 #include "ed_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace ed {
 
@@ -54,6 +55,12 @@ __device__ __forceinline__ uint32_t between_bits(int norb, int a, int b)
     return upto & ~((1u << b0) - 1u);
 }
 
+// -v where bit 31 of `flip` is set, without an FP64 instruction.
+__device__ __forceinline__ double signed_by(double v, int flip)
+{
+    return __hiloint2double(__double2hiint(v) ^ (flip & 0x80000000), __double2loint(v));
+}
+
 // ---- diagonal sums (q0 and q3 for J == K, q1 for every pair, q2 for J == K).
 // With n_u(J), n_d(J) the occupations of site J in the up and down strings and
 // b = bra*ket of an element, Sz_J = (n_u(J) - n_d(J))/2 factorises the sums
@@ -62,11 +69,16 @@ __device__ __forceinline__ uint32_t between_bits(int norb, int a, int b)
 //   sum b Sz_J Sz_K = (sum_u C n_u(J) n_u(K) - sum_u [n_u(J) T_K + n_u(K) T_J]
 //                      + sum_d W n_d(J) n_d(K)) / 4,
 //   <n_up J> = sum_u C n_u(J),  <n_down J> = sum_d W n_d(J),
-//   <n_up n_down J> = sum_u n_u(J) T_J(u),
-// so an element costs ~norb FP64 operations for all pairs at once.  A CTA
-// owns a tile of 256 columns (one per thread) and a range of rows; each
-// tile's sums are complete contributions (everything is linear in them), so
-// tiles add up without a global column array.
+//   <n_up n_down J> = sum_u n_u(J) T_J(u).
+// This kernel forms the column parts; W comes from the rows that
+// rdm_uphop_kernel stages.  A CTA owns a tile of 256 columns (one per thread)
+// and a range of rows; each tile's sums are complete contributions
+// (everything is linear in them), so tiles add up without a global column
+// array.  Bound by the FP64 pipe, so an element costs a product, one addition
+// to its run of rows (the low half of the string's bits changes only from run
+// to run, in row order) and one for every set bit of the high half (uniform
+// over the CTA): ~6 FP64 operations, where one per set bit, the column sum and
+// the row sums over the CTA were 22 (14 sites half filled: 905 -> 314 us).
 constexpr int kDiagThreads = 256;
 
 template <typename T, int MS>
@@ -77,118 +89,203 @@ __global__ void __launch_bounds__(kDiagThreads) rdm_diag_kernel(const T *__restr
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *Ts = reinterpret_cast<double *>(smem_raw);       // [MS][kDiagThreads]
     double *Cs = Ts + MS * kDiagThreads;                      // [kDiagThreads]
-    double *accW = Cs + kDiagThreads;                         // [npairs]
-    __shared__ double red[kDiagThreads / 32];
+    constexpr int H = MS / 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ncx = (int)((a.nsup + kDiagThreads - 1) / kDiagThreads);
     const int cx = blockIdx.x % ncx, ry = blockIdx.x / ncx;
     const int64_t u = (int64_t)cx * kDiagThreads + threadIdx.x;
     const bool act = u < a.nsup;
     const int64_t r0 = a.nsdn * ry / nry, r1 = a.nsdn * (ry + 1) / nry;
-    for (int q = threadIdx.x; q < a.npairs; q += blockDim.x) accW[q] = 0.0;
-    double C = 0.0, Tk[MS];
+    const int norb = a.norb, lo = norb / 2;    // bits [0, lo) per run, [lo, norb) per row
+    const uint32_t lomask = (1u << lo) - 1u;
+    double C = 0.0, S = 0.0, Tl[H], Th[H];
 #pragma unroll
-    for (int k = 0; k < MS; ++k) Tk[k] = 0.0;
-    const int norb = a.norb;
-    for (int64_t d = r0; d < r1; ++d) {
-        const uint32_t sd = __ldg(a.dstr + d);
-        const double b = act ? (double)__ldg(bra + d * a.ld + u) * (double)__ldg(ket + d * a.ld + u) : 0.0;
-        C += b;
+    for (int k = 0; k < H; ++k) Tl[k] = Th[k] = 0.0;
+    uint32_t run = 0;
+    auto flush = [&]() {
 #pragma unroll
-        for (int k = 0; k < MS; ++k)   // bit k of a string is site norb-k
-            if ((sd >> k) & 1u) Tk[k] += b;
-        // W(d): the row's sum over this tile's columns
-        double w = warp_sum(b);
-        __syncthreads();
-        if (lane == 0) red[warp] = w;
-        __syncthreads();
-        w = 0.0;
+        for (int k = 0; k < H; ++k)
+            if ((run >> k) & 1u) Tl[k] += S;
+        C += S;
+        S = 0.0;
+    };
+    constexpr int G = 4;                   // rows' loads in flight
+    for (int64_t d0 = r0; d0 < r1; d0 += G) {
+        double b[G];
+        uint32_t sd[G];
 #pragma unroll
-        for (int q = 0; q < kDiagThreads / 32; ++q) w += red[q];
-        for (int q = threadIdx.x; q < a.npairs; q += blockDim.x) {
-            const uint32_t bJ = bit_of(norb, a.pj[q]), bK = bit_of(norb, a.pk[q]);
-            if ((sd & bJ) && (sd & bK)) accW[q] += w;
+        for (int i = 0; i < G; ++i) {
+            const bool in = d0 + i < r1;
+            const int64_t d = in ? d0 + i : r1 - 1;
+            sd[i] = __ldg(a.dstr + d);
+            b[i] = (in && act) ? (double)__ldg(bra + d * a.ld + u) * (double)__ldg(ket + d * a.ld + u) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            if ((sd[i] & lomask) != run) {
+                flush();
+                run = sd[i] & lomask;
+            }
+            S += b[i];
+#pragma unroll
+            for (int k = 0; k < H; ++k)     // (a string has no bit past norb)
+                if ((sd[i] >> (lo + k)) & 1u) add_branch(Th[k], b[i]);
         }
     }
+    flush();
 #pragma unroll
-    for (int k = 0; k < MS; ++k) Ts[k * kDiagThreads + threadIdx.x] = Tk[k];
+    for (int k = 0; k < H; ++k) {
+        if (k < lo) Ts[k * kDiagThreads + threadIdx.x] = Tl[k];
+        if (lo + k < norb) Ts[(lo + k) * kDiagThreads + threadIdx.x] = Th[k];
+    }
     Cs[threadIdx.x] = C;
     __syncthreads();
-    // per pair: sums over the tile's columns (warp w takes pairs w, w+8, ...)
+    // per pair: sums over the tile's columns (warp w takes pairs w, w+8, ...); a column past nsup holds zeros
+    constexpr int NC = kDiagThreads / 32;
+    uint32_t su[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) su[i] = __ldg(a.ustr + min((int64_t)cx * kDiagThreads + i * 32 + lane, a.nsup - 1));
     for (int q = warp; q < a.npairs; q += kDiagThreads / 32) {
         const int J = a.pj[q], K = a.pk[q];
         const uint32_t bJ = bit_of(norb, J), bK = bit_of(norb, K);
-        const int kJ = norb - J, kK = norb - K;   // bit positions
-        double s_cc = 0.0, s_ct = 0.0, s_c = 0.0, s_t = 0.0;
-        for (int t = lane; t < kDiagThreads; t += 32) {
-            const int64_t uu = (int64_t)cx * kDiagThreads + t;
-            if (uu >= a.nsup) continue;
-            const uint32_t su = __ldg(a.ustr + uu);
-            const double nJ = (su & bJ) ? 1.0 : 0.0, nK = (su & bK) ? 1.0 : 0.0;
-            const double c = Cs[t];
-            s_cc += nJ * nK * c;
-            s_ct += nJ * Ts[kK * kDiagThreads + t] + nK * Ts[kJ * kDiagThreads + t];
-            s_c += nJ * c;
-            s_t += nJ * Ts[kJ * kDiagThreads + t];
+        const double *TJ = Ts + (norb - J) * kDiagThreads, *TK = Ts + (norb - K) * kDiagThreads;
+        double s_c = 0.0, s_t = 0.0;     // sum C n_u(J) n_u(K);  sum n_u(J) T_K + n_u(K) T_J (J == K: once)
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            const int t = i * 32 + lane;
+            const bool nJ = (su[i] & bJ) != 0, nK = (su[i] & bK) != 0;
+            s_c += (nJ && nK) ? Cs[t] : 0.0;
+            s_t += nJ ? TK[t] : 0.0;
+            if (J != K) s_t += nK ? TJ[t] : 0.0;
         }
-        s_cc = warp_sum(s_cc);
-        s_ct = warp_sum(s_ct);
         s_c = warp_sum(s_c);
         s_t = warp_sum(s_t);
         if (lane == 0) {
             double *o = partials + ((int64_t)blockIdx.x * a.npairs + q) * 4;
-            const double wq = accW[q];
             o[0] = (J == K) ? s_c : 0.0;
-            o[1] = 0.25 * (s_cc - s_ct + wq);
-            o[2] = (J == K) ? wq : 0.0;
+            o[1] = 0.25 * (s_c - (J == K ? 2.0 * s_t : s_t));
+            o[2] = 0.0;
             o[3] = (J == K) ? s_t : 0.0;
         }
     }
 }
 
+// R values of one string (staged side by side).
+template <typename T, int R> __device__ __forceinline__ void load_rows(const T *p, T (&v)[R])
+{
+    if constexpr (R * sizeof(T) >= 16) {
+        constexpr int N = 16 / sizeof(T);
+        using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+#pragma unroll
+        for (int q = 0; q < R / N; ++q) {
+            const V w = reinterpret_cast<const V *>(p)[q];
+#pragma unroll
+            for (int k = 0; k < N; ++k) v[q * N + k] = reinterpret_cast<const T *>(&w)[k];
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = p[r];
+    }
+}
+
 // ---- up hops within a row (q0 for J != K): for each pair, the strings of
-// its list, sum sign * bra[d][u] * ket[d][u'].  Rows are staged in shared
-// memory; warp w takes pairs w, w+8, ...; per-pair sums accumulate in shared
-// memory over the CTA's rows.
-template <typename T>
-__global__ void __launch_bounds__(256) rdm_uphop_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
-                                                        const RdmArgs a, double *__restrict__ partials)
+// its list, sum sign * bra[d][u] * ket[d][u'], and the row sums W(d) of the
+// diagonal quantities (q1, q2).  R rows are staged side by side in shared
+// memory, so one list entry, one pair of gathers and one sum over the lanes
+// serve R rows; warps over pairs; per-pair sums accumulate in shared memory
+// over the CTA's rows.  Bound by the FP64 pipe: one FMA per entry and row
+// (the sign goes in without one): 14 sites half filled, K <= J, 1,300 us with
+// one row at a time -> 570 us (floor 458).
+constexpr int kUphopThreads = 512;
+
+template <typename T, int R>
+__global__ void __launch_bounds__(kUphopThreads) rdm_uphop_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
+                                                                  const RdmArgs a, double *__restrict__ partials)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *acc = reinterpret_cast<double *>(smem_raw);          // [npairs]
-    T *bs = reinterpret_cast<T *>(acc + a.npairs);
+    double *acc = reinterpret_cast<double *>(smem_raw);          // [npairs], padded to 16 bytes
+    constexpr int NQ = kMaxPairs / kUphopThreads;
+    double accW[NQ];                                              // row sums of pairs threadIdx.x, + kUphopThreads
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) accW[i] = 0.0;
+    __shared__ double W[R];
+    T *bs = reinterpret_cast<T *>(acc + (a.npairs + 1) / 2 * 2);  // [nsup][R]
     const bool same = (bra == ket);
-    T *ks = same ? bs : bs + a.nsup;
+    T *ks = same ? bs : bs + (int64_t)a.nsup * R;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nsup = (int)a.nsup;
     for (int q = threadIdx.x; q < a.npairs; q += blockDim.x) acc[q] = 0.0;
-    for (int64_t d = blockIdx.x; d < a.nsdn; d += gridDim.x) {
+    for (int64_t d0 = (int64_t)blockIdx.x * R; d0 < a.nsdn; d0 += (int64_t)gridDim.x * R) {
         __syncthreads();
-        for (int64_t i = threadIdx.x; i < a.nsup; i += blockDim.x) {
-            bs[i] = bra[d * a.ld + i];
-            if (!same) ks[i] = ket[d * a.ld + i];
+        for (int i = threadIdx.x; i < nsup; i += blockDim.x) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const bool in = d0 + r < a.nsdn;
+                bs[i * R + r] = in ? bra[(d0 + r) * a.ld + i] : (T)0;
+                if (!same) ks[i * R + r] = in ? ket[(d0 + r) * a.ld + i] : (T)0;
+            }
         }
         __syncthreads();
-        for (int q = warp; q < a.npairs; q += 8) {
+        for (int task = warp; task < a.npairs + R; task += kUphopThreads / 32) {
+            if (task < R) {
+                double w = 0.0;
+                for (int i = lane; i < nsup; i += 32) w = fma((double)bs[i * R + task], (double)ks[i * R + task], w);
+                w = warp_sum(w);
+                if (lane == 0) W[task] = w;
+                continue;
+            }
+            const int q = task - R;
             const int J = a.pj[q], K = a.pk[q];
             if (J == K) continue;
             const int pid = (J - 1) * a.norb + (K - 1);
             const int e0 = __ldg(a.upl_off + pid), e1 = __ldg(a.upl_off + pid + 1);
             double s = 0.0;
+#pragma unroll 2
             for (int e = e0 + lane; e < e1; e += 32) {
                 const int2 en = __ldg(a.upl_ent + e);
-                const double b = (double)bs[en.x];
-                s = fma((en.y < 0) ? -b : b, (double)ks[en.y & 0x7fffffff], s);   // one FP64 op per entry
+                T x[R], y[R];
+                load_rows<T, R>(bs + en.x * R, x);
+                load_rows<T, R>(ks + (en.y & 0x7fffffff) * R, y);
+#pragma unroll
+                for (int r = 0; r < R; ++r) s = fma(signed_by((double)x[r], en.y), (double)y[r], s);
             }
             s = warp_sum(s);
             if (lane == 0) acc[q] += s;
         }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            const int q = threadIdx.x + i * kUphopThreads;
+            if (q >= a.npairs) break;
+            const uint32_t both = bit_of(a.norb, a.pj[q]) | bit_of(a.norb, a.pk[q]);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (d0 + r < a.nsdn && (__ldg(a.dstr + d0 + r) & both) == both) accW[i] += W[r];
+        }
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < a.npairs; q += blockDim.x) {
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        const int q = threadIdx.x + i * kUphopThreads;
+        if (q >= a.npairs) break;
         double *o = partials + ((int64_t)blockIdx.x * a.npairs + q) * 4;
         o[0] = acc[q];
-        o[1] = o[2] = o[3] = 0.0;
+        o[1] = 0.25 * accW[i];
+        o[2] = (a.pj[q] == a.pk[q]) ? accW[i] : 0.0;
+        o[3] = 0.0;
     }
+}
+
+template <typename T, int R>
+static int launch_uphop(cudaStream_t st, const T *bra, const T *ket, const RdmArgs &a, int nsm, int maxblk, double *part,
+                        int *rows)
+{
+    const size_t smem = (size_t)(a.npairs + 1) / 2 * 16 + (size_t)(bra == ket ? 1 : 2) * R * a.nsup * sizeof(T);
+    ED_CHECK_CUDA(cudaFuncSetAttribute(rdm_uphop_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    *rows = (int)std::min<int64_t>((a.nsdn + R - 1) / R, std::min(4 * nsm, maxblk));
+    rdm_uphop_kernel<T, R><<<*rows, kUphopThreads, smem, st>>>(bra, ket, a, part);
+    ED_CHECK_LAUNCH();
+    return ED_OK;
 }
 
 // ---- sums across rows (q4: down hop J->K of the row; q5: up hop J->K with
@@ -220,7 +317,8 @@ __global__ void __launch_bounds__(256) rdm_cross_kernel(const T *__restrict__ br
                 const int64_t r = rank_holes(a.lut, holes_dev(sd - bJ + bK, a.norb));
                 const T *k2 = ket + r * a.ld;
                 double s = 0.0;
-                for (int64_t u = lane; u < a.nsup; u += 32) s += (double)bs[u] * (double)__ldg(k2 + u);
+#pragma unroll 4
+                for (int u = lane; u < (int)a.nsup; u += 32) s = fma((double)bs[u], (double)__ldg(k2 + u), s);
                 s = warp_sum(s);
                 if (lane == 0) acc[2 * q] += (__popc(sd & btw) & 1) ? -s : s;
             }
@@ -230,10 +328,10 @@ __global__ void __launch_bounds__(256) rdm_cross_kernel(const T *__restrict__ br
                 const int pid = (J - 1) * a.norb + (K - 1);
                 const int e0 = __ldg(a.upl_off + pid), e1 = __ldg(a.upl_off + pid + 1);
                 double s = 0.0;
+#pragma unroll 4
                 for (int e = e0 + lane; e < e1; e += 32) {
                     const int2 en = __ldg(a.upl_ent + e);
-                    const double b = (double)bs[en.x];
-                    s = fma((en.y < 0) ? -b : b, (double)__ldg(k2 + (en.y & 0x7fffffff)), s);
+                    s = fma(signed_by((double)bs[en.x], en.y), (double)__ldg(k2 + (en.y & 0x7fffffff)), s);
                 }
                 s = warp_sum(s);
                 if (lane == 0) acc[2 * q + 1] -= (__popc(sd & btw) & 1) ? -s : s;
@@ -264,20 +362,20 @@ static int rdm_hub(ed_sector *s, cudaStream_t st, int64_t ld, const T *bra, cons
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     nsm = std::max(nsm, 1);
-    // ---- row-local sums: diagonal tiles then up-hop rows, their partials stacked for one reduction.
-    // Each pass gets a few CTAs per SM (both are bound by the FP64 pipe of every SM they occupy);
-    // the partial rows of the two together stay within kRdmRows.
+    // ---- row-local sums: diagonal tiles then up-hop rows, their partials stacked for one reduction;
+    // the partial rows of the two together stay within kRdmRows.  About one diagonal tile per SM: a
+    // tile's sums over the pairs cost more than a few rows more or less.
     constexpr int kMaxTiles = kRdmRows / 2;
     const int ncx = (int)((s->nsup + kDiagThreads - 1) / kDiagThreads);
     if (ncx > kMaxTiles) { set_error("rows of %lld strings are too long for the RDM tiles", (long long)s->nsup); return ED_ERR_RANGE; }
-    int nry = (int)std::max<int64_t>(1, std::min<int64_t>(s->nsdn, std::min(2 * nsm, kMaxTiles) / ncx));
+    int nry = (int)std::max<int64_t>(1, std::min<int64_t>(s->nsdn, std::min(nsm, kMaxTiles) / ncx));
     if (ncx * nry > kMaxTiles) nry = std::max(1, kMaxTiles / ncx);
     const int nbA = ncx * nry;
     const bool small = s->norb <= 16;
-    const size_t smemA = (size_t)((small ? 16 : 32) + 1) * kDiagThreads * sizeof(double) + (size_t)npairs * sizeof(double);
-    const int nbB = (int)std::min<int64_t>(s->nsdn, std::min(4 * nsm, kRdmRows - nbA));
-    const size_t smemB = (size_t)npairs * sizeof(double) + (size_t)(bra == ket ? 1 : 2) * s->nsup * sizeof(T);
-    if (smemA > (size_t)maxsm || smemB > (size_t)maxsm) {
+    const size_t smemA = (size_t)((small ? 16 : 32) + 1) * kDiagThreads * sizeof(double);
+    const int nvec = bra == ket ? 1 : 2;
+    const size_t row = (size_t)nvec * s->nsup * sizeof(T), headB = (size_t)(npairs + 1) / 2 * 16;
+    if (smemA > (size_t)maxsm || headB + row > (size_t)maxsm) {
         set_error("RDM pass of %lld strings exceeds shared memory", (long long)s->nsup);
         return ED_ERR_RANGE;
     }
@@ -290,12 +388,17 @@ static int rdm_hub(ed_sector *s, cudaStream_t st, int64_t ld, const T *bra, cons
         rdm_diag_kernel<T, 32><<<nbA, kDiagThreads, smemA, st>>>(bra, ket, a, nry, part1);
     }
     ED_CHECK_LAUNCH();
-    if (nbB > 0) {
-        ED_CHECK_CUDA(cudaFuncSetAttribute(rdm_uphop_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemB));
-        rdm_uphop_kernel<T><<<nbB, 256, smemB, st>>>(bra, ket, a, part1 + (int64_t)nbA * 4 * npairs);
-        ED_CHECK_LAUNCH();
+    // four rows at a time where two CTAs of them fit an SM and there are rows for all SMs, else two, else one
+    int nbB = 0, rc = ED_OK;
+    if (s->nsdn > 0) {
+        double *pB = part1 + (int64_t)nbA * 4 * npairs;
+        auto fits = [&](int R) { return headB + R * row <= (size_t)maxsm / 2 && s->nsdn >= (int64_t)R * nsm; };
+        if (fits(4)) rc = launch_uphop<T, 4>(st, bra, ket, a, nsm, kRdmRows - nbA, pB, &nbB);
+        else if (fits(2)) rc = launch_uphop<T, 2>(st, bra, ket, a, nsm, kRdmRows - nbA, pB, &nbB);
+        else rc = launch_uphop<T, 1>(st, bra, ket, a, nsm, kRdmRows - nbA, pB, &nbB);
+        if (rc) return rc;
     }
-    int rc = launch_reduce(part1, nbA + std::max(nbB, 0), 4 * npairs, out, st);
+    rc = launch_reduce(part1, nbA + nbB, 4 * npairs, out, st);
     if (rc) return rc;
     const int want_dn = (flags & 1) ? 1 : 0, want_sx = (flags & 2) ? 1 : 0;
     if (want_dn || want_sx) {
