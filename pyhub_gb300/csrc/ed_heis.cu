@@ -201,6 +201,7 @@ int heis_struct_build(ed_sector *s)
     double ab_zz_sum = 0.0;   // sum of zz/4 over the A-B bonds (every bond taken as "equal")
     for (int b : ab) ab_zz_sum += 0.25 * ht.zz[b];
     std::vector<uint32_t> col_abbits, row_bbits;
+    std::vector<double> ab_lut;
     std::vector<int32_t> ab_rank;   // [q][column]: rank of the column's pattern with the bond's A bit flipped
     if (hs->ab_fast) {
         ab_rank.resize(ab.size() * col_pat.size());
@@ -208,6 +209,12 @@ int heis_struct_build(ed_sector *s)
             for (size_t c = 0; c < col_pat.size(); ++c)
                 ab_rank[q * col_pat.size() + c] = rankA[col_pat[c] ^ (1u << (ht.bj[ab[q]] - 1))];
         hs->ncols = (int64_t)col_pat.size();
+        if (!ab.empty()) ab_lut.assign(4 * 256, 0.0);
+        for (size_t k = 0; k < ab_lut.size(); ++k)
+            for (size_t q = 0; q < 8; ++q) {
+                const size_t bond = k / 256 * 8 + q;
+                if (bond < ab.size() && ((k >> q) & 1)) ab_lut[k] += 0.5 * ht.zz[ab[bond]];
+            }
         col_abbits.resize(col_pat.size());
         for (size_t c = 0; c < col_pat.size(); ++c) {
             uint32_t w = 0;
@@ -276,7 +283,7 @@ int heis_struct_build(ed_sector *s)
         (rc = up(&hs->bb_cf64, bb_cf)) || (rc = up(&hs->rows_of_m, rows_of_m)) ||
         (rc = up(&hs->aa_pk32, aa_pk32)) || (rc = up(&hs->col_abbits, col_abbits)) ||
         (rc = up(&hs->row_bbits, row_bbits)) || (rc = up(&hs->diagA32, diagA32)) || (rc = up(&hs->ab_rank, ab_rank)) ||
-        (rc = up(&hs->diagB32, diagB32)))
+        (rc = up(&hs->diagB32, diagB32)) || (rc = up(&hs->ab_lut, ab_lut)))
         return rc;
     return ED_OK;
 }
@@ -287,7 +294,8 @@ void heis_struct_free(HeisStruct *hs)
     void *ptrs[] = {hs->col_pat, hs->rankA, hs->diagA, hs->aa_off, hs->aa_src, hs->aa_cf32,
                     hs->aa_cf64, hs->row_pat, hs->row_m, hs->row_off, hs->rowidx, hs->diagB,
                     hs->bb_ptr, hs->bb_src, hs->bb_cf32, hs->bb_cf64, hs->rows_of_m,
-                    hs->aa_pk32, hs->col_abbits, hs->row_bbits, hs->diagA32, hs->diagB32, hs->ab_rank};
+                    hs->aa_pk32, hs->col_abbits, hs->row_bbits, hs->diagA32, hs->diagB32, hs->ab_rank,
+                    hs->ab_lut};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete hs;
@@ -307,12 +315,22 @@ struct HsArgs {
     const int2 *aa_pk32;           // {column, FP32 coefficient bits} of the A-A flips
     const uint32_t *col_abbits, *row_bbits;
     const int32_t *ab_rank;        // [q][column] rank after flipping bond q's A bit (packed path)
+    const double *ab_lut;
     int64_t ncols;
     int ab_fast;
     int8_t ab_pa[kMaxAB], ab_pb[kMaxAB];
     double ab_fjk[kMaxAB], ab_fkj[kMaxAB], ab_zz[kMaxAB];
     double scale;
+    int8_t m_order[kMaxHalf + 1];  // the hole counts of A by falling row length
+    int by_length;                 // one-row pass: rows in that order, else in the vector's
 };
+
+// Work item `at` of a CTA's walk in round k: rounds alternate in direction over items sorted by falling
+// length, so that the CTAs' sums of lengths stay close.
+__device__ __forceinline__ int64_t zigzag(int64_t k)
+{
+    return k * gridDim.x + ((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+}
 
 constexpr int kHeisRowThreads = 512;
 
@@ -340,9 +358,28 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
     const T *acf = reinterpret_cast<const T *>(a.aa_cf);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kHeisRowThreads / 32;
     const T sc = (T)a.scale;
-    for (int64_t row = blockIdx.x; row < a.nrows; row += gridDim.x) {
+    constexpr bool kLut = sizeof(T) == 8;
+    for (int64_t k = 0; k * gridDim.x < a.nrows; ++k) {
+        int m;
+        int64_t row;
+        if (a.by_length) {
+            int64_t g = zigzag(k);
+            if (g >= a.nrows) continue;
+            int o = 0;
+            m = a.m_order[0];
+            for (;;) {
+                const int64_t nr_m = a.row_base[m + 1] - a.row_base[m];
+                if (g < nr_m) break;
+                g -= nr_m;
+                m = a.m_order[++o];
+            }
+            row = __ldg(a.rows_of_m + a.row_base[m] + g);
+        } else {
+            row = k * gridDim.x + blockIdx.x;
+            if (row >= a.nrows) continue;
+            m = __ldg(a.row_m + row);
+        }
         const uint32_t hb = __ldg(a.row_pat + row);
-        const int m = __ldg(a.row_m + row);
         const int64_t off = __ldg(a.row_off + row);
         const int len = (int)a.ncol[m];
         const int64_t cbase = a.col_base[m];
@@ -390,10 +427,13 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
                 // antiparallel A-B bonds: the set bits of (column's A bits ^ row's B bits); their
                 // zz/4 was counted as "equal" in diagB, so each one drops the diagonal by zz/2
                 uint32_t diff = __ldg(a.col_abbits + cbase + cc) ^ rbits;
+                // FP64 (bound by the FP64 pipe): eight bonds' zz drops from a table, one subtraction for them
+                if (kLut)
+                    for (int g = 0; g * 8 < a.nab; ++g) d -= (T)__ldg(a.ab_lut + g * 256 + ((diff >> (8 * g)) & 255u));
                 while (diff) {
                     const int q = __ffs(diff) - 1;
                     diff &= diff - 1;
-                    d -= ab_w2[q];
+                    if (!kLut) d -= ab_w2[q];
                     const int64_t src = ab_src[q];
                     if (src >= 0) acc += ab_c[q] * __ldg(x + src + __ldg(a.ab_rank + q * a.ncols + cbase + cc));
                 }
@@ -408,7 +448,8 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
                 const int64_t src = ab_src[q];
                 if (src >= 0) acc += ab_c[q] * __ldg(x + src + __ldg(a.rankA + (ha ^ (1u << a.ab_pa[q]))));
             }
-            if (ok) y[off + c] = (d * xs[cc] + acc) * sc;
+            const T v = d * xs[cc] + acc;
+            if (ok) y[off + c] = (sc == (T)1) ? v : v * sc;
         }
     }
 }
@@ -451,6 +492,10 @@ __device__ __forceinline__ void heis_col4_group(const HsArgs &a, int at, const f
 // four rows.  Each row's sums are the one-row kernel's, in its order (slots,
 // then the antiparallel A-B bonds in increasing order), so the product is the same.
 // Work items are groups of four rows of rows_of_m, hole count by hole count.
+// Bound by the latency of its loads: the A-B bonds' dependent pair (rank of the
+// flipped column, then the element) goes four bonds at a time, up to 16
+// elements in flight (one bond at a time: 4x7 957 us, now 600); two CTAs per SM
+// where their rows fit.
 __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(const float *__restrict__ x,
                                                                           float *__restrict__ y, const HsArgs a,
                                                                           int64_t nitems)
@@ -460,17 +505,18 @@ __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(cons
     float *ab_c = reinterpret_cast<float *>(ab_src + 4 * a.nab);   // [4][nab] flip element
     float *ab_w2 = ab_c + 4 * a.nab;                               // [nab] zz/2: drop of an antiparallel bond
     float4 *xs4 = reinterpret_cast<float4 *>(smem_raw + heis_col4_head_bytes(a.nab));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kHeisCol4Threads / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const float sc = (float)a.scale;
     const float *dA32 = static_cast<const float *>(a.diagA), *dB32 = static_cast<const float *>(a.diagB);
-    for (int64_t it = blockIdx.x; it < nitems; it += gridDim.x) {
-        int m = 0;
-        int64_t g = it;
+    for (int64_t k = 0; k * gridDim.x < nitems; ++k) {
+        int64_t g = zigzag(k);
+        if (g >= nitems) continue;
+        int o = 0, m = a.m_order[0];
         for (;;) {
             const int64_t ng = (a.row_base[m + 1] - a.row_base[m] + 3) / 4;
             if (g < ng) break;
             g -= ng;
-            ++m;
+            m = a.m_order[++o];
         }
         const int nr = (int)min((int64_t)4, a.row_base[m + 1] - a.row_base[m] - 4 * g);
         int64_t off[4];
@@ -496,8 +542,8 @@ __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(cons
                 else dst[r] = 0.f;
             }
         }
-        for (int k = threadIdx.x; k < 4 * a.nab; k += blockDim.x) {
-            const int r = k / a.nab, q = k - r * a.nab;
+        for (int t = threadIdx.x; t < 4 * a.nab; t += blockDim.x) {
+            const int r = t / a.nab, q = t - r * a.nab;
             int64_t src = -1;
             float cf = 0.f;
             if (r < nr) {
@@ -507,8 +553,8 @@ __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(cons
                 src = (r2 >= 0) ? __ldg(a.row_off + r2) : (int64_t)-1;
                 cf = (float)(hk ? a.ab_fkj[q] : a.ab_fjk[q]);
             }
-            ab_src[k] = src;
-            ab_c[k] = cf;
+            ab_src[t] = src;
+            ab_c[t] = cf;
             if (r == 0) ab_w2[q] = (float)(2.0 * a.ab_zz[q]);
         }
         cp_async_wait_all();
@@ -540,17 +586,33 @@ __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(cons
                 diff[r] = (r < nr) ? (ca ^ rbits[r]) : 0u;
                 any |= diff[r];
             }
-            while (any) {
-                const int q = __ffs(any) - 1;
-                any &= any - 1;
-                const int rk = __ldg(a.ab_rank + q * a.ncols + cbase + cc);
+            // four bonds at a time: their ranks, then their up to 16 source elements, are in flight together
+            for (int q0 = 0; q0 < a.nab; q0 += 4) {
+                const uint32_t any4 = (any >> q0) & 15u;
+                if (!any4) continue;
+                int rk[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    if (!((diff[r] >> q) & 1u)) continue;
-                    d[r] -= ab_w2[q];
-                    const int64_t src = ab_src[r * a.nab + q];
-                    if (src >= 0) acc[r] += ab_c[r * a.nab + q] * __ldg(x + src + rk);
-                }
+                for (int i = 0; i < 4; ++i)
+                    rk[i] = ((any4 >> i) & 1u) ? __ldg(a.ab_rank + (int64_t)(q0 + i) * a.ncols + cbase + cc) : 0;
+                float v[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        v[i][r] = 0.f;
+                        if ((diff[r] >> (q0 + i)) & 1u) {
+                            const int64_t src = ab_src[r * a.nab + q0 + i];
+                            if (src >= 0) v[i][r] = __ldg(x + src + rk[i]);
+                        }
+                    }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if ((diff[r] >> (q0 + i)) & 1u) {
+                            d[r] -= ab_w2[q0 + i];
+                            acc[r] += ab_c[r * a.nab + q0 + i] * v[i][r];
+                        }
             }
             if (ok) {
                 const float4 xv = xs4[cc];
@@ -608,8 +670,49 @@ __global__ void __launch_bounds__(256) heis_slab_kernel(const T *__restrict__ x,
             }
             const bool last = eb + 32 >= nn;
             T sxy = 0, syy = 0;
-            // four 32-column chunks per pass: four independent loads per neighbour row
-            for (int64_t cb = c0; cb < c1; cb += 128) {
+            // four 32-column chunks per pass.  Bound by L2 latency (rows start at any element, so a load is
+            // 4 or 8 bytes per lane): a pass that lies inside the row issues the loads of G neighbour rows,
+            // 4 G of them, before the first sum (4x7 FP32: 584 us with one row's loads, 274 with four rows').
+            constexpr int G = sizeof(T) == 4 ? 4 : 2;
+            int64_t cb = c0;
+            for (; cb + 128 <= c1; cb += 128) {
+                const T *xc = x + cb + lane;
+                T *yc = y + off + cb + lane;
+                T acc[4] = {0, 0, 0, 0}, yv[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) yv[j] = yc[32 * j];
+                int e = 0;
+                for (; e + G <= ne; e += G) {
+                    T v[G][4], w[G];
+#pragma unroll
+                    for (int i = 0; i < G; ++i) {
+                        const int64_t so = __shfl_sync(0xffffffffu, my_off, e + i);
+                        w[i] = __shfl_sync(0xffffffffu, my_cf, e + i);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) v[i][j] = __ldg(xc + so + 32 * j);
+                    }
+#pragma unroll
+                    for (int i = 0; i < G; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[j] += w[i] * v[i][j];
+                }
+                for (; e < ne; ++e) {
+                    const int64_t so = __shfl_sync(0xffffffffu, my_off, e);
+                    const T w = __shfl_sync(0xffffffffu, my_cf, e);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[j] += w * __ldg(xc + so + 32 * j);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    yv[j] += acc[j] * sc;
+                    yc[32 * j] = yv[j];
+                    if (last && partials) {
+                        sxy += x[off + cb + lane + 32 * j] * yv[j];
+                        syy += yv[j] * yv[j];
+                    }
+                }
+            }
+            if (cb < c1) {
                 T acc[4] = {0, 0, 0, 0};
 #pragma unroll 2
                 for (int e = 0; e < ne; ++e) {
@@ -627,7 +730,7 @@ __global__ void __launch_bounds__(256) heis_slab_kernel(const T *__restrict__ x,
                     if (c < c1) {
                         const T yv = y[off + c] + acc[j] * sc;
                         y[off + c] = yv;
-                        if (last) {
+                        if (last && partials) {
                             sxy += x[off + c] * yv;
                             syy += yv * yv;
                         }
@@ -1145,6 +1248,7 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     a.col_abbits = h.col_abbits;
     a.row_bbits = h.row_bbits;
     a.ab_rank = h.ab_rank;
+    a.ab_lut = h.ab_lut;
     a.ncols = h.ncols;
     a.ab_fast = h.ab_fast ? 1 : 0;
     a.bb_cf = (sizeof(T) == 4) ? (const void *)h.bb_cf32 : (const void *)h.bb_cf64;
@@ -1153,6 +1257,11 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
         a.ab_fjk[q] = h.ab_fjk[q]; a.ab_fkj[q] = h.ab_fkj[q]; a.ab_zz[q] = h.ab_zz[q];
     }
     a.scale = scale;
+    for (int m = 0; m <= h.nA; ++m) a.m_order[m] = (int8_t)m;
+    std::sort(a.m_order, a.m_order + h.nA + 1, [&](int8_t x, int8_t y) { return h.ncol[x] > h.ncol[y]; });
+    // rows by length give the CTAs even shares (FP64: 4x6 157 -> 149 us, 4x7 3.69 -> 3.51 ms); vectors far
+    // above L2 keep memory order, where the A-B bonds' source rows are near (4x8: 60 ms, by length 67)
+    a.by_length = (double)s->dim * sizeof(T) <= 1.0e9 ? 1 : 0;
     const int nsm = num_sms();
     // ---- pass R
     int maxsm = 0;
@@ -1170,12 +1279,14 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
         for (int m = 0; m <= h.nA; ++m) nitems += (h.row_base[m + 1] - h.row_base[m] + 3) / 4;
         ED_CHECK_CUDA(cudaFuncSetAttribute(heis_row_col4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem4));
+        // two CTAs of 512 threads per SM where two groups of rows fit (one stages while the other works)
+        const int threads = 2 * (smem4 + 1024) <= (size_t)maxsm ? 512 : kHeisCol4Threads;
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, heis_row_col4_kernel, kHeisCol4Threads, smem4);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, heis_row_col4_kernel, threads, smem4);
         if (per_sm < 1) per_sm = 1;
         int64_t blocks = std::min<int64_t>(nitems, (int64_t)nsm * per_sm);
         if (blocks < 1) blocks = 1;
-        heis_row_col4_kernel<<<(unsigned)blocks, kHeisCol4Threads, smem4, st>>>(
+        heis_row_col4_kernel<<<(unsigned)blocks, threads, smem4, st>>>(
             reinterpret_cast<const float *>(x), reinterpret_cast<float *>(y), a, nitems);
     } else {
         const size_t smem = heis_row_head_bytes(h.nab, sizeof(T)) + (size_t)std::max<int64_t>(h.max_len, 1) * sizeof(T);
@@ -1185,18 +1296,26 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
         heis_row_kernel<T><<<(unsigned)blocks, kHeisRowThreads, smem, st>>>(x, y, a);
     }
     ED_CHECK_LAUNCH();
-    // ---- pass S
+    // ---- pass S: one wave of resident CTAs walks the items (slab, eight rows).  A slab takes at most
+    // ~48 MB of L2; small sectors cut the columns further, down to one pass of 128, until every CTA
+    // has several items (a share of 3.4 items each would leave a wave 15% empty).
     SlabPlan p;
     p.nblk = 0;
     p.item_base[0] = 0;
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, heis_slab_kernel<T>, 256, 0);
+    int64_t blocks2 = std::min<int64_t>((int64_t)nsm * std::max(per_sm, 1), kMaxPartialBlocksHeis);
+    int64_t groups = 0;
+    for (int m = 0; m <= h.nA; ++m) groups += (h.row_base[m + 1] - h.row_base[m] + 7) / 8;
+    const int64_t cuts = std::max<int64_t>(1, 8 * blocks2 / std::max<int64_t>(groups, 1));
     for (int m = 0; m <= h.nA; ++m) {
         const int64_t nr = h.row_base[m + 1] - h.row_base[m];
         if (nr == 0) continue;
         const int64_t len = h.ncol[m];
-        // the x slab of the block (nr rows x w) should take at most ~48 MB of L2
         int64_t w = (int64_t)(48.0e6 / ((double)nr * sizeof(T)));
         w = w / 32 * 32;
         if (w < 256) w = 256;
+        w = std::min(w, std::max<int64_t>(128, (len / cuts + 127) / 128 * 128));
         if (w > len) w = len;
         const int b = p.nblk++;
         p.m[b] = m;
@@ -1204,7 +1323,6 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
         p.ngroups[b] = (nr + 7) / 8;
         p.item_base[b + 1] = p.item_base[b] + ((len + w - 1) / w) * p.ngroups[b];
     }
-    int64_t blocks2 = std::min<int64_t>((int64_t)nsm * 8, kMaxPartialBlocksHeis);
     if (blocks2 > p.item_base[p.nblk]) blocks2 = p.item_base[p.nblk];
     if (blocks2 < 1) blocks2 = 1;
     heis_slab_kernel<T><<<(unsigned)blocks2, 256, 0, st>>>(x, y, a, p, dots ? partials : nullptr);
