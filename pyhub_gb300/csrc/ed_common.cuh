@@ -53,6 +53,7 @@ constexpr double kTol14 = (double)1.0e-14f;
 // between J and K).  CSR over targets.
 struct HopTable {
     int norb = 0, ne = 0;
+    int max_row = 0;        // most hops of one string
     int64_t n = 0;          // strings
     int64_t nnz = 0;
     uint32_t *str = nullptr;   // [n]
@@ -189,6 +190,8 @@ struct ed_sector {
     double u_site[ed::kMaxSites];  // U per site, indexed by bit (bit b <-> site norb-b)
     bool u_uniform = true;
     double u_value = 0.0;
+    double *u_lut = nullptr;       // [4][256]: on-site energy of the doubly occupied bits of one byte
+    float *u_lut32 = nullptr;
     ed::HeisTables heis;
     ed::HeisStruct *hs = nullptr;  // Heisenberg row tables
     ed::UijklTables *uijkl = nullptr;   // U_ijkl terms (ed_sector_set_uijkl), else NULL

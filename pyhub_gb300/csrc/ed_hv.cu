@@ -16,6 +16,8 @@
 // row/pass structure (rows of B-half patterns over A-half patterns).
 #include "ed_common.cuh"
 
+#include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 namespace ed {
@@ -25,34 +27,31 @@ struct HubArgs {
     const uint32_t *ustr; const int32_t *uptr; const int32_t *usrc; const void *ucf; const void *uediag;
     const uint32_t *dstr; const int32_t *dptr; const int32_t *dsrc; const void *dcf; const void *dediag;
     int64_t nslice;
-    const int32_t *ell_off; const int32_t *ell_src;
+    const int32_t *ell_off; const int32_t *ell_src; const void *ell_cf;
     const int2 *ell_pk32;
-    double u_site[kMaxSites];
-    float u_site32[kMaxSites];
+    const void *u_lut;        // [nbytes][256], float or double like the vectors
+    int nbytes;               // bytes of a string with an on-site interaction (1 when there is none: zeros)
     int u_uniform;
     double u_value;
     double scale;
 };
 
+// on-site energy of the doubly occupied bits `both`, byte by byte from the table
 template <typename T>
-__device__ __forceinline__ const T *u_sites(const HubArgs &a)
+__device__ __forceinline__ T u_table(const HubArgs &a, uint32_t both)
 {
-    return (sizeof(T) == 4) ? reinterpret_cast<const T *>(a.u_site32) : reinterpret_cast<const T *>(a.u_site);
+    const T *lut = static_cast<const T *>(a.u_lut);
+    T e = __ldg(lut + (both & 255u));
+    for (int b = 1; b < a.nbytes; ++b) e += __ldg(lut + b * 256 + ((both >> (8 * b)) & 255u));
+    return e;
 }
 
-// on-site energy of the doubly occupied bits `both`; uval = U in T (uniform U)
+// the same; uval = U in T (uniform U, where a count is cheaper in FP32)
 template <typename T>
 __device__ __forceinline__ T u_energy(const HubArgs &a, uint32_t both, T uval)
 {
-    if (a.u_uniform) return uval * (T)__popc(both);
-    const T *us = u_sites<T>(a);
-    T e = 0;
-    while (both) {
-        int b = __ffs(both) - 1;
-        e += us[b];
-        both &= both - 1;
-    }
-    return e;
+    if (sizeof(T) == 4 && a.u_uniform) return uval * (T)__popc(both);
+    return u_table<T>(a, both);
 }
 
 // Copy n elements from global src to shared dst (dst 16-byte aligned).
@@ -106,7 +105,7 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *xs = reinterpret_cast<T *>(smem_raw);
-    const T *__restrict__ ecf = static_cast<const T *>(a.ucf);
+    const T *__restrict__ ecf = static_cast<const T *>(a.ell_cf);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int64_t nsup = a.nsup, ld = a.ld;
     const T uval = (T)a.u_value, sc = (T)a.scale;
@@ -146,7 +145,7 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
             if (ok) {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    if (r < nr) y[(d0 + r) * ld + u] = acc[r] * sc;
+                    if (r < nr) y[(d0 + r) * ld + u] = (sc == (T)1) ? acc[r] : acc[r] * sc;
             }
         }
         __syncthreads();
@@ -216,8 +215,13 @@ __global__ void __launch_bounds__(1024) hub_row_col4_kernel(const float *__restr
             const float4 xv = xs4[uu];
             const float xr[4] = {xv.x, xv.y, xv.z, xv.w};
             float acc[4];
+            if (a.u_uniform) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[r] = (eu + ed[r] + u_energy<float>(a, su & sd[r], uval)) * xr[r];
+                for (int r = 0; r < 4; ++r) acc[r] = (eu + ed[r] + uval * (float)__popc(su & sd[r])) * xr[r];
+            } else {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) acc[r] = (eu + ed[r] + u_table<float>(a, su & sd[r])) * xr[r];
+            }
             const int s0 = __ldg(a.ell_off + sl), ns = __ldg(a.ell_off + sl + 1) - s0;
             const int64_t at0 = (int64_t)s0 * 32 + lane;
             int k = 0;
@@ -237,19 +241,26 @@ __global__ void __launch_bounds__(1024) hub_row_col4_kernel(const float *__restr
     }
 }
 
-constexpr int kSlabLoads = 4;   // neighbour-row loads in flight per warp in the slab pass (8 costs occupancy)
+// A down hop of a row: source row and coefficient.
+template <typename T> struct alignas(sizeof(T) == 4 ? 8 : 16) RowHop {
+    int src;
+    T cf;
+};
 
 // Pass 2: down hops, y[d][slab] += sum_e c_e x[src_e][slab]; optional dots.
 // Work items (slab, group of 8 rows) are visited slab-major by a persistent
 // grid so that the CTAs in flight share one or two slabs of x in L2.  A warp
-// holds its row's neighbour list in registers (one entry per lane) and issues
-// the neighbour loads of a chunk back to back.
-template <typename T, int VW>
+// keeps its row's neighbour list in shared memory (one 8- or 16-byte broadcast
+// read per hop; two or three shuffles per hop before), walks U chunks of 32*VW columns together
+// and issues the loads of L neighbour rows back to back.
+template <typename T, int VW, int U, int L>
 __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, T *__restrict__ y,
                                                        const HubArgs a, int64_t slab_w, int64_t ngroups,
                                                        int64_t nitems, double *__restrict__ partials)
 {
+    __shared__ RowHop<T> lists[8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    RowHop<T> *hop = lists[warp];
     const T *__restrict__ cf = static_cast<const T *>(a.dcf);
     const int64_t nsup = a.nsup, ld = a.ld;
     const T sc = (T)a.scale;
@@ -264,77 +275,80 @@ __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, 
         const T *xd = x + d * ld;
         float pxy = 0.f, pyy = 0.f;
         double qxy = 0.0, qyy = 0.0;
+        auto dot = [&](T xv, T yv) {
+            if constexpr (sizeof(T) == 4) { pxy += xv * yv; pyy += yv * yv; }
+            else { qxy += xv * yv; qyy += yv * yv; }
+        };
         for (int b0 = 0; b0 < nn; b0 += 32) {
             const int nb = min(32, nn - b0);
-            const int my_src = (lane < nb) ? __ldg(a.dsrc + e0 + b0 + lane) : 0;
-            const T my_cf = (lane < nb) ? __ldg(cf + e0 + b0 + lane) * sc : (T)0;
+            __syncwarp();
+            if (lane < nb) {
+                hop[lane].src = __ldg(a.dsrc + e0 + b0 + lane);
+                hop[lane].cf = __ldg(cf + e0 + b0 + lane) * sc;
+            }
+            __syncwarp();
             const bool last = (b0 + 32 >= nn);
-            // chunks of 32*VW columns; the loop is warp-uniform so every lane
-            // takes part in the shuffles, lanes past c1 are masked
-            for (int64_t cb = c0; cb < c1; cb += 32 * VW) {
-                const int64_t c = cb + (int64_t)lane * VW;
-                const bool full = c + VW <= c1;
-                const int nk = full ? VW : (c < c1 ? (int)(c1 - c) : 0);
-                T acc[VW];
+            int64_t cb = c0;
+            // whole passes of U chunks
+            for (; cb + 32 * VW * U <= c1; cb += 32 * VW * U) {
+                using V = typename std::conditional<VW == 1, T, typename std::conditional<sizeof(T) == 4, float4, double2>::type>::type;
+                const V *xc = reinterpret_cast<const V *>(x + cb) + lane;
+                V *yc = reinterpret_cast<V *>(yr + cb) + lane;
+                V acc[U];
 #pragma unroll
-                for (int k = 0; k < VW; ++k) acc[k] = (k < nk) ? yr[c + k] : (T)0;
-                int e = 0;
-                for (; e + kSlabLoads <= nb; e += kSlabLoads) {
-                    T v[kSlabLoads][VW];
-                    T wgt[kSlabLoads];
+                for (int u = 0; u < U; ++u) acc[u] = yc[u * 32];
+                auto hops = [&](auto count, int e) {
+                    constexpr int N = decltype(count)::value;
+                    V v[N][U];
+                    T w[N];
 #pragma unroll
-                    for (int i = 0; i < kSlabLoads; ++i) {
-                        const int64_t sidx = __shfl_sync(0xffffffffu, my_src, e + i);
-                        wgt[i] = __shfl_sync(0xffffffffu, my_cf, e + i);
-                        const T *xr = x + sidx * ld + c;
-                        if (full) {
-                            if constexpr (VW == 4 && sizeof(T) == 4) {
-                                const float4 t4 = __ldg(reinterpret_cast<const float4 *>(xr));
-                                v[i][0] = t4.x; v[i][1] = t4.y; v[i][2] = t4.z; v[i][3] = t4.w;
-                            } else if constexpr (VW == 2 && sizeof(T) == 8) {
-                                const double2 t2 = __ldg(reinterpret_cast<const double2 *>(xr));
-                                v[i][0] = t2.x; v[i][1] = t2.y;
-                            } else {
+                    for (int i = 0; i < N; ++i) {
+                        const RowHop<T> h = hop[e + i];
+                        w[i] = h.cf;
+                        const V *xr = reinterpret_cast<const V *>(reinterpret_cast<const T *>(xc) + h.src * ld);
 #pragma unroll
-                                for (int k = 0; k < VW; ++k) v[i][k] = __ldg(xr + k);
-                            }
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < VW; ++k) v[i][k] = (k < nk) ? __ldg(xr + k) : (T)0;
-                        }
+                        for (int u = 0; u < U; ++u) v[i][u] = __ldg(xr + u * 32);
                     }
 #pragma unroll
-                    for (int i = 0; i < kSlabLoads; ++i)
+                    for (int i = 0; i < N; ++i)
 #pragma unroll
-                        for (int k = 0; k < VW; ++k) acc[k] += wgt[i] * v[i][k];
+                        for (int u = 0; u < U; ++u)
+#pragma unroll
+                            for (int k = 0; k < VW; ++k)
+                                reinterpret_cast<T *>(&acc[u])[k] += w[i] * reinterpret_cast<const T *>(&v[i][u])[k];
+                };
+                int e = 0;
+                for (; e + L <= nb; e += L) hops(std::integral_constant<int, L>(), e);
+                if (L > 2 && e + 2 <= nb) {
+                    hops(std::integral_constant<int, 2>(), e);
+                    e += 2;
                 }
-                for (; e < nb; ++e) {
-                    const int64_t sidx = __shfl_sync(0xffffffffu, my_src, e);
-                    const T wg = __shfl_sync(0xffffffffu, my_cf, e);
+                for (; e < nb; ++e) hops(std::integral_constant<int, 1>(), e);
 #pragma unroll
-                    for (int k = 0; k < VW; ++k)
-                        if (k < nk) acc[k] += wg * __ldg(x + sidx * ld + c + k);
-                }
-#pragma unroll
-                for (int k = 0; k < VW; ++k)
-                    if (k < nk) yr[c + k] = acc[k];
+                for (int u = 0; u < U; ++u) yc[u * 32] = acc[u];
                 if (partials && last) {
 #pragma unroll
-                    for (int k = 0; k < VW; ++k) {
-                        if (k >= nk) continue;
-                        const T xv = __ldg(xd + c + k);
-                        if constexpr (sizeof(T) == 4) { pxy += xv * acc[k]; pyy += acc[k] * acc[k]; }
-                        else { qxy += xv * acc[k]; qyy += acc[k] * acc[k]; }
+                    for (int u = 0; u < U; ++u) {
+                        const V xv = __ldg(reinterpret_cast<const V *>(xd + cb) + lane + u * 32);
+#pragma unroll
+                        for (int k = 0; k < VW; ++k)
+                            dot(reinterpret_cast<const T *>(&xv)[k], reinterpret_cast<const T *>(&acc[u])[k]);
                     }
                 }
+            }
+            // the rest of the slab, a column per lane
+            for (int64_t c = cb + lane; c < c1; c += 32) {
+                T acc = yr[c];
+#pragma unroll 4
+                for (int e = 0; e < nb; ++e) acc += hop[e].cf * __ldg(x + hop[e].src * ld + c);
+                yr[c] = acc;
+                if (partials && last) dot(__ldg(xd + c), acc);
             }
         }
         if (nn == 0 && partials) {
             // no down hops: the dots still need this row's y
             for (int64_t cc = c0 + lane; cc < c1; cc += 32) {
-                const T yv = yr[cc], xv = __ldg(xd + cc);
-                if constexpr (sizeof(T) == 4) { pxy += xv * yv; pyy += yv * yv; }
-                else { qxy += xv * yv; qyy += yv * yv; }
+                dot(__ldg(xd + cc), yr[cc]);
             }
         }
         dxy += (double)pxy + qxy;
@@ -349,6 +363,100 @@ __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, 
         if (threadIdx.x == 0) {
             double sxy = 0.0, syy = 0.0;
             for (int w = 0; w < 8; ++w) { sxy += red[0][w]; syy += red[1][w]; }
+            partials[2 * blockIdx.x] = sxy;
+            partials[2 * blockIdx.x + 1] = syy;
+        }
+    }
+}
+
+// Both passes in one, for small sectors: R rows are staged side by side in shared memory, a thread owns
+// one of them (its row constants stay in registers) and every blockDim/R-th column: diagonal, down
+// hops from the neighbour rows in L2, up hops from the staged rows, scale, store, dots.  Bound by
+// latency (a thread's loads for one column are in flight together, nothing else), which a launch less
+// and no second trip of y outweigh while the sector is small.  Items (row block, column share) are cut
+// so that every resident CTA walks several.  With ADD the product is added to y.
+template <typename T, int R, bool ADD>
+__global__ void __launch_bounds__(512, 2) hub_fused_kernel(const T *__restrict__ x, T *y, const HubArgs a, int maxrow,
+                                                           int csplit, int64_t nitems, double *__restrict__ partials)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    RowHop<T> *nb = reinterpret_cast<RowHop<T> *>(smem_raw);   // [R][maxrow]
+    T *xs = reinterpret_cast<T *>(nb + R * maxrow);             // [nsup][R]
+    const int nsup = (int)a.nsup;
+    const int64_t ld = a.ld;
+    const T sc = (T)a.scale;
+    const T *ued_t = static_cast<const T *>(a.uediag), *ded_t = static_cast<const T *>(a.dediag);
+    const T *ucf = static_cast<const T *>(a.ucf), *dcf = static_cast<const T *>(a.dcf);
+    const int r = threadIdx.x % R, step = blockDim.x / R;
+    double dxy = 0.0, dyy = 0.0;
+    int64_t staged = -1;
+    for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x) {
+        const int64_t rb = item / csplit;
+        const int cs = (int)(item - rb * csplit);
+        const int64_t d0 = rb * R, d = d0 + r;
+        const bool row = d < a.nsdn;
+        int nn = 0;
+        if (row) nn = __ldg(a.dptr + d + 1) - __ldg(a.dptr + d);
+        if (rb != staged) {
+            __syncthreads();      // the previous rows' readers are done
+            for (int i = threadIdx.x; i < nsup; i += blockDim.x) {
+#pragma unroll
+                for (int q = 0; q < R; ++q) xs[i * R + q] = (d0 + q < a.nsdn) ? __ldg(x + (d0 + q) * ld + i) : (T)0;
+            }
+            if (row) {
+                const int e0 = __ldg(a.dptr + d);
+                for (int e = threadIdx.x / R; e < nn; e += step) {
+                    nb[r * maxrow + e].src = __ldg(a.dsrc + e0 + e);
+                    nb[r * maxrow + e].cf = __ldg(dcf + e0 + e);
+                }
+            }
+            staged = rb;
+            __syncthreads();
+        }
+        if (!row) continue;
+        const uint32_t sd = __ldg(a.dstr + d);
+        const T ed = __ldg(ded_t + d);
+        const RowHop<T> *hop = nb + r * maxrow;
+        const int c0 = (int)((int64_t)nsup * cs / csplit), c1 = (int)((int64_t)nsup * (cs + 1) / csplit);
+        T pxy = 0, pyy = 0;
+        for (int c = c0 + threadIdx.x / R; c < c1; c += step) {
+            const T xv = xs[c * R + r];
+            T acc = (__ldg(ued_t + c) + ed + u_table<T>(a, __ldg(a.ustr + c) & sd)) * xv;
+            const T *xc = x + c;
+            int e = 0;
+            for (; e + 4 <= nn; e += 4) {
+                T v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = __ldg(xc + hop[e + i].src * ld);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc += hop[e + i].cf * v[i];
+            }
+            for (; e < nn; ++e) acc += hop[e].cf * __ldg(xc + hop[e].src * ld);
+            const int u1 = __ldg(a.uptr + c + 1);
+#pragma unroll 4
+            for (int q = __ldg(a.uptr + c); q < u1; ++q) acc += __ldg(ucf + q) * xs[__ldg(a.usrc + q) * R + r];
+            if (sc != (T)1) acc *= sc;
+            T *yp = y + d * ld + c;
+            if (ADD) acc += *yp;
+            *yp = acc;
+            if (partials) {
+                pxy += xv * acc;
+                pyy += acc * acc;
+            }
+        }
+        dxy += (double)pxy;
+        dyy += (double)pyy;
+    }
+    if (partials) {
+        __shared__ double red[2][16];
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        dxy = warp_sum(dxy);
+        dyy = warp_sum(dyy);
+        if (lane == 0) { red[0][warp] = dxy; red[1][warp] = dyy; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double sxy = 0.0, syy = 0.0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { sxy += red[0][w]; syy += red[1][w]; }
             partials[2 * blockIdx.x] = sxy;
             partials[2 * blockIdx.x + 1] = syy;
         }
@@ -399,6 +507,13 @@ int launch_reduce(const double *partials, int nblocks, int m, double *out, cudaS
 
 static constexpr int kMaxPartialBlocks = 1024;
 
+// Sectors that take the one-pass product.  Measured one pass / two: 8-site ring FP64 9.4 / 12.8 us (one launch
+// instead of two), 11 sites half filled (213,444) FP64 22.5 / 26.7, FP32 11.9 / 18.5; 16 sites (3,3)
+// (313,600) 28.7 / 26.7 and 16.4 / 13.9, 3x4 half filled 101 / 81 and 48 / 23.  Rows of at most 128
+// strings leave most of a row CTA idle: 16 sites (2,8), 1.5 M states, 115 / 125 and 41 / 68.
+constexpr int64_t kFuseStates = 1 << 18;
+constexpr int64_t kFuseRow = 128;
+
 // L2 budget of one x slab in the slab pass: 48 MB (a third of the 129 MB
 // L2, leaving room for the y slab in flight and the tables); the
 // environment variable PYHUB_ED_SLAB_L2_BYTES overrides it for tuning.
@@ -412,6 +527,42 @@ static double slab_l2_bytes()
     return v;
 }
 
+// Largest shared memory a kernel may ask for on the current device.
+static int max_smem()
+{
+    static std::atomic<int> known[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int v = (dev >= 0 && dev < 64) ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (v == 0) {
+        cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (dev >= 0 && dev < 64) known[dev].store(v, std::memory_order_relaxed);
+    }
+    return v;
+}
+
+template <typename T, int R>
+static int launch_fused(ed_sector *s, cudaStream_t st, const T *x, T *y, HubArgs &a, bool add, double *dots,
+                        double *partials)
+{
+    const int nsm = num_sms(), maxrow = std::max(s->dn.max_row, 1);
+    const size_t smem = (size_t)R * maxrow * sizeof(RowHop<T>) + (size_t)R * s->nsup * sizeof(T);
+    auto *kfn = add ? hub_fused_kernel<T, R, true> : hub_fused_kernel<T, R, false>;
+    if (smem > 48 * 1024)
+        ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int threads = (int)std::min<int64_t>(512, std::max<int64_t>(64, (R * s->nsup / 2 + 31) / 32 * 32));
+    // CTAs resident per SM: by threads (at most 1024 by registers) and by shared memory
+    const int per_sm = (int)std::max<int64_t>(1, std::min<int64_t>(1024 / threads, (228 * 1024) / (int64_t)(smem + 1024)));
+    const int64_t rb = (s->nsdn + R - 1) / R, resident = std::min<int64_t>((int64_t)nsm * per_sm, kMaxPartialBlocks);
+    const int64_t most = std::max<int64_t>(1, s->nsup * R / threads);    // a column for every thread
+    const int csplit = (int)std::min<int64_t>(most, std::max<int64_t>(1, 6 * resident / rb));
+    const int64_t nitems = rb * csplit, blocks = std::min(nitems, resident);
+    kfn<<<(unsigned)blocks, threads, smem, st>>>(x, y, a, maxrow, csplit, nitems, dots ? partials : nullptr);
+    ED_CHECK_LAUNCH();
+    if (dots) return launch_reduce(partials, (int)blocks, 2, dots, st);
+    return ED_OK;
+}
+
 template <typename T>
 static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, double scale, double *dots,
                   double *partials)
@@ -422,16 +573,15 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     a.dstr = s->dn.str; a.dptr = s->dn.ptr; a.dsrc = s->dn.src;
     a.uediag = (sizeof(T) == 4) ? (const void *)s->up.ediag32 : (const void *)s->up.ediag;
     a.dediag = (sizeof(T) == 4) ? (const void *)s->dn.ediag32 : (const void *)s->dn.ediag;
-    if (sizeof(T) == 4) { a.ucf = s->up.ell_cf32; a.dcf = s->dn.cf32; }
-    else { a.ucf = s->up.ell_cf64; a.dcf = s->dn.cf64; }
+    a.dcf = (sizeof(T) == 4) ? (const void *)s->dn.cf32 : (const void *)s->dn.cf64;
+    a.ucf = (sizeof(T) == 4) ? (const void *)s->up.cf32 : (const void *)s->up.cf64;
     a.nslice = s->up.nslice;
     a.ell_off = s->up.ell_off;
     a.ell_src = s->up.ell_src;
+    a.ell_cf = (sizeof(T) == 4) ? (const void *)s->up.ell_cf32 : (const void *)s->up.ell_cf64;
     a.ell_pk32 = s->up.ell_pk32;
-    for (int b = 0; b < kMaxSites; ++b) {
-        a.u_site[b] = s->u_site[b];
-        a.u_site32[b] = (float)s->u_site[b];
-    }
+    a.u_lut = (sizeof(T) == 4) ? (const void *)s->u_lut32 : (const void *)s->u_lut;
+    a.nbytes = (s->u_uniform && s->u_value == 0.0) ? 1 : (s->norb + 7) / 8;
     a.u_uniform = s->u_uniform ? 1 : 0;
     a.u_value = s->u_value;
     a.scale = scale;
@@ -440,17 +590,29 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     // ---- pass 1
     const int64_t sld = (s->nsup + VWS - 1) / VWS * VWS;
     const bool vec_ok = (ld % VWS == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    int maxsm = 0;
-    {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    }
+    const int maxsm = max_smem();
     const size_t row_bytes = (size_t)sld * sizeof(T);
     if (row_bytes > (size_t)maxsm) {
         set_error("up-string row of %lld entries does not fit in shared memory (%d bytes)",
                   (long long)s->nsup, maxsm);
         return ED_ERR_RANGE;
+    }
+    const size_t lists = (size_t)std::max(s->dn.max_row, 1) * sizeof(RowHop<T>);
+    if ((s->dim <= kFuseStates || s->nsup <= kFuseRow) && lists + (size_t)s->nsup * sizeof(T) <= (size_t)maxsm) {
+        // the U_ijkl terms go into a cleared y first, so that the dots see the whole product
+        const bool add = s->uijkl != nullptr;
+        if (add) {
+            ED_CHECK_CUDA(cudaMemset2DAsync(y, (size_t)ld * sizeof(T), 0, (size_t)s->nsup * sizeof(T), (size_t)s->nsdn, st));
+            const int rc = uijkl_hv(s, st, sizeof(T) == 4 ? ED_F32 : ED_F64, ld, x, y, scale);
+            if (rc != ED_OK) return rc;
+        }
+        // four rows side by side, else two, where two CTAs of them fit an SM and the SMs have rows enough
+        auto fits = [&](int R) {
+            return R * (lists + s->nsup * sizeof(T)) <= (size_t)maxsm / 2 && s->nsdn >= (int64_t)R * nsm;
+        };
+        if (fits(4)) return launch_fused<T, 4>(s, st, x, y, a, add, dots, partials);
+        if (fits(2)) return launch_fused<T, 2>(s, st, x, y, a, add, dots, partials);
+        return launch_fused<T, 1>(s, st, x, y, a, add, dots, partials);
     }
     // FP32: four rows per 1024-thread CTA (one CTA per SM) when they fit, so every
     // hop-table slot serves four rows and one 128-bit gather reads all four;
@@ -495,28 +657,29 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     if (slab_w < 256) slab_w = 256;
     if (slab_w > s->nsup) slab_w = (s->nsup + VWS - 1) / VWS * VWS;
     const int64_t ngroups = (s->nsdn + 7) / 8;
-    const int64_t nslab = (s->nsup + slab_w - 1) / slab_w;
-    const int64_t nitems = ngroups * nslab;
+    const bool vec2 = (ld % VWS == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
+                      ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
+    // chunks x rows in flight, measured (4x4 / 14 random bonds): FP32 2 x 2 1,012 us / 148 us the whole
+    // product, 1 x 4 1,070 / 154, 4 x 2 1,790 / 250 (registers); FP64 4 x 2 5.37 ms / 742 us, 2 x 4 6.26 / 743
+    auto *kfn = !vec2 ? hub_slab_kernel<T, 1, 1, 4>
+                      : sizeof(T) == 4 ? hub_slab_kernel<T, VWS, 2, 2> : hub_slab_kernel<T, VWS, 4, 2>;
     // one wave of resident CTAs: each walks its share of the items, so a grid past the
     // resident count would leave a second, partial wave running whole shares
-    const bool vec2pre = (ld % VWS == 0);
     int per_sm = 0;
-    if (vec2pre)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hub_slab_kernel<T, VWS>, 256, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hub_slab_kernel<T, 1>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, 256, 0);
     if (per_sm < 1) per_sm = 1;
     int64_t blocks2 = (int64_t)nsm * per_sm;
     if (blocks2 > kMaxPartialBlocks) blocks2 = kMaxPartialBlocks;
+    // narrower slabs where a CTA's share would be a few items (the last of them would leave a part of
+    // the wave idle: 14 sites FP32 160 -> 148 us)
+    while (slab_w > 256 && ngroups * ((s->nsup + slab_w - 1) / slab_w) < 8 * blocks2)
+        slab_w = std::max<int64_t>(256, slab_w / 2 / 256 * 256);
+    const int64_t nslab = (s->nsup + slab_w - 1) / slab_w;
+    const int64_t nitems = ngroups * nslab;
     if (blocks2 > nitems) blocks2 = nitems;
     if (blocks2 < 1) blocks2 = 1;
-    const bool vec2 = (ld % VWS == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
-                      ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
     double *part = dots ? partials : nullptr;
-    if (vec2)
-        hub_slab_kernel<T, VWS><<<(unsigned)blocks2, 256, 0, st>>>(x, y, a, slab_w, ngroups, nitems, part);
-    else
-        hub_slab_kernel<T, 1><<<(unsigned)blocks2, 256, 0, st>>>(x, y, a, slab_w, ngroups, nitems, part);
+    kfn<<<(unsigned)blocks2, 256, 0, st>>>(x, y, a, slab_w, ngroups, nitems, part);
     ED_CHECK_LAUNCH();
     if (dots) return launch_reduce(partials, (int)blocks2, 2, dots, st);
     return ED_OK;

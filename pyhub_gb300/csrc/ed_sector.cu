@@ -423,6 +423,8 @@ static int upload_hop(const HostHop &h, int norb, int ne, HopTable &d, TablePool
     d.ne = ne;
     d.n = (int64_t)h.str.size();
     d.nnz = (int64_t)h.src.size();
+    d.max_row = 0;
+    for (size_t q = 0; q + 1 < h.ptr.size(); ++q) d.max_row = std::max(d.max_row, (int)(h.ptr[q + 1] - h.ptr[q]));
     std::vector<float> c32(h.coef.begin(), h.coef.end());
     std::vector<float> e32(h.ediag.begin(), h.ediag.end());
     pool.add(&d.str, h.str.data(), h.str.size());
@@ -618,7 +620,16 @@ int ed_sector_create(int norb, int nup, int ndn, int kind, const double *t, cons
             s->u_site[norb - p] = U[p - 1];  // bit norb-p holds site p
             if (U[p - 1] != U[0]) s->u_uniform = false;
         }
+        std::vector<double> ulut(4 * 256, 0.0);
+        for (int k = 0; k < 4 * 256; ++k)
+            for (int q = 0; q < 8; ++q) {
+                const int b = k / 256 * 8 + q;
+                if (b < norb && ((k >> q) & 1)) ulut[(size_t)k] += s->u_site[b];
+            }
+        std::vector<float> ulut32(ulut.begin(), ulut.end());
         TablePool pool;
+        pool.add(&s->u_lut, ulut.data(), ulut.size());
+        pool.add(&s->u_lut32, ulut32.data(), ulut32.size());
         HostHop hu;
         rc = build_hop_host(norb, nup, t, hu);
         if (!rc) rc = upload_hop(hu, norb, nup, s->up, pool);
