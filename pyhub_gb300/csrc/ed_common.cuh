@@ -44,6 +44,7 @@ void clear_error();
     } while (0)
 
 constexpr int kMaxSites = 32;
+constexpr int kULut = 4 * 256 + kMaxSites + 1;   // entries of a sector's on-site energy table
 // The reference compares |t| against the REAL*4 literal 1.E-14.
 constexpr double kTol14 = (double)1.0e-14f;
 
@@ -190,7 +191,8 @@ struct ed_sector {
     double u_site[ed::kMaxSites];  // U per site, indexed by bit (bit b <-> site norb-b)
     bool u_uniform = true;
     double u_value = 0.0;
-    double *u_lut = nullptr;       // [4][256]: on-site energy of the doubly occupied bits of one byte
+    double *u_lut = nullptr;       // [4][256]: on-site energy of the doubly occupied bits of one byte; then
+                                   // U times 0, 1, .. norb when U is uniform
     float *u_lut32 = nullptr;
     ed::HeisTables heis;
     ed::HeisStruct *hs = nullptr;  // Heisenberg row tables

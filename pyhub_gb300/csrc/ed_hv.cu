@@ -29,7 +29,7 @@ struct HubArgs {
     int64_t nslice;
     const int32_t *ell_off; const int32_t *ell_src; const void *ell_cf;
     const int2 *ell_pk32;
-    const void *u_lut;        // [nbytes][256], float or double like the vectors
+    const void *u_lut;        // [4][256], then U times a count; float or double like the vectors
     int nbytes;               // bytes of a string with an on-site interaction (1 when there is none: zeros)
     int u_uniform;
     double u_value;
@@ -50,7 +50,10 @@ __device__ __forceinline__ T u_table(const HubArgs &a, uint32_t both)
 template <typename T>
 __device__ __forceinline__ T u_energy(const HubArgs &a, uint32_t both, T uval)
 {
-    if (sizeof(T) == 4 && a.u_uniform) return uval * (T)__popc(both);
+    if (a.u_uniform) {
+        if constexpr (sizeof(T) == 4) return uval * (T)__popc(both);
+        return __ldg(static_cast<const T *>(a.u_lut) + 4 * 256 + __popc(both));   // no FP64 operation
+    }
     return u_table<T>(a, both);
 }
 
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(512, 2) hub_fused_kernel(const T *__restrict__
         T pxy = 0, pyy = 0;
         for (int c = c0 + threadIdx.x / R; c < c1; c += step) {
             const T xv = xs[c * R + r];
-            T acc = (__ldg(ued_t + c) + ed + u_table<T>(a, __ldg(a.ustr + c) & sd)) * xv;
+            T acc = (__ldg(ued_t + c) + ed + u_energy<T>(a, __ldg(a.ustr + c) & sd, (T)a.u_value)) * xv;
             const T *xc = x + c;
             int e = 0;
             for (; e + 4 <= nn; e += 4) {

@@ -620,12 +620,13 @@ int ed_sector_create(int norb, int nup, int ndn, int kind, const double *t, cons
             s->u_site[norb - p] = U[p - 1];  // bit norb-p holds site p
             if (U[p - 1] != U[0]) s->u_uniform = false;
         }
-        std::vector<double> ulut(4 * 256, 0.0);
+        std::vector<double> ulut(kULut, 0.0);
         for (int k = 0; k < 4 * 256; ++k)
             for (int q = 0; q < 8; ++q) {
                 const int b = k / 256 * 8 + q;
                 if (b < norb && ((k >> q) & 1)) ulut[(size_t)k] += s->u_site[b];
             }
+        for (int k = 0; k <= norb && s->u_uniform; ++k) ulut[(size_t)(4 * 256 + k)] = s->u_value * k;
         std::vector<float> ulut32(ulut.begin(), ulut.end());
         TablePool pool;
         pool.add(&s->u_lut, ulut.data(), ulut.size());

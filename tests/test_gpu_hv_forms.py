@@ -97,3 +97,26 @@ def test_hubbard_product_forms(edlib, n, nu, nd, dt):
             tol = 1e-12 if dt == "f64" else 2e-5
             assert abs(float(dots[0]) - float((x * got).sum())) <= tol * float((x * got).abs().sum()) + 1e-300
             assert abs(float(dots[1]) - float((got * got).sum())) <= tol * float((got * got).sum()) + 1e-300
+
+
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("U", ["uniform", "sites"])
+def test_uijkl_drops_the_on_site_interaction(edlib, dt, U):
+    """A sector built with an on-site U loses it when the U_ijkl interaction is set, as one built without."""
+    import torch
+    td = torch.float32 if dt == "f32" else torch.float64
+    n = 6
+    rng = np.random.default_rng(2)
+    t = rng.integers(-2, 3, (n, n)).astype(float)
+    t = np.triu(t) + np.triu(t, 1).T
+    Ul = rng.integers(-2, 3, (n,) * 4).astype(float)
+    u = np.full(n, 3.0) if U == "uniform" else np.arange(1.0, n + 1)
+    x = torch.randint(-4, 5, (400,), device="cuda").to(td)
+    ys = []
+    for uu in (u, np.zeros(n)):
+        sec = edlib.Sector(n, 3, 3, edlib.ED_HUBBARD, t=t, U=uu)
+        sec.set_uijkl(Ul)
+        y = sec.zeros(td)
+        sec.hv(sec.from_ref(x), y)
+        ys.append(sec.to_ref(y))
+    assert torch.equal(ys[0], ys[1])
