@@ -124,6 +124,7 @@ struct HeisStruct {
     uint32_t *col_abbits = nullptr;  // per column: its A bits at the A-B bonds
     uint32_t *row_bbits = nullptr;   // per row: its B bits at the A-B bonds
     double *ab_lut = nullptr;        // [4][256]: zz/2 summed over the set bits of eight A-B bonds
+    float *ab_lut32 = nullptr;
     int32_t *ab_rank = nullptr;      // [q][column]: rank after flipping A-B bond q's A bit
     int64_t ncols = 0;               // columns over all m (the stride of ab_rank)
     int nab = 0;

@@ -266,6 +266,7 @@ int heis_struct_build(ed_sector *s)
         hs->ab_fkj[q] = ht.flip_kj[b];
         hs->ab_zz[q] = 0.25 * ht.zz[b];
     }
+    std::vector<float> ab_lut32(ab_lut.begin(), ab_lut.end());
     std::vector<float> aa_cf32(aa_cf.begin(), aa_cf.end()), bb_cf32(bb_cf.begin(), bb_cf.end());
     std::vector<float> diagA32(diagA.begin(), diagA.end()), diagB32(diagB.begin(), diagB.end());
     std::vector<int2> aa_pk32(aa_src.size());
@@ -283,7 +284,7 @@ int heis_struct_build(ed_sector *s)
         (rc = up(&hs->bb_cf64, bb_cf)) || (rc = up(&hs->rows_of_m, rows_of_m)) ||
         (rc = up(&hs->aa_pk32, aa_pk32)) || (rc = up(&hs->col_abbits, col_abbits)) ||
         (rc = up(&hs->row_bbits, row_bbits)) || (rc = up(&hs->diagA32, diagA32)) || (rc = up(&hs->ab_rank, ab_rank)) ||
-        (rc = up(&hs->diagB32, diagB32)) || (rc = up(&hs->ab_lut, ab_lut)))
+        (rc = up(&hs->diagB32, diagB32)) || (rc = up(&hs->ab_lut, ab_lut)) || (rc = up(&hs->ab_lut32, ab_lut32)))
         return rc;
     return ED_OK;
 }
@@ -295,7 +296,7 @@ void heis_struct_free(HeisStruct *hs)
                     hs->aa_cf64, hs->row_pat, hs->row_m, hs->row_off, hs->rowidx, hs->diagB,
                     hs->bb_ptr, hs->bb_src, hs->bb_cf32, hs->bb_cf64, hs->rows_of_m,
                     hs->aa_pk32, hs->col_abbits, hs->row_bbits, hs->diagA32, hs->diagB32, hs->ab_rank,
-                    hs->ab_lut};
+                    hs->ab_lut, hs->ab_lut32};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete hs;
@@ -315,7 +316,7 @@ struct HsArgs {
     const int2 *aa_pk32;           // {column, FP32 coefficient bits} of the A-A flips
     const uint32_t *col_abbits, *row_bbits;
     const int32_t *ab_rank;        // [q][column] rank after flipping bond q's A bit (packed path)
-    const double *ab_lut;
+    const void *ab_lut;            // [4][256] zz drops of eight bonds, float or double
     int64_t ncols;
     int ab_fast;
     int8_t ab_pa[kMaxAB], ab_pb[kMaxAB];
@@ -337,7 +338,7 @@ constexpr int kHeisRowThreads = 512;
 // bytes of the A-B bond facts ahead of the staged row (16-byte aligned)
 __host__ __device__ inline size_t heis_row_head_bytes(int nab, size_t tsize)
 {
-    const size_t b = (size_t)nab * (sizeof(int64_t) + 3 * tsize + sizeof(uint32_t));
+    const size_t b = (size_t)nab * (sizeof(int64_t) + 2 * tsize + sizeof(uint32_t));
     return (b + 15) / 16 * 16;
 }
 constexpr int64_t kMaxPartialBlocksHeis = 1024;   // the partials that ed_scratch_bytes provides for
@@ -352,13 +353,11 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
     int64_t *ab_src = reinterpret_cast<int64_t *>(smem_raw);      // source row offset, -1 if impossible
     T *ab_c = reinterpret_cast<T *>(ab_src + a.nab);               // flip element for the required A state
     T *ab_dsame = ab_c + a.nab;                                    // zz/4 (generic path)
-    T *ab_w2 = ab_dsame + a.nab;                                   // zz/2: drop of an antiparallel bond
-    uint32_t *ab_need = reinterpret_cast<uint32_t *>(ab_w2 + a.nab);  // required A bit (1: A site down)
+    uint32_t *ab_need = reinterpret_cast<uint32_t *>(ab_dsame + a.nab);  // required A bit (1: A site down)
     T *xs = reinterpret_cast<T *>(smem_raw + heis_row_head_bytes(a.nab, sizeof(T)));
     const T *acf = reinterpret_cast<const T *>(a.aa_cf);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kHeisRowThreads / 32;
     const T sc = (T)a.scale;
-    constexpr bool kLut = sizeof(T) == 8;
     for (int64_t k = 0; k * gridDim.x < a.nrows; ++k) {
         int m;
         int64_t row;
@@ -397,7 +396,6 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
             ab_need[q] = 1u - hk;
             ab_c[q] = (T)(hk ? a.ab_fkj[q] : a.ab_fjk[q]);   // target hj = 1-hk: hj ? fjk : fkj
             ab_dsame[q] = (T)a.ab_zz[q];
-            ab_w2[q] = (T)(2.0 * a.ab_zz[q]);
         }
         cp_async_wait_all();
         __syncthreads();
@@ -427,13 +425,12 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
                 // antiparallel A-B bonds: the set bits of (column's A bits ^ row's B bits); their
                 // zz/4 was counted as "equal" in diagB, so each one drops the diagonal by zz/2
                 uint32_t diff = __ldg(a.col_abbits + cbase + cc) ^ rbits;
-                // FP64 (bound by the FP64 pipe): eight bonds' zz drops from a table, one subtraction for them
-                if (kLut)
-                    for (int g = 0; g * 8 < a.nab; ++g) d -= (T)__ldg(a.ab_lut + g * 256 + ((diff >> (8 * g)) & 255u));
+                // eight bonds' zz drops from a table: one subtraction for them
+                const T *lut = static_cast<const T *>(a.ab_lut);
+                for (int g = 0; g * 8 < a.nab; ++g) d -= __ldg(lut + g * 256 + ((diff >> (8 * g)) & 255u));
                 while (diff) {
                     const int q = __ffs(diff) - 1;
                     diff &= diff - 1;
-                    if (!kLut) d -= ab_w2[q];
                     const int64_t src = ab_src[q];
                     if (src >= 0) acc += ab_c[q] * __ldg(x + src + __ldg(a.ab_rank + q * a.ncols + cbase + cc));
                 }
@@ -456,10 +453,17 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
 
 constexpr int kHeisCol4Threads = 1024;
 
+// An A-B bond of one staged row: the source row's first element (a sector has fewer than 2^31) and the
+// flip element.  A column antiparallel to the row at the bond always has that row.
+struct alignas(8) AbFact {
+    int src;
+    float c;
+};
+
 // bytes of the four rows' A-B bond facts ahead of the staged columns (16-byte aligned)
 __host__ __device__ inline size_t heis_col4_head_bytes(int nab)
 {
-    const size_t b = (size_t)nab * (4 * sizeof(int64_t) + 4 * sizeof(float) + sizeof(float));
+    const size_t b = (size_t)nab * 4 * sizeof(AbFact);
     return (b + 15) / 16 * 16;
 }
 
@@ -501,9 +505,7 @@ __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(cons
                                                                           int64_t nitems)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    int64_t *ab_src = reinterpret_cast<int64_t *>(smem_raw);      // [4][nab] source row offset, -1 if impossible
-    float *ab_c = reinterpret_cast<float *>(ab_src + 4 * a.nab);   // [4][nab] flip element
-    float *ab_w2 = ab_c + 4 * a.nab;                               // [nab] zz/2: drop of an antiparallel bond
+    AbFact *facts = reinterpret_cast<AbFact *>(smem_raw);          // [4][nab]
     float4 *xs4 = reinterpret_cast<float4 *>(smem_raw + heis_col4_head_bytes(a.nab));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const float sc = (float)a.scale;
@@ -544,18 +546,17 @@ __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(cons
         }
         for (int t = threadIdx.x; t < 4 * a.nab; t += blockDim.x) {
             const int r = t / a.nab, q = t - r * a.nab;
-            int64_t src = -1;
-            float cf = 0.f;
+            AbFact f = {0, 0.f};
             if (r < nr) {
                 const uint32_t h = (r == 0) ? hb[0] : (r == 1) ? hb[1] : (r == 2) ? hb[2] : hb[3];
                 const uint32_t hk = (h >> a.ab_pb[q]) & 1u;
                 const int32_t r2 = __ldg(a.rowidx + (h ^ (1u << a.ab_pb[q])));
-                src = (r2 >= 0) ? __ldg(a.row_off + r2) : (int64_t)-1;
-                cf = (float)(hk ? a.ab_fkj[q] : a.ab_fjk[q]);
+                if (r2 >= 0) {
+                    f.src = (int)__ldg(a.row_off + r2);
+                    f.c = (float)(hk ? a.ab_fkj[q] : a.ab_fjk[q]);
+                }
             }
-            ab_src[t] = src;
-            ab_c[t] = cf;
-            if (r == 0) ab_w2[q] = (float)(2.0 * a.ab_zz[q]);
+            facts[t] = f;
         }
         cp_async_wait_all();
         __syncthreads();
@@ -580,39 +581,38 @@ __global__ void __launch_bounds__(kHeisCol4Threads, 1) heis_row_col4_kernel(cons
             for (; q < ns; ++q) heis_col4_group<1>(a, at0 + q * 32, xs4, acc);
             // antiparallel A-B bonds of each row: the set bits of (column's A bits ^ row's B bits)
             const uint32_t ca = __ldg(a.col_abbits + cbase + cc);
-            uint32_t diff[4], any = 0u;
+            const float *lut = static_cast<const float *>(a.ab_lut);
+            uint32_t diff[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 diff[r] = (r < nr) ? (ca ^ rbits[r]) : 0u;
-                any |= diff[r];
+#pragma unroll
+                for (int g8 = 0; g8 < 4; ++g8)
+                    if (g8 * 8 < a.nab) d[r] -= __ldg(lut + g8 * 256 + ((diff[r] >> (8 * g8)) & 255u));
             }
             // four bonds at a time: their ranks, then their up to 16 source elements, are in flight together
+            const int32_t *rank = a.ab_rank + cbase + cc;
+            const int ncols = (int)a.ncols;     // at most 32 x 2^16 table entries
             for (int q0 = 0; q0 < a.nab; q0 += 4) {
-                const uint32_t any4 = (any >> q0) & 15u;
-                if (!any4) continue;
                 int rk[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    rk[i] = ((any4 >> i) & 1u) ? __ldg(a.ab_rank + (int64_t)(q0 + i) * a.ncols + cbase + cc) : 0;
                 float v[4][4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < 4; ++i) rk[i] = (q0 + i < a.nab) ? __ldg(rank + (q0 + i) * ncols) : 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (q0 + i >= a.nab) break;
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
                         v[i][r] = 0.f;
-                        if ((diff[r] >> (q0 + i)) & 1u) {
-                            const int64_t src = ab_src[r * a.nab + q0 + i];
-                            if (src >= 0) v[i][r] = __ldg(x + src + rk[i]);
-                        }
+                        if ((diff[r] >> (q0 + i)) & 1u) v[i][r] = __ldg(x + (facts[r * a.nab + q0 + i].src + rk[i]));
                     }
+                }
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < 4; ++i) {
+                    if (q0 + i >= a.nab) break;
 #pragma unroll
-                    for (int r = 0; r < 4; ++r)
-                        if ((diff[r] >> (q0 + i)) & 1u) {
-                            d[r] -= ab_w2[q0 + i];
-                            acc[r] += ab_c[r * a.nab + q0 + i] * v[i][r];
-                        }
+                    for (int r = 0; r < 4; ++r) acc[r] += facts[r * a.nab + q0 + i].c * v[i][r];
+                }
             }
             if (ok) {
                 const float4 xv = xs4[cc];
@@ -1248,7 +1248,7 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     a.col_abbits = h.col_abbits;
     a.row_bbits = h.row_bbits;
     a.ab_rank = h.ab_rank;
-    a.ab_lut = h.ab_lut;
+    a.ab_lut = (sizeof(T) == 4) ? (const void *)h.ab_lut32 : (const void *)h.ab_lut;
     a.ncols = h.ncols;
     a.ab_fast = h.ab_fast ? 1 : 0;
     a.bb_cf = (sizeof(T) == 4) ? (const void *)h.bb_cf32 : (const void *)h.bb_cf64;
