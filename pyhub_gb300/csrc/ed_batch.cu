@@ -190,6 +190,12 @@ template <typename T, int R> __host__ __device__ constexpr int staged_stride()
     return ((R * (int)sizeof(T) / 16) % 2 == 0) ? R + 16 / (int)sizeof(T) : R;
 }
 
+// Shared memory of the H*v for rows of ld elements (FP32: and the zero columns).
+template <typename T, int R> static size_t hv_smem(int64_t ld)
+{
+    return (size_t)(ld + (sizeof(T) == 4 ? kZeroCols : 0)) * staged_stride<T, R>() * sizeof(T);
+}
+
 template <typename T, int R>
 __device__ __forceinline__ void load_column(const T *p, T (&v)[R])
 {
@@ -305,6 +311,8 @@ __device__ __forceinline__ void hv_item(const BatchInst *__restrict__ inst, int6
                 xs[c * S + r] = (T)0;
         }
     }
+    if (sizeof(T) == 4)      // the zero columns of the hop table's padding
+        for (int q = threadIdx.x; q < kZeroCols * S; q += blockDim.x) xs[zero_col(nsup) * S + q] = (T)0;
     for (int r = warp; r < R; r += nwarps) {
         int e0 = 0, nn = 0;
         if (r < nr) {
@@ -733,7 +741,7 @@ static int run_batch(ed_batch *bt, cudaStream_t st, T *work, const T *x0, int ns
     T *U[2] = {work, work + tot};
     T *Y = kept ? work : work + 2 * tot;
     double *pa = scratch, *pb = scratch + bt->nblocks, *scal = scratch + 2 * bt->nblocks;
-    const size_t smem = (size_t)bt->max_ld * staged_stride<T, R>() * sizeof(T);
+    const size_t smem = hv_smem<T, R>(bt->max_ld);
     const unsigned nb = (unsigned)bt->nblocks;
     const unsigned ns = (unsigned)((bt->ninst * 32 + 255) / 256);
     // two kept vectors: u_{k+1} overwrites u_{k-1} in place, so u_k lives in slot k % 2
@@ -776,10 +784,9 @@ static int rows_index(int rows) { return rows == 4 ? 0 : (rows == 8 ? 1 : 2); }
 
 static size_t hv_smem_bytes(int dtype, int64_t ld, int rows)
 {
-    static const int s32[3] = {staged_stride<float, 4>(), staged_stride<float, 8>(), staged_stride<float, 16>()};
-    static const int s64[3] = {staged_stride<double, 4>(), staged_stride<double, 8>(), staged_stride<double, 16>()};
     const int k = rows_index(rows);
-    return (dtype == ED_F32) ? (size_t)ld * s32[k] * sizeof(float) : (size_t)ld * s64[k] * sizeof(double);
+    if (dtype == ED_F32) return k == 0 ? hv_smem<float, 4>(ld) : k == 1 ? hv_smem<float, 8>(ld) : hv_smem<float, 16>(ld);
+    return k == 0 ? hv_smem<double, 4>(ld) : k == 1 ? hv_smem<double, 8>(ld) : hv_smem<double, 16>(ld);
 }
 
 template <typename T, int R>
@@ -1122,7 +1129,7 @@ static int run_persistent(ed_batch *bt, cudaStream_t st, T *work, const T *x0, i
     P.stall_inst = bt->stall_inst;
     ED_CHECK_CUDA(cudaMemsetAsync(ints, 0, sizeof(int) * (2 * (size_t)bt->ninst + 4), st));
     if (bt->nblocks == 0) return ED_OK;
-    const size_t smem = (size_t)bt->max_ld * staged_stride<T, R>() * sizeof(T);
+    const size_t smem = hv_smem<T, R>(bt->max_ld);
     auto kfn = batch_persistent_kernel<T, R>;
     ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;

@@ -67,7 +67,7 @@ struct HopTable {
     // The same table in sliced-ELL form for the row pass: strings in slices of
     // 32; slice s holds width[s] slots, slot-major, so that the 32 lanes of a
     // warp read one slot with one coalesced load.  Padding slots point at the
-    // string itself with coefficient 0.
+    // string itself with coefficient 0; in ell_pk32 at a zero column.
     int64_t nslice = 0, ell_slots = 0;
     int32_t *ell_off = nullptr;    // [nslice+1] first slot of each slice
     int32_t *ell_src = nullptr;    // [ell_slots*32]
@@ -146,6 +146,11 @@ struct UijklTables {
 
 int uijkl_hv(ed_sector *s, cudaStream_t st, int dtype, int64_t ld, const void *x, void *y, double scale);
 void uijkl_free(UijklTables *u);
+
+// Slots of a packed FP32 hop table without a hop: the kernels stage kZeroCols zero columns from zero_col(n)
+// on (n staged columns), one per residue mod 8, and such a slot reads one of them.
+constexpr int kZeroCols = 8;
+__host__ __device__ inline int64_t zero_col(int64_t n) { return (n + 7) / 8 * 8; }
 
 int heis_struct_build(ed_sector *s);
 void heis_struct_free(HeisStruct *hs);

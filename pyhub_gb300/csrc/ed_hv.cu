@@ -113,6 +113,10 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
     const int64_t nsup = a.nsup, ld = a.ld;
     const T uval = (T)a.u_value, sc = (T)a.scale;
     const T *ued_t = static_cast<const T *>(a.uediag), *ded_t = static_cast<const T *>(a.dediag);
+    if (sizeof(T) == 4 && threadIdx.x < kZeroCols) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) xs[r * sld + zero_col(nsup) + threadIdx.x] = (T)0;
+    }
     for (int64_t d0 = (int64_t)blockIdx.x * R; d0 < a.nsdn; d0 += (int64_t)gridDim.x * R) {
         const int nr = (int)min((int64_t)R, a.nsdn - d0);
 #pragma unroll
@@ -185,7 +189,8 @@ __global__ void __launch_bounds__(1024) hub_row_col4_kernel(const float *__restr
                                                             const HubArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4 *xs4 = reinterpret_cast<float4 *>(smem_raw);   // [nsup]
+    float4 *xs4 = reinterpret_cast<float4 *>(smem_raw);   // [nsup], then the zero columns
+    if (threadIdx.x < kZeroCols) xs4[zero_col(a.nsup) + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int64_t nsup = a.nsup, ld = a.ld;
     const float uval = (float)a.u_value, sc = (float)a.scale;
@@ -591,7 +596,7 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     const int nsm = num_sms();
     constexpr int VWS = 16 / sizeof(T);
     // ---- pass 1
-    const int64_t sld = (s->nsup + VWS - 1) / VWS * VWS;
+    const int64_t sld = sizeof(T) == 4 ? zero_col(s->nsup) + kZeroCols : (s->nsup + VWS - 1) / VWS * VWS;
     const bool vec_ok = (ld % VWS == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const int maxsm = max_smem();
     const size_t row_bytes = (size_t)sld * sizeof(T);
@@ -623,9 +628,10 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     constexpr int R2 = 2;
     const bool two = (size_t)R2 * row_bytes * 2 <= (size_t)maxsm;
     const int threads = 512;
-    if (sizeof(T) == 4 && (size_t)s->nsup * 16 <= (size_t)maxsm) {
+    const size_t smem4 = (size_t)(zero_col(s->nsup) + kZeroCols) * 16;
+    if (sizeof(T) == 4 && smem4 <= (size_t)maxsm) {
         // four rows per 1024-thread CTA, staged as 16-byte columns
-        const size_t smem = (size_t)s->nsup * 16;
+        const size_t smem = smem4;
         int64_t blocks = (s->nsdn + 3) / 4;
         if (blocks > nsm) blocks = nsm;
         ED_CHECK_CUDA(cudaFuncSetAttribute(hub_row_col4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

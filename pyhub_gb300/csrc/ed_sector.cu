@@ -247,6 +247,131 @@ static uint64_t hash_structure(const HostHop &h)
     return x;
 }
 
+// The slots of a lane's hops may come in any order, so each slot is filled to spread the lanes' sources
+// over the shared-memory banks of the kernels that gather them.  They gather a 16-byte column piece
+// per lane, 8 lanes (a quarter warp) at a time, and a column's bank group is (source mod 8) (the
+// column strides are odd multiples of 16 bytes): a slot of a quarter is read at once when its sources
+// differ mod 8.  With a hop as an edge between its lane and its residue, such an order is an edge
+// colouring of a bipartite multigraph, and one with max(degree) colours exists (Konig); it is found by
+// flipping alternating paths.  A residue with more hops than slots keeps its surplus as conflicts.  A
+// lane without a hop in a slot reads a zero column of a free residue.  Conflicts per quarter read at
+// 16 sites (4x4): 0.53 filled greedily with the lane's own string as padding, 0.02 so; the FP32 row
+// pass 1,100 -> 936 us, the batched product 2,560 -> 2,350 us (padding skipped by a test instead: 1,147
+// and 2,454, the test keeps a group's gathers from being issued together).
+// The quarters' colours are then lined up so that a slot's 32 sources differ mod 32 where they can
+// (kernels that gather a 4-byte word per lane).
+// slot[k * 32 + l]: the place in lane l's list of the hop it takes in slot k, or -1 (w slots, at least
+// as many as any lane has hops).
+static void ell_color_slice(const std::vector<int32_t> (&src)[32], int w, std::vector<int32_t> &slot)
+{
+    slot.assign((size_t)std::max(w, 0) * 32, -1);
+    std::vector<uint32_t> used32((size_t)std::max(w, 0), 0u);
+    struct Edge {
+        int lane, res, j;
+    };
+    std::vector<Edge> edges;
+    std::vector<int> over;
+    std::vector<int> at_l, at_r;     // [8][w]: edge of a colour at a lane / residue, -1 free
+    for (int q = 0; q < 4; ++q) {
+        edges.clear();
+        over.clear();
+        int deg[8] = {}, colours = 0;
+        for (int l = 0; l < 8; ++l) {
+            const std::vector<int32_t> &L = src[q * 8 + l];
+            colours = std::max(colours, (int)L.size());
+            for (size_t j = 0; j < L.size(); ++j) edges.push_back({l, L[j] & 7, (int)j});
+        }
+        at_l.assign((size_t)8 * std::max(w, 1), -1);
+        at_r.assign((size_t)8 * std::max(w, 1), -1);
+        for (size_t i = 0; i < edges.size(); ++i) {
+            const Edge e = edges[i];
+            if (deg[e.res] >= w) {
+                over.push_back((int)i);
+                continue;
+            }
+            colours = std::max(colours, ++deg[e.res]);
+            int *L = &at_l[(size_t)e.lane * w], *R = &at_r[(size_t)e.res * w];
+            int a = 0, b = 0;        // a free at the lane, b free at the residue
+            while (L[a] >= 0) ++a;
+            while (R[b] >= 0) ++b;
+            if (R[a] >= 0) {
+                // swap colours a and b along the path that starts with the residue's edge of colour a
+                // (it cannot reach the lane, which has none)
+                int carry = R[a], c = a;
+                bool at_res = true;
+                R[a] = -1;
+                while (carry >= 0) {
+                    const int c2 = c == a ? b : a;
+                    const Edge &f = edges[(size_t)carry];
+                    int *near_side = at_res ? &at_r[(size_t)f.res * w] : &at_l[(size_t)f.lane * w];
+                    int *far_side = at_res ? &at_l[(size_t)f.lane * w] : &at_r[(size_t)f.res * w];
+                    if (far_side[c] == carry) far_side[c] = -1;
+                    const int next = far_side[c2];
+                    near_side[c2] = carry;
+                    far_side[c2] = carry;
+                    carry = next;
+                    c = c2;
+                    at_res = !at_res;
+                }
+            }
+            L[a] = (int)i;
+            R[a] = (int)i;
+        }
+        for (int i : over) {
+            int *L = &at_l[(size_t)edges[(size_t)i].lane * w];
+            int a = 0;
+            while (L[a] >= 0) ++a;
+            L[a] = i;
+            colours = std::max(colours, a + 1);
+        }
+        // colour -> slot (within the quarter's first `colours` slots)
+        std::vector<char> taken((size_t)std::max(w, 1), 0);
+        for (int k = 0; k < colours; ++k) {
+            int pick = -1, best = 1 << 30;
+            uint32_t bits = 0;
+            for (int c = 0; c < colours; ++c) {
+                if (taken[(size_t)c]) continue;
+                uint32_t m = 0;
+                int clash = 0;
+                for (int l = 0; l < 8; ++l) {
+                    const int i = at_l[(size_t)l * w + c];
+                    if (i < 0) continue;
+                    const uint32_t bit = 1u << (src[q * 8 + l][(size_t)edges[(size_t)i].j] & 31);
+                    clash += ((used32[(size_t)k] | m) & bit) ? 1 : 0;
+                    m |= bit;
+                }
+                if (clash < best) {
+                    best = clash;
+                    pick = c;
+                    bits = m;
+                }
+                if (best == 0) break;
+            }
+            taken[(size_t)pick] = 1;
+            used32[(size_t)k] |= bits;
+            for (int l = 0; l < 8; ++l) {
+                const int i = at_l[(size_t)l * w + pick];
+                if (i >= 0) slot[(size_t)k * 32 + q * 8 + l] = edges[(size_t)i].j;
+            }
+        }
+    }
+}
+
+// The zero columns that a slot's lanes without a hop (-1) read: one whose residue no other lane of the
+// quarter uses.
+static void ell_fill_padding(int32_t (&src)[32], int64_t n)
+{
+    for (int q = 0; q < 4; ++q) {
+        unsigned used = 0;
+        for (int l = 8 * q; l < 8 * q + 8; ++l)
+            if (src[l] >= 0) used |= 1u << (src[l] & 7);
+        int r = 0;       // a quarter with a padding lane has at most seven sources
+        while (r < 7 && ((used >> r) & 1u)) ++r;
+        for (int l = 8 * q; l < 8 * q + 8; ++l)
+            if (src[l] < 0) src[l] = (int32_t)(zero_col(n) + r);
+    }
+}
+
 static std::shared_ptr<const EllOrder> ell_order(const HostHop &h)
 {
     const uint64_t key = hash_structure(h);
@@ -271,67 +396,20 @@ static std::shared_ptr<const EllOrder> ell_order(const HostHop &h)
     }
     const int64_t slots = off[(size_t)ns];
     o->entry.assign((size_t)std::max<int64_t>(slots * 32, 1), -1);
-    // Slot order within a lane is free, so each slot is filled to spread the
-    // 32 lanes' sources over the shared-memory banks of the kernels that
-    // gather them:
-    //   * the batched kernel gathers 16-byte column pieces for 8 lanes at a
-    //     time (one quarter warp); a column's bank group is (source mod 8);
-    //   * the row kernels gather one 4- or 8-byte word per lane from a staged
-    //     row; its bank is (source mod 32) for FP32.
-    // Greedy per slot, lanes with the most neighbours left first: prefer a
-    // neighbour whose (source mod 32) no lane of the warp and whose
-    // (source mod 8) no lane of the quarter uses yet, then one that is new
-    // for the quarter only, then one new for the warp only.  Padding slots
-    // read the lane's own string (consecutive strings: distinct banks) with
-    // weight 0.
+    std::vector<int32_t> srcs[32], slot;
     for (int64_t sl = 0; sl < ns; ++sl) {
-        const int64_t w = off[(size_t)sl + 1] - off[(size_t)sl];
-        std::vector<std::vector<int32_t>> left(32);   // remaining neighbour entries (hop-table positions)
+        const int w = off[(size_t)sl + 1] - off[(size_t)sl];
         for (int l = 0; l < 32; ++l) {
             const int64_t u = sl * 32 + l;
-            if (u >= n) continue;
-            for (int32_t e = h.ptr[(size_t)u]; e < h.ptr[(size_t)u + 1]; ++e) left[(size_t)l].push_back(e);
+            srcs[l].clear();
+            if (u < n) srcs[l].assign(h.src.begin() + h.ptr[(size_t)u], h.src.begin() + h.ptr[(size_t)u + 1]);
         }
-        for (int64_t k = 0; k < w; ++k) {
-            bool used32[32] = {};
-            bool used8[4][8] = {};
-            int order[32];
-            {
-                // lanes by remaining neighbours, most first (stable within equal counts)
-                int m = 0;
-                for (int64_t cnt = w; cnt >= 0 && m < 32; --cnt)
-                    for (int l = 0; l < 32; ++l)
-                        if ((int64_t)left[(size_t)l].size() == cnt) order[m++] = l;
+        ell_color_slice(srcs, w, slot);
+        for (int k = 0; k < w; ++k)
+            for (int l = 0; l < 32; ++l) {
+                const int32_t j = slot[(size_t)(k * 32 + l)];
+                if (j >= 0) o->entry[(size_t)((off[(size_t)sl] + k) * 32 + l)] = h.ptr[(size_t)(sl * 32 + l)] + j;
             }
-            for (int oi = 0; oi < 32; ++oi) {
-                const int l = order[oi], qw = l >> 3;
-                const int64_t u = sl * 32 + l;
-                const size_t at = (size_t)((off[(size_t)sl] + k) * 32 + l);
-                const int64_t uu = u < n ? u : n - 1;
-                std::vector<int32_t> &L = left[(size_t)l];
-                const bool must = (int64_t)L.size() >= w - k;   // no spare slot left for this lane
-                int pick = -1, best = -1;
-                for (size_t j = 0; j < L.size(); ++j) {
-                    const int32_t sj = h.src[(size_t)L[j]];
-                    const int score = (used8[qw][sj & 7] ? 0 : 2) + (used32[sj & 31] ? 0 : 1);
-                    if (score > best) { best = score; pick = (int)j; }
-                    if (score == 3) break;
-                }
-                const int pad_score = (used8[qw][uu & 7] ? 0 : 2) + (used32[uu & 31] ? 0 : 1);
-                if (pick >= 0 && !must && best < pad_score) pick = -1;   // padding now is the cleaner choice
-                int32_t sat;
-                if (pick >= 0) {
-                    const int32_t e = L[(size_t)pick];
-                    L.erase(L.begin() + pick);
-                    o->entry[at] = e;
-                    sat = h.src[(size_t)e];
-                } else {
-                    sat = (int32_t)uu;
-                }
-                used8[qw][sat & 7] = true;
-                used32[sat & 31] = true;
-            }
-        }
     }
     std::lock_guard<std::mutex> lk(g_ell_mu);
     // a sweep over many different lattices must not grow the cache without bound: past
@@ -369,11 +447,16 @@ static int upload_ell(const HostHop &h, HopTable &d, TablePool &pool)
                 }
             }
     std::vector<float> c32(c64.begin(), c64.end());
-    std::vector<int2> pk(src.size());
-    for (size_t q = 0; q < src.size(); ++q) {
-        int32_t bits;
-        std::memcpy(&bits, &c32[q], sizeof(bits));
-        pk[q] = make_int2(src[q], bits);
+    std::vector<int2> pk(src.size(), make_int2(0, 0));
+    for (int64_t k = 0; k < slots; ++k) {
+        int32_t sk[32];
+        for (int l = 0; l < 32; ++l) sk[l] = o->entry[(size_t)(k * 32 + l)] >= 0 ? src[(size_t)(k * 32 + l)] : -1;
+        ell_fill_padding(sk, n);
+        for (int l = 0; l < 32; ++l) {
+            int32_t bits;
+            std::memcpy(&bits, &c32[(size_t)(k * 32 + l)], sizeof(bits));
+            pk[(size_t)(k * 32 + l)] = make_int2(sk[l], bits);
+        }
     }
     d.nslice = ns;
     d.ell_slots = slots;
