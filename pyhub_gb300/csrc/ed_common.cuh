@@ -269,6 +269,7 @@ __device__ __forceinline__ double sum_rows_cta(const double *__restrict__ v, int
 }
 
 int num_sms();
+int max_smem();      // largest shared memory a kernel may ask for on the current device (ed_hv.cu)
 
 // Empty-site pattern of a string of norb sites (site POS in bit norb-POS):
 // bit j set when site j+1 is empty.

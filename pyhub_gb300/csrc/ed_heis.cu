@@ -209,7 +209,7 @@ int heis_struct_build(ed_sector *s)
             for (size_t c = 0; c < col_pat.size(); ++c)
                 ab_rank[q * col_pat.size() + c] = rankA[col_pat[c] ^ (1u << (ht.bj[ab[q]] - 1))];
         hs->ncols = (int64_t)col_pat.size();
-        if (!ab.empty()) ab_lut.assign(4 * 256, 0.0);
+        ab_lut.assign(4 * 256, 0.0);      // also without A-B bonds: the kernels always look the first eight up
         for (size_t k = 0; k < ab_lut.size(); ++k)
             for (size_t q = 0; q < 8; ++q) {
                 const size_t bond = k / 256 * 8 + q;
@@ -408,6 +408,16 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
             T d = __ldg(static_cast<const T *>(a.diagA) + cbase + cc) + db;
             T acc = 0;
             const int s0 = __ldg(a.aa_off + sbase + sl), ns = __ldg(a.aa_off + sbase + sl + 1) - s0;
+            // antiparallel A-B bonds: the set bits of (column's A bits ^ row's B bits); their zz/4 was counted
+            // as "equal" in diagB, so each one drops the diagonal by zz/2.  Eight bonds' drops come from a
+            // table; the first look-up is in flight during the A-A flips
+            const T *lut = static_cast<const T *>(a.ab_lut);
+            uint32_t diff = 0u;
+            T drop = 0;
+            if (a.ab_fast) {
+                diff = __ldg(a.col_abbits + cbase + cc) ^ rbits;
+                drop = __ldg(lut + (diff & 255u));
+            }
             if (sizeof(T) == 4) {
 #pragma unroll 4
                 for (int q = 0; q < ns; ++q) {
@@ -422,12 +432,8 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
                 }
             }
             if (a.ab_fast) {
-                // antiparallel A-B bonds: the set bits of (column's A bits ^ row's B bits); their
-                // zz/4 was counted as "equal" in diagB, so each one drops the diagonal by zz/2
-                uint32_t diff = __ldg(a.col_abbits + cbase + cc) ^ rbits;
-                // eight bonds' zz drops from a table: one subtraction for them
-                const T *lut = static_cast<const T *>(a.ab_lut);
-                for (int g = 0; g * 8 < a.nab; ++g) d -= __ldg(lut + g * 256 + ((diff >> (8 * g)) & 255u));
+                d -= drop;
+                for (int g = 1; g * 8 < a.nab; ++g) d -= __ldg(lut + g * 256 + ((diff >> (8 * g)) & 255u));
                 while (diff) {
                     const int q = __ffs(diff) - 1;
                     diff &= diff - 1;
@@ -635,9 +641,12 @@ struct SlabPlan {
     int64_t slab_w[kMaxHalf + 1], ngroups[kMaxHalf + 1];
 };
 
+constexpr int kHeisSlabCtas = 3;     // CTAs per SM: up to 80 registers a thread
+
 template <typename T>
-__global__ void __launch_bounds__(256) heis_slab_kernel(const T *__restrict__ x, T *__restrict__ y, const HsArgs a,
-                                                        const SlabPlan p, double *__restrict__ partials)
+__global__ void __launch_bounds__(256, kHeisSlabCtas) heis_slab_kernel(const T *__restrict__ x, T *__restrict__ y,
+                                                                       const HsArgs a, const SlabPlan p,
+                                                                       double *__restrict__ partials)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const T *bcf = reinterpret_cast<const T *>(a.bb_cf);
@@ -1259,17 +1268,14 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     a.scale = scale;
     for (int m = 0; m <= h.nA; ++m) a.m_order[m] = (int8_t)m;
     std::sort(a.m_order, a.m_order + h.nA + 1, [&](int8_t x, int8_t y) { return h.ncol[x] > h.ncol[y]; });
-    // rows by length give the CTAs even shares (FP64: 4x6 157 -> 149 us, 4x7 3.69 -> 3.51 ms); vectors far
-    // above L2 keep memory order, where the A-B bonds' source rows are near (4x8: 60 ms, by length 67)
-    a.by_length = (double)s->dim * sizeof(T) <= 1.0e9 ? 1 : 0;
     const int nsm = num_sms();
+    // rows by length give the CTAs even shares (FP64: 4x6 157 -> 149 us, 4x7 3.69 -> 3.51 ms); vectors far
+    // above L2 keep memory order, where the A-B bonds' source rows are near (4x8: 60 ms, by length 67), and
+    // so do rows that have a CTA each (4x4: the row pass 5.5 us, by length 6.6: the look-up leads the chain
+    // of loads)
+    a.by_length = (double)s->dim * sizeof(T) <= 1.0e9 && h.nrows > (int64_t)nsm * 4 ? 1 : 0;
     // ---- pass R
-    int maxsm = 0;
-    {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    }
+    const int maxsm = max_smem();
     const size_t smem4 = heis_col4_head_bytes(h.nab) + (size_t)std::max<int64_t>(h.max_len, 1) * 16;
     // FP32 with the packed A-B path: four rows of one hole count per CTA when their columns
     // fit (PYHUB_ED_HEIS_ROWS=1 selects the one-row pass; both give the same product)
@@ -1277,20 +1283,19 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     if (sizeof(T) == 4 && h.ab_fast && smem4 <= (size_t)maxsm && !(one && one[0] == '1')) {
         int64_t nitems = 0;
         for (int m = 0; m <= h.nA; ++m) nitems += (h.row_base[m + 1] - h.row_base[m] + 3) / 4;
-        ED_CHECK_CUDA(cudaFuncSetAttribute(heis_row_col4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem4));
+        if (smem4 > 48 * 1024)
+            ED_CHECK_CUDA(cudaFuncSetAttribute(heis_row_col4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem4));
         // two CTAs of 512 threads per SM where two groups of rows fit (one stages while the other works)
         const int threads = 2 * (smem4 + 1024) <= (size_t)maxsm ? 512 : kHeisCol4Threads;
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, heis_row_col4_kernel, threads, smem4);
-        if (per_sm < 1) per_sm = 1;
-        int64_t blocks = std::min<int64_t>(nitems, (int64_t)nsm * per_sm);
+        int64_t blocks = std::min<int64_t>(nitems, (int64_t)nsm * (threads == 512 ? 2 : 1));
         if (blocks < 1) blocks = 1;
         heis_row_col4_kernel<<<(unsigned)blocks, threads, smem4, st>>>(
             reinterpret_cast<const float *>(x), reinterpret_cast<float *>(y), a, nitems);
     } else {
         const size_t smem = heis_row_head_bytes(h.nab, sizeof(T)) + (size_t)std::max<int64_t>(h.max_len, 1) * sizeof(T);
-        ED_CHECK_CUDA(cudaFuncSetAttribute(heis_row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 48 * 1024)
+            ED_CHECK_CUDA(cudaFuncSetAttribute(heis_row_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int64_t blocks = std::min<int64_t>(h.nrows, (int64_t)nsm * 4);
         if (blocks < 1) blocks = 1;
         heis_row_kernel<T><<<(unsigned)blocks, kHeisRowThreads, smem, st>>>(x, y, a);
@@ -1302,9 +1307,7 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     SlabPlan p;
     p.nblk = 0;
     p.item_base[0] = 0;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, heis_slab_kernel<T>, 256, 0);
-    int64_t blocks2 = std::min<int64_t>((int64_t)nsm * std::max(per_sm, 1), kMaxPartialBlocksHeis);
+    int64_t blocks2 = std::min<int64_t>((int64_t)nsm * kHeisSlabCtas, kMaxPartialBlocksHeis);
     int64_t groups = 0;
     for (int m = 0; m <= h.nA; ++m) groups += (h.row_base[m + 1] - h.row_base[m] + 7) / 8;
     const int64_t cuts = std::max<int64_t>(1, 8 * blocks2 / std::max<int64_t>(groups, 1));

@@ -536,7 +536,7 @@ static double slab_l2_bytes()
 }
 
 // Largest shared memory a kernel may ask for on the current device.
-static int max_smem()
+int max_smem()
 {
     static std::atomic<int> known[64];
     int dev = 0;
