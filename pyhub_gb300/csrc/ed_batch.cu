@@ -39,10 +39,10 @@ struct BatchInst {
     const float *uediag32, *dediag32;
     const double *u_site;             // device, indexed by bit
     const float *u_site32;
-    const int32_t *ell_off, *ell_src; // sliced-ELL up-hop table of the sector
-    const float *ell_cf32;
-    const double *ell_cf64;
+    const int32_t *ell_off;           // sliced-ELL up-hop tables of the sector, FP32
     const int2 *ell_pk32;
+    const int32_t *ell64_off, *ell64_col, *ell64_src;   // and FP64
+    const double *ell64_cf;
     int nslice;
     double u_value;
     float u_value32;
@@ -223,8 +223,8 @@ __device__ __forceinline__ void up_group(const BatchInst &a, const T *xs, int at
             src[j] = pk.x;
             w[j] = (T)__int_as_float(pk.y);
         } else {
-            src[j] = __ldg(a.ell_src + at + 32 * j);
-            w[j] = (T)__ldg(a.ell_cf64 + at + 32 * j);
+            src[j] = __ldg(a.ell64_src + at + 32 * j);
+            w[j] = (T)__ldg(a.ell64_cf + at + 32 * j);
         }
     }
 #pragma unroll
@@ -350,8 +350,8 @@ __device__ __forceinline__ void hv_item(const BatchInst *__restrict__ inst, int6
     __syncthreads();
     // ---- phase A
     for (int sl = warp; sl < a.nslice; sl += nwarps) {
-        const int c = sl * 32 + lane;
-        const bool ok = c < nsup;
+        const int c = sizeof(T) == 4 ? sl * 32 + lane : __ldg(a.ell64_col + sl * 32 + lane);
+        const bool ok = sizeof(T) == 4 ? c < nsup : c >= 0;
         const int cc = ok ? c : nsup - 1;
         const uint32_t su = __ldg(a.ustr + cc);
         const T ued = __ldg(ued_t + cc);
@@ -359,7 +359,8 @@ __device__ __forceinline__ void hv_item(const BatchInst *__restrict__ inst, int6
         load_column<T, R>(xs + cc * S, xv);
 #pragma unroll
         for (int r = 0; r < R; ++r) acc[r] = (ued + row_ed[r] + u_energy_b<T>(a, su & row_str[r])) * xv[r];
-        const int s0 = __ldg(a.ell_off + sl), ns = __ldg(a.ell_off + sl + 1) - s0;
+        const int32_t *off = sizeof(T) == 4 ? a.ell_off : a.ell64_off;
+        const int s0 = __ldg(off + sl), ns = __ldg(off + sl + 1) - s0;
         // slots in groups: all table loads of a group are in flight before
         // its first gather
         int q = 0;
@@ -867,8 +868,9 @@ extern "C" int ed_batch_create_rows(int ninst, ed_sector *const *secs, int rows,
         a.ucf32 = s->up.cf32; a.dcf32 = s->dn.cf32; a.ucf64 = s->up.cf64; a.dcf64 = s->dn.cf64;
         a.uediag = s->up.ediag; a.dediag = s->dn.ediag;
         a.uediag32 = s->up.ediag32; a.dediag32 = s->dn.ediag32;
-        a.ell_off = s->up.ell_off; a.ell_src = s->up.ell_src;
-        a.ell_cf32 = s->up.ell_cf32; a.ell_cf64 = s->up.ell_cf64;
+        a.ell_off = s->up.ell_off;
+        a.ell64_off = s->up.ell64_off; a.ell64_col = s->up.ell64_col;
+        a.ell64_src = s->up.ell64_src; a.ell64_cf = s->up.ell64_cf;
         a.ell_pk32 = s->up.ell_pk32;
         a.nslice = (int)s->up.nslice;
         for (int q = 0; q < kMaxSites; ++q) {

@@ -66,14 +66,17 @@ struct HopTable {
     float *ediag32 = nullptr;  // [n]  the same, rounded to FP32 (FP32 kernels read it directly)
     // The same table in sliced-ELL form for the row pass: strings in slices of
     // 32; slice s holds width[s] slots, slot-major, so that the 32 lanes of a
-    // warp read one slot with one coalesced load.  Padding slots point at the
-    // string itself with coefficient 0; in ell_pk32 at a zero column.
-    int64_t nslice = 0, ell_slots = 0;
+    // warp read one slot with one coalesced load.  FP32: strings in order, one
+    // 8-byte load per slot, slots without a hop at a zero column.  FP64: strings
+    // by number of hops, slots without a hop at the string itself
+    // with coefficient 0.
+    int64_t nslice = 0;
     int32_t *ell_off = nullptr;    // [nslice+1] first slot of each slice
-    int32_t *ell_src = nullptr;    // [ell_slots*32]
-    float *ell_cf32 = nullptr;
-    double *ell_cf64 = nullptr;
-    int2 *ell_pk32 = nullptr;      // [ell_slots*32] {src, FP32 coefficient bits}: one 8-byte load per slot
+    int2 *ell_pk32 = nullptr;      // [slots*32] {src, FP32 coefficient bits}
+    int32_t *ell64_off = nullptr;  // [nslice+1]
+    int32_t *ell64_col = nullptr;  // [nslice*32] string of each lane, -1 past the last
+    int32_t *ell64_src = nullptr;  // [slots*32]
+    double *ell64_cf = nullptr;
     // Per ordered site pair (J,K), J != K, at index (J-1)*norb + (K-1): the
     // strings u with J occupied and K empty, as {u, u' | sign << 31} with
     // u' = u - J + K and sign = parity of the occupied sites strictly between

@@ -27,7 +27,9 @@ struct HubArgs {
     const uint32_t *ustr; const int32_t *uptr; const int32_t *usrc; const void *ucf; const void *uediag;
     const uint32_t *dstr; const int32_t *dptr; const int32_t *dsrc; const void *dcf; const void *dediag;
     int64_t nslice;
-    const int32_t *ell_off; const int32_t *ell_src; const void *ell_cf;
+    const int32_t *ell_off;        // of the type's table
+    const int32_t *ell64_col, *ell64_src;
+    const double *ell64_cf;
     const int2 *ell_pk32;
     const void *u_lut;        // [4][256], then U times a count; float or double like the vectors
     int nbytes;               // bytes of a string with an on-site interaction (1 when there is none: zeros)
@@ -77,8 +79,7 @@ __device__ __forceinline__ void stage_row(T *dst, const T *__restrict__ src, int
 // staged rows; the G table loads are issued before the first gather (FP32:
 // one packed 8-byte {source, coefficient} load per slot).
 template <typename T, int R, int G>
-__device__ __forceinline__ void row_group(const HubArgs &a, const T *__restrict__ ecf, int64_t at, const T *xs,
-                                          int64_t sld, T (&acc)[R])
+__device__ __forceinline__ void row_group(const HubArgs &a, int64_t at, const T *xs, int64_t sld, T (&acc)[R])
 {
     int q[G];
     T c[G];
@@ -89,8 +90,8 @@ __device__ __forceinline__ void row_group(const HubArgs &a, const T *__restrict_
             q[i] = pk.x;
             c[i] = (T)__int_as_float(pk.y);
         } else {
-            q[i] = __ldg(a.ell_src + at + i * 32);
-            c[i] = __ldg(ecf + at + i * 32);
+            q[i] = __ldg(a.ell64_src + at + i * 32);
+            c[i] = (T)__ldg(a.ell64_cf + at + i * 32);
         }
     }
 #pragma unroll
@@ -108,7 +109,6 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *xs = reinterpret_cast<T *>(smem_raw);
-    const T *__restrict__ ecf = static_cast<const T *>(a.ell_cf);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int64_t nsup = a.nsup, ld = a.ld;
     const T uval = (T)a.u_value, sc = (T)a.scale;
@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
             ed[r] = (r < nr) ? __ldg(ded_t + d0 + r) : (T)0;
         }
         for (int64_t sl = warp; sl < a.nslice; sl += nwarps) {
-            const int64_t u = sl * 32 + lane;
-            const bool ok = u < nsup;
+            const int64_t u = sizeof(T) == 4 ? sl * 32 + lane : (int64_t)__ldg(a.ell64_col + sl * 32 + lane);
+            const bool ok = sizeof(T) == 4 ? u < nsup : u >= 0;
             const int64_t uu = ok ? u : nsup - 1;
             const uint32_t su = __ldg(a.ustr + uu);
             const T eu = __ldg(ued_t + uu);
@@ -143,12 +143,12 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
             const int64_t at0 = (int64_t)s0 * 32 + lane;
             // slots in groups: all table loads of a group are in flight before its first gather
             int k = 0;
-            for (; k + 8 <= ns; k += 8) row_group<T, R, 8>(a, ecf, at0 + k * 32, xs, sld, acc);
+            for (; k + 8 <= ns; k += 8) row_group<T, R, 8>(a, at0 + k * 32, xs, sld, acc);
             if (k + 4 <= ns) {
-                row_group<T, R, 4>(a, ecf, at0 + k * 32, xs, sld, acc);
+                row_group<T, R, 4>(a, at0 + k * 32, xs, sld, acc);
                 k += 4;
             }
-            for (; k < ns; ++k) row_group<T, R, 1>(a, ecf, at0 + k * 32, xs, sld, acc);
+            for (; k < ns; ++k) row_group<T, R, 1>(a, at0 + k * 32, xs, sld, acc);
             if (ok) {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
@@ -584,9 +584,10 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     a.dcf = (sizeof(T) == 4) ? (const void *)s->dn.cf32 : (const void *)s->dn.cf64;
     a.ucf = (sizeof(T) == 4) ? (const void *)s->up.cf32 : (const void *)s->up.cf64;
     a.nslice = s->up.nslice;
-    a.ell_off = s->up.ell_off;
-    a.ell_src = s->up.ell_src;
-    a.ell_cf = (sizeof(T) == 4) ? (const void *)s->up.ell_cf32 : (const void *)s->up.ell_cf64;
+    a.ell_off = (sizeof(T) == 4) ? s->up.ell_off : s->up.ell64_off;
+    a.ell64_col = s->up.ell64_col;
+    a.ell64_src = s->up.ell64_src;
+    a.ell64_cf = s->up.ell64_cf;
     a.ell_pk32 = s->up.ell_pk32;
     a.u_lut = (sizeof(T) == 4) ? (const void *)s->u_lut32 : (const void *)s->u_lut;
     a.nbytes = (s->u_uniform && s->u_value == 0.0) ? 1 : (s->norb + 7) / 8;

@@ -217,14 +217,18 @@ struct TablePool {
     }
 };
 
-// Slot layout of a sliced-ELL table: slice offsets and, per (slot, lane),
-// the hop-table entry it holds (-1: padding).  It depends only on the hop
+// Slot layouts of the sliced-ELL tables: slice offsets and, per (slot, lane),
+// the hop-table entry it holds (-1: padding).  They depend only on the hop
 // structure (ptr, src), not on the coefficients, so sectors that share a
-// lattice and particle number (every cluster of a parameter sweep) share it.
-struct EllOrder {
-    std::vector<int32_t> ptr, src;   // the structure it was built for
+// lattice and particle number (every cluster of a parameter sweep) share them.
+struct EllSlots {
     std::vector<int32_t> off;        // [nslice+1]
     std::vector<int32_t> entry;      // [slots*32]
+};
+struct EllOrder {
+    std::vector<int32_t> ptr, src;   // the structure it was built for
+    EllSlots plain, sorted;          // columns in order (FP32), by number of hops (FP64)
+    std::vector<int32_t> cols;       // [nslice*32] column of each lane of `sorted`, -1 past the last
 };
 
 static std::mutex g_ell_mu;
@@ -372,6 +376,58 @@ static void ell_fill_padding(int32_t (&src)[32], int64_t n)
     }
 }
 
+// Slots of all slices.  Lane l of slice s has column cols[s * 32 + l], none below 0, its hops in order; with
+// cols == NULL column s * 32 + l, its hops by colour (the FP64 products have no use for that: 372 us at 14
+// sites either way).
+static EllSlots ell_slots_of(const HostHop &h, const int32_t *cols)
+{
+    const int64_t n = (int64_t)h.str.size(), ns = (n + 31) / 32;
+    EllSlots o;
+    o.off.assign((size_t)ns + 1, 0);
+    std::vector<int32_t> srcs[32], slot;
+    for (int64_t sl = 0; sl < ns; ++sl) {
+        int64_t at[32];
+        size_t w = 0;
+        for (int l = 0; l < 32; ++l) {
+            const int64_t u = cols ? cols[sl * 32 + l] : (sl * 32 + l < n ? sl * 32 + l : -1);
+            srcs[l].clear();
+            at[l] = u < 0 ? 0 : h.ptr[(size_t)u];
+            if (u >= 0) srcs[l].assign(h.src.begin() + h.ptr[(size_t)u], h.src.begin() + h.ptr[(size_t)u + 1]);
+            w = std::max(w, srcs[l].size());
+        }
+        o.off[(size_t)sl + 1] = o.off[(size_t)sl] + (int32_t)w;
+        if (cols) {
+            slot.assign(w * 32, -1);
+            for (int l = 0; l < 32; ++l)
+                for (size_t j = 0; j < srcs[l].size(); ++j) slot[j * 32 + (size_t)l] = (int32_t)j;
+        } else {
+            ell_color_slice(srcs, (int)w, slot);
+        }
+        for (size_t k = 0; k < w; ++k)
+            for (int l = 0; l < 32; ++l) {
+                const int32_t j = slot[k * 32 + (size_t)l];
+                o.entry.push_back(j >= 0 ? (int32_t)at[l] + j : -1);
+            }
+    }
+    return o;
+}
+
+// Columns of the FP64 table's lanes, by number of hops: a slice has as many slots as its longest list, and
+// a warp's FP64 operation costs the pipe the same for one lane as for 32 (neighbouring strings of 4x4:
+// 21.6 slots for 17.1 hops, by number 17.1).  The results then go to scattered places of the row, which
+// the FP64 products have time for (row pass 14 sites 436 -> 373 us, whole product 4x4 12.0 -> 11.0 ms,
+// windows of 256 strings between: 400 us, 11.7 ms).  The FP32 products are bound by the passes over shared
+// memory and L1, and a scattered store costs as many as the slots it would save: strings in order.
+static std::vector<int32_t> ell_columns(const HostHop &h)
+{
+    const int64_t n = (int64_t)h.str.size();
+    std::vector<int32_t> cols((size_t)((n + 31) / 32 * 32), -1);
+    for (int64_t u = 0; u < n; ++u) cols[(size_t)u] = (int32_t)u;
+    auto hops = [&](int32_t u) { return h.ptr[(size_t)u + 1] - h.ptr[(size_t)u]; };
+    std::stable_sort(cols.begin(), cols.begin() + n, [&](int32_t x, int32_t y) { return hops(x) > hops(y); });
+    return cols;
+}
+
 static std::shared_ptr<const EllOrder> ell_order(const HostHop &h)
 {
     const uint64_t key = hash_structure(h);
@@ -385,32 +441,9 @@ static std::shared_ptr<const EllOrder> ell_order(const HostHop &h)
     auto o = std::make_shared<EllOrder>();
     o->ptr = h.ptr;
     o->src = h.src;
-    const int64_t n = (int64_t)h.str.size();
-    const int64_t ns = (n + 31) / 32;
-    std::vector<int32_t> &off = o->off;
-    off.assign((size_t)ns + 1, 0);
-    for (int64_t sl = 0; sl < ns; ++sl) {
-        int32_t w = 0;
-        for (int64_t u = sl * 32; u < std::min(n, sl * 32 + 32); ++u) w = std::max(w, h.ptr[(size_t)u + 1] - h.ptr[(size_t)u]);
-        off[(size_t)sl + 1] = off[(size_t)sl] + w;
-    }
-    const int64_t slots = off[(size_t)ns];
-    o->entry.assign((size_t)std::max<int64_t>(slots * 32, 1), -1);
-    std::vector<int32_t> srcs[32], slot;
-    for (int64_t sl = 0; sl < ns; ++sl) {
-        const int w = off[(size_t)sl + 1] - off[(size_t)sl];
-        for (int l = 0; l < 32; ++l) {
-            const int64_t u = sl * 32 + l;
-            srcs[l].clear();
-            if (u < n) srcs[l].assign(h.src.begin() + h.ptr[(size_t)u], h.src.begin() + h.ptr[(size_t)u + 1]);
-        }
-        ell_color_slice(srcs, w, slot);
-        for (int k = 0; k < w; ++k)
-            for (int l = 0; l < 32; ++l) {
-                const int32_t j = slot[(size_t)(k * 32 + l)];
-                if (j >= 0) o->entry[(size_t)((off[(size_t)sl] + k) * 32 + l)] = h.ptr[(size_t)(sl * 32 + l)] + j;
-            }
-    }
+    o->plain = ell_slots_of(h, nullptr);
+    o->cols = ell_columns(h);
+    o->sorted = ell_slots_of(h, o->cols.data());
     std::lock_guard<std::mutex> lk(g_ell_mu);
     // a sweep over many different lattices must not grow the cache without bound: past
     // kEllCacheMax structures it starts over (orders in use stay alive through their owners)
@@ -427,43 +460,33 @@ static int upload_ell(const HostHop &h, HopTable &d, TablePool &pool)
 {
     const std::shared_ptr<const EllOrder> o = ell_order(h);
     const int64_t n = (int64_t)h.str.size();
-    const int64_t ns = (int64_t)o->off.size() - 1;
-    const int64_t slots = o->off[(size_t)ns];
-    const std::vector<int32_t> &off = o->off;
-    std::vector<int32_t> src((size_t)std::max<int64_t>(slots * 32, 1));
-    std::vector<double> c64((size_t)std::max<int64_t>(slots * 32, 1), 0.0);
-    for (int64_t sl = 0; sl < ns; ++sl)
-        for (int64_t k = off[(size_t)sl]; k < off[(size_t)sl + 1]; ++k)
-            for (int l = 0; l < 32; ++l) {
-                const size_t at = (size_t)(k * 32 + l);
-                const int32_t e = o->entry[at];
-                const int64_t u = sl * 32 + l;
-                if (e >= 0) {
-                    src[at] = h.src[(size_t)e];
-                    c64[at] = h.coef[(size_t)e];
-                } else {
-                    src[at] = (int32_t)(u < n ? u : n - 1);
-                    c64[at] = 0.0;
-                }
-            }
-    std::vector<float> c32(c64.begin(), c64.end());
-    std::vector<int2> pk(src.size(), make_int2(0, 0));
-    for (int64_t k = 0; k < slots; ++k) {
+    const EllSlots &p = o->plain, &q = o->sorted;
+    std::vector<int2> pk(std::max<size_t>(p.entry.size(), 1), make_int2(0, 0));
+    for (size_t k = 0; k < p.entry.size(); k += 32) {
         int32_t sk[32];
-        for (int l = 0; l < 32; ++l) sk[l] = o->entry[(size_t)(k * 32 + l)] >= 0 ? src[(size_t)(k * 32 + l)] : -1;
+        for (int l = 0; l < 32; ++l) sk[l] = p.entry[k + l] >= 0 ? h.src[(size_t)p.entry[k + l]] : -1;
         ell_fill_padding(sk, n);
         for (int l = 0; l < 32; ++l) {
+            const float c = p.entry[k + l] >= 0 ? (float)h.coef[(size_t)p.entry[k + l]] : 0.f;
             int32_t bits;
-            std::memcpy(&bits, &c32[(size_t)(k * 32 + l)], sizeof(bits));
-            pk[(size_t)(k * 32 + l)] = make_int2(sk[l], bits);
+            std::memcpy(&bits, &c, sizeof(bits));
+            pk[k + l] = make_int2(sk[l], bits);
         }
     }
-    d.nslice = ns;
-    d.ell_slots = slots;
-    pool.add(&d.ell_off, off.data(), off.size());
-    pool.add(&d.ell_src, src.data(), src.size());
-    pool.add(&d.ell_cf32, c32.data(), c32.size());
-    pool.add(&d.ell_cf64, c64.data(), c64.size());
+    std::vector<int32_t> src(std::max<size_t>(q.entry.size(), 1), 0);
+    std::vector<double> c64(src.size(), 0.0);
+    d.nslice = (int64_t)p.off.size() - 1;
+    for (int64_t sl = 0; sl < d.nslice; ++sl)
+        for (size_t at = (size_t)q.off[(size_t)sl] * 32; at < (size_t)q.off[(size_t)sl + 1] * 32; ++at) {
+            const int32_t e = q.entry[at], u = o->cols[(size_t)sl * 32 + at % 32];
+            src[at] = e >= 0 ? h.src[(size_t)e] : u >= 0 ? u : (int32_t)(n - 1);
+            if (e >= 0) c64[at] = h.coef[(size_t)e];
+        }
+    pool.add(&d.ell_off, p.off.data(), p.off.size());
+    pool.add(&d.ell64_off, q.off.data(), q.off.size());
+    pool.add(&d.ell64_col, o->cols.data(), o->cols.size());
+    pool.add(&d.ell64_src, src.data(), src.size());
+    pool.add(&d.ell64_cf, c64.data(), c64.size());
     pool.add(&d.ell_pk32, pk.data(), pk.size());
     return ED_OK;
 }
