@@ -37,14 +37,13 @@ struct BatchInst {
     const double *ucf64, *dcf64;
     const double *uediag, *dediag;
     const float *uediag32, *dediag32;
-    const double *u_site;             // device, indexed by bit
+    const double *u_site;             // device, indexed by bit (uniform U: U times a count)
     const float *u_site32;
     const int32_t *ell_off;           // sliced-ELL up-hop tables of the sector, FP32
     const int2 *ell_pk32;
     const int32_t *ell64_off, *ell64_col, *ell64_src;   // and FP64
     const double *ell64_cf;
     int nslice;
-    double u_value;
     float u_value32;
     int u_uniform;
     int64_t blk0;                     // first CTA of this instance
@@ -60,7 +59,7 @@ struct ed_batch {
     int64_t nblocks = 0;
     ed::BatchInst *dev = nullptr;      // [ninst]
     int32_t *blk_inst = nullptr;       // [nblocks] device: instance of every CTA
-    double *u_site_all = nullptr;      // [ninst][kMaxSites] device
+    double *u_site_all = nullptr;      // [ninst][kMaxSites + 1] device
     float *u_site_all32 = nullptr;     // the same in FP32
     std::vector<int64_t> offsets, dims;
     int max_nsup = 0;
@@ -88,7 +87,10 @@ __device__ __forceinline__ double sum_partials_warp(const double *__restrict__ p
 template <typename T>
 __device__ __forceinline__ T u_energy_b(const BatchInst &a, uint32_t both)
 {
-    if (a.u_uniform) return ((sizeof(T) == 4) ? (T)a.u_value32 : (T)a.u_value) * (T)__popc(both);
+    if (a.u_uniform) {
+        if constexpr (sizeof(T) == 4) return (T)a.u_value32 * (T)__popc(both);
+        return (T)__ldg(a.u_site + __popc(both));   // no FP64 operation
+    }
     const T *us = (sizeof(T) == 4) ? reinterpret_cast<const T *>(a.u_site32) : reinterpret_cast<const T *>(a.u_site);
     T e = 0;
     while (both) {
@@ -845,7 +847,7 @@ extern "C" int ed_batch_create_rows(int ninst, ed_sector *const *secs, int rows,
     ED_REQUIRE(ninst >= 1 && secs != nullptr, "need at least one instance");
     ED_REQUIRE(rows == 4 || rows == 8 || rows == 16, "rows per CTA must be 4, 8 or 16, got %d", rows);
     std::vector<BatchInst> host((size_t)ninst);
-    std::vector<double> usite((size_t)ninst * kMaxSites);
+    std::vector<double> usite((size_t)ninst * (kMaxSites + 1));
     std::vector<float> usite32((size_t)ninst * kMaxSites);
     std::vector<int32_t> binst;
     std::vector<int64_t> offsets, dims;
@@ -874,11 +876,11 @@ extern "C" int ed_batch_create_rows(int ninst, ed_sector *const *secs, int rows,
         a.ell_pk32 = s->up.ell_pk32;
         a.nslice = (int)s->up.nslice;
         for (int q = 0; q < kMaxSites; ++q) {
-            usite[(size_t)i * kMaxSites + q] = s->u_site[q];
+            usite[(size_t)i * (kMaxSites + 1) + q] = s->u_uniform ? s->u_value * q : s->u_site[q];
             usite32[(size_t)i * kMaxSites + q] = (float)s->u_site[q];
         }
+        usite[(size_t)i * (kMaxSites + 1) + kMaxSites] = s->u_uniform ? s->u_value * kMaxSites : 0.0;
         a.u_site = nullptr;   // set after the upload below
-        a.u_value = s->u_value;
         a.u_value32 = (float)s->u_value;
         a.u_uniform = s->u_uniform ? 1 : 0;
         a.blk0 = blk;
@@ -942,7 +944,7 @@ extern "C" int ed_batch_create_rows(int ninst, ed_sector *const *secs, int rows,
         return ED_ERR_CUDA;
     }
     for (int i = 0; i < ninst; ++i) {
-        host[(size_t)i].u_site = bt->u_site_all + (size_t)i * kMaxSites;
+        host[(size_t)i].u_site = bt->u_site_all + (size_t)i * (kMaxSites + 1);
         host[(size_t)i].u_site32 = bt->u_site_all32 + (size_t)i * kMaxSites;
     }
     if (cudaMemcpy(bt->dev, host.data(), sizeof(BatchInst) * ninst, cudaMemcpyHostToDevice) != cudaSuccess ||
