@@ -40,7 +40,9 @@ struct BatchInst {
     const double *u_site;             // device, indexed by bit (uniform U: U times a count)
     const float *u_site32;
     const int32_t *ell_off;           // sliced-ELL up-hop tables of the sector, FP32
-    const int2 *ell_pk32;
+    const int2 *ell_pk32;             // or ell_sg32 (hop_slot)
+    const int32_t *ell_sg32;
+    float mag32[2];
     const int32_t *ell64_off, *ell64_col, *ell64_src;   // and FP64
     const double *ell64_cf;
     int nslice;
@@ -212,7 +214,7 @@ __device__ __forceinline__ void load_column(const T *p, T (&v)[R])
 
 // G up-hop slots of one lane (table entries at `at`, `at`+32, ...): the G
 // table loads are issued before the first gather.
-template <typename T, int G, int R>
+template <typename T, int G, int R, bool TWO>
 __device__ __forceinline__ void up_group(const BatchInst &a, const T *xs, int at, T (&acc)[R])
 {
     constexpr int S = staged_stride<T, R>();
@@ -221,9 +223,9 @@ __device__ __forceinline__ void up_group(const BatchInst &a, const T *xs, int at
 #pragma unroll
     for (int j = 0; j < G; ++j) {
         if (sizeof(T) == 4) {
-            const int2 pk = __ldg(a.ell_pk32 + at + 32 * j);
-            src[j] = pk.x;
-            w[j] = (T)__int_as_float(pk.y);
+            float c;
+            hop_slot<TWO>(a.ell_pk32, a.ell_sg32, a.mag32[0], a.mag32[1], at + 32 * j, src[j], c);
+            w[j] = (T)c;
         } else {
             src[j] = __ldg(a.ell64_src + at + 32 * j);
             w[j] = (T)__ldg(a.ell64_cf + at + 32 * j);
@@ -365,13 +367,18 @@ __device__ __forceinline__ void hv_item(const BatchInst *__restrict__ inst, int6
         const int s0 = __ldg(off + sl), ns = __ldg(off + sl + 1) - s0;
         // slots in groups: all table loads of a group are in flight before
         // its first gather
-        int q = 0;
-        for (; q + 8 <= ns; q += 8) up_group<T, 8, R>(a, xs, (s0 + q) * 32 + lane, acc);
-        if (q + 4 <= ns) {
-            up_group<T, 4, R>(a, xs, (s0 + q) * 32 + lane, acc);
-            q += 4;
-        }
-        for (; q < ns; ++q) up_group<T, 1, R>(a, xs, (s0 + q) * 32 + lane, acc);
+        auto walk = [&](auto two) {
+            constexpr bool TWO = decltype(two)::value;
+            int q = 0;
+            for (; q + 8 <= ns; q += 8) up_group<T, 8, R, TWO>(a, xs, (s0 + q) * 32 + lane, acc);
+            if (q + 4 <= ns) {
+                up_group<T, 4, R, TWO>(a, xs, (s0 + q) * 32 + lane, acc);
+                q += 4;
+            }
+            for (; q < ns; ++q) up_group<T, 1, R, TWO>(a, xs, (s0 + q) * 32 + lane, acc);
+        };
+        if (sizeof(T) == 4 && a.ell_sg32) walk(std::true_type());
+        else walk(std::false_type());
         if (ok) {
 #pragma unroll
             for (int r = 0; r < R; ++r)
@@ -873,7 +880,9 @@ extern "C" int ed_batch_create_rows(int ninst, ed_sector *const *secs, int rows,
         a.ell_off = s->up.ell_off;
         a.ell64_off = s->up.ell64_off; a.ell64_col = s->up.ell64_col;
         a.ell64_src = s->up.ell64_src; a.ell64_cf = s->up.ell64_cf;
-        a.ell_pk32 = s->up.ell_pk32;
+        a.ell_pk32 = s->up.ell_pk32; a.ell_sg32 = s->up.ell_sg32;
+        a.mag32[0] = s->up.mag32[0];
+        a.mag32[1] = s->up.mag32[1];
         a.nslice = (int)s->up.nslice;
         for (int q = 0; q < kMaxSites; ++q) {
             usite[(size_t)i * (kMaxSites + 1) + q] = s->u_uniform ? s->u_value * q : s->u_site[q];

@@ -73,6 +73,9 @@ struct HopTable {
     int64_t nslice = 0;
     int32_t *ell_off = nullptr;    // [nslice+1] first slot of each slice
     int2 *ell_pk32 = nullptr;      // [slots*32] {src, FP32 coefficient bits}
+    // instead, where the coefficients have at most two magnitudes: src, mag32[1] in bit 30, minus in bit 31
+    int32_t *ell_sg32 = nullptr;   // [slots*32]
+    float mag32[2] = {0.f, 0.f};
     int32_t *ell64_off = nullptr;  // [nslice+1]
     int32_t *ell64_col = nullptr;  // [nslice*32] string of each lane, -1 past the last
     int32_t *ell64_src = nullptr;  // [slots*32]
@@ -219,6 +222,24 @@ struct ed_sector {
 namespace ed {
 
 // ------------------------------------------------------------ device helpers
+
+// Source and coefficient of an FP32 hop-table slot.  TWO: the coefficients are +-m0 and +-m1, and a slot is
+// one word: every row group reads the table again, at two passes of the L1 data pipe per slot or one
+// (beside four for 16-byte gathers: 4x4 FP32 row pass 937 -> 837 us).
+template <bool TWO>
+__device__ __forceinline__ void hop_slot(const int2 *pk, const int32_t *sg, float m0, float m1, int64_t at, int &src,
+                                         float &c)
+{
+    if (TWO) {
+        const int32_t e = __ldg(sg + at);
+        src = e & 0x3fffffff;
+        c = __int_as_float(__float_as_int((e & 0x40000000) ? m1 : m0) ^ (e & (int32_t)0x80000000));
+    } else {
+        const int2 e = __ldg(pk + at);
+        src = e.x;
+        c = __int_as_float(e.y);
+    }
+}
 
 // Asynchronous global -> shared copy of one element (cp.async, 4 or 8 bytes):
 // a thread's copies are all in flight at once; cp_async_wait_all precedes the

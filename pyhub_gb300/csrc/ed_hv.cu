@@ -30,7 +30,9 @@ struct HubArgs {
     const int32_t *ell_off;        // of the type's table
     const int32_t *ell64_col, *ell64_src;
     const double *ell64_cf;
-    const int2 *ell_pk32;
+    const int2 *ell_pk32;          // or ell_sg32 (hop_slot)
+    const int32_t *ell_sg32;
+    float mag32[2];
     const void *u_lut;        // [4][256], then U times a count; float or double like the vectors
     int nbytes;               // bytes of a string with an on-site interaction (1 when there is none: zeros)
     int u_uniform;
@@ -78,7 +80,7 @@ __device__ __forceinline__ void stage_row(T *dst, const T *__restrict__ src, int
 // G up-hop slots of one lane (table entries at, at+32, ...) applied to the R
 // staged rows; the G table loads are issued before the first gather (FP32:
 // one packed 8-byte {source, coefficient} load per slot).
-template <typename T, int R, int G>
+template <typename T, int R, int G, bool TWO>
 __device__ __forceinline__ void row_group(const HubArgs &a, int64_t at, const T *xs, int64_t sld, T (&acc)[R])
 {
     int q[G];
@@ -86,9 +88,9 @@ __device__ __forceinline__ void row_group(const HubArgs &a, int64_t at, const T 
 #pragma unroll
     for (int i = 0; i < G; ++i) {
         if (sizeof(T) == 4) {
-            const int2 pk = __ldg(a.ell_pk32 + at + i * 32);
-            q[i] = pk.x;
-            c[i] = (T)__int_as_float(pk.y);
+            float w;
+            hop_slot<TWO>(a.ell_pk32, a.ell_sg32, a.mag32[0], a.mag32[1], at + i * 32, q[i], w);
+            c[i] = (T)w;
         } else {
             q[i] = __ldg(a.ell64_src + at + i * 32);
             c[i] = (T)__ldg(a.ell64_cf + at + i * 32);
@@ -103,7 +105,7 @@ __device__ __forceinline__ void row_group(const HubArgs &a, int64_t at, const T 
 // Pass 1: diagonal + up hops, R rows per CTA iteration.  Each warp owns one
 // 32-string slice at a time and walks its sliced-ELL slots (coalesced,
 // four slots in flight), gathering the sources from the staged rows.
-template <typename T, int R>
+template <typename T, int R, bool TWO>
 __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T *__restrict__ y,
                                                       const HubArgs a, int64_t sld, int vec_ok)
 {
@@ -143,12 +145,12 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
             const int64_t at0 = (int64_t)s0 * 32 + lane;
             // slots in groups: all table loads of a group are in flight before its first gather
             int k = 0;
-            for (; k + 8 <= ns; k += 8) row_group<T, R, 8>(a, at0 + k * 32, xs, sld, acc);
+            for (; k + 8 <= ns; k += 8) row_group<T, R, 8, TWO>(a, at0 + k * 32, xs, sld, acc);
             if (k + 4 <= ns) {
-                row_group<T, R, 4>(a, at0 + k * 32, xs, sld, acc);
+                row_group<T, R, 4, TWO>(a, at0 + k * 32, xs, sld, acc);
                 k += 4;
             }
-            for (; k < ns; ++k) row_group<T, R, 1>(a, at0 + k * 32, xs, sld, acc);
+            for (; k < ns; ++k) row_group<T, R, 1, TWO>(a, at0 + k * 32, xs, sld, acc);
             if (ok) {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
@@ -164,16 +166,14 @@ __global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T
 // rows with one 128-bit shared load.  A quarter warp's 8 lanes hit 8 bank
 // groups when their sources differ mod 8, which the sliced-ELL slot order
 // arranges (ed_sector.cu, ell_order).
-template <int G>
+template <int G, bool TWO>
 __device__ __forceinline__ void col_group(const HubArgs &a, int64_t at, const float4 *xs4, float (&acc)[4])
 {
     int q[G];
     float c[G];
 #pragma unroll
     for (int i = 0; i < G; ++i) {
-        const int2 pk = __ldg(a.ell_pk32 + at + i * 32);
-        q[i] = pk.x;
-        c[i] = __int_as_float(pk.y);
+        hop_slot<TWO>(a.ell_pk32, a.ell_sg32, a.mag32[0], a.mag32[1], at + i * 32, q[i], c[i]);
     }
 #pragma unroll
     for (int i = 0; i < G; ++i) {
@@ -185,6 +185,7 @@ __device__ __forceinline__ void col_group(const HubArgs &a, int64_t at, const fl
     }
 }
 
+template <bool TWO>
 __global__ void __launch_bounds__(1024) hub_row_col4_kernel(const float *__restrict__ x, float *__restrict__ y,
                                                             const HubArgs a)
 {
@@ -233,12 +234,12 @@ __global__ void __launch_bounds__(1024) hub_row_col4_kernel(const float *__restr
             const int s0 = __ldg(a.ell_off + sl), ns = __ldg(a.ell_off + sl + 1) - s0;
             const int64_t at0 = (int64_t)s0 * 32 + lane;
             int k = 0;
-            for (; k + 8 <= ns; k += 8) col_group<8>(a, at0 + k * 32, xs4, acc);
+            for (; k + 8 <= ns; k += 8) col_group<8, TWO>(a, at0 + k * 32, xs4, acc);
             if (k + 4 <= ns) {
-                col_group<4>(a, at0 + k * 32, xs4, acc);
+                col_group<4, TWO>(a, at0 + k * 32, xs4, acc);
                 k += 4;
             }
-            for (; k < ns; ++k) col_group<1>(a, at0 + k * 32, xs4, acc);
+            for (; k < ns; ++k) col_group<1, TWO>(a, at0 + k * 32, xs4, acc);
             if (ok) {
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
@@ -589,6 +590,9 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     a.ell64_src = s->up.ell64_src;
     a.ell64_cf = s->up.ell64_cf;
     a.ell_pk32 = s->up.ell_pk32;
+    a.ell_sg32 = s->up.ell_sg32;
+    a.mag32[0] = s->up.mag32[0];
+    a.mag32[1] = s->up.mag32[1];
     a.u_lut = (sizeof(T) == 4) ? (const void *)s->u_lut32 : (const void *)s->u_lut;
     a.nbytes = (s->u_uniform && s->u_value == 0.0) ? 1 : (s->norb + 7) / 8;
     a.u_uniform = s->u_uniform ? 1 : 0;
@@ -626,8 +630,7 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     // FP32: four rows per 1024-thread CTA (one CTA per SM) when they fit, so every
     // hop-table slot serves four rows and one 128-bit gather reads all four;
     // else two rows per CTA with two CTAs per SM; else one.
-    constexpr int R2 = 2;
-    const bool two = (size_t)R2 * row_bytes * 2 <= (size_t)maxsm;
+    const bool two = 4 * row_bytes <= (size_t)maxsm;
     const int threads = 512;
     const size_t smem4 = (size_t)(zero_col(s->nsup) + kZeroCols) * 16;
     if (sizeof(T) == 4 && smem4 <= (size_t)maxsm) {
@@ -635,24 +638,17 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
         const size_t smem = smem4;
         int64_t blocks = (s->nsdn + 3) / 4;
         if (blocks > nsm) blocks = nsm;
-        ED_CHECK_CUDA(cudaFuncSetAttribute(hub_row_col4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
-        hub_row_col4_kernel<<<(unsigned)blocks, 1024, smem, st>>>(reinterpret_cast<const float *>(x),
-                                                                  reinterpret_cast<float *>(y), a);
-    } else if (two) {
-        size_t smem = (size_t)R2 * row_bytes;
-        ED_CHECK_CUDA(cudaFuncSetAttribute(hub_row_kernel<T, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int64_t blocks = (s->nsdn + R2 - 1) / R2;
-        int64_t cap = (int64_t)nsm * 2;
-        if (blocks > cap) blocks = cap;
-        hub_row_kernel<T, R2><<<(unsigned)blocks, threads, smem, st>>>(x, y, a, sld, vec_ok ? 1 : 0);
+        auto *kfn = a.ell_sg32 ? hub_row_col4_kernel<true> : hub_row_col4_kernel<false>;
+        ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kfn<<<(unsigned)blocks, 1024, smem, st>>>(reinterpret_cast<const float *>(x), reinterpret_cast<float *>(y), a);
     } else {
-        size_t smem = row_bytes;
-        ED_CHECK_CUDA(cudaFuncSetAttribute(hub_row_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int64_t blocks = s->nsdn;
-        int64_t cap = (int64_t)nsm * 2;
-        if (blocks > cap) blocks = cap;
-        hub_row_kernel<T, 1><<<(unsigned)blocks, threads, smem, st>>>(x, y, a, sld, vec_ok ? 1 : 0);
+        const int R = two ? 2 : 1;
+        const size_t smem = (size_t)R * row_bytes;
+        auto *kfn = two ? hub_row_kernel<T, 2, false> : hub_row_kernel<T, 1, false>;
+        if (sizeof(T) == 4 && a.ell_sg32) kfn = two ? hub_row_kernel<T, 2, sizeof(T) == 4> : hub_row_kernel<T, 1, sizeof(T) == 4>;
+        ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const int64_t blocks = std::min<int64_t>((s->nsdn + R - 1) / R, (int64_t)nsm * 2);
+        kfn<<<(unsigned)blocks, threads, smem, st>>>(x, y, a, sld, vec_ok ? 1 : 0);
     }
     ED_CHECK_LAUNCH();
     // ---- the U_ijkl terms, if any (before pass 2, whose fused dots need the whole product)

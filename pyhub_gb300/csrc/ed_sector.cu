@@ -487,7 +487,26 @@ static int upload_ell(const HostHop &h, HopTable &d, TablePool &pool)
     pool.add(&d.ell64_col, o->cols.data(), o->cols.size());
     pool.add(&d.ell64_src, src.data(), src.size());
     pool.add(&d.ell64_cf, c64.data(), c64.size());
-    pool.add(&d.ell_pk32, pk.data(), pk.size());
+    // at most two magnitudes (a lattice with t, or t and t'): one word per slot
+    int nmag = 0;
+    for (double c : h.coef) {
+        const float m = std::fabs((float)c);
+        int k = 0;
+        while (k < nmag && d.mag32[k] != m) ++k;
+        if (k == 2) { nmag = 3; break; }
+        if (k == nmag) d.mag32[nmag++] = m;
+    }
+    if (nmag <= 2 && zero_col(n) + kZeroCols < (1 << 30)) {
+        std::vector<int32_t> sg(pk.size());
+        for (size_t k = 0; k < pk.size(); ++k) {
+            float c;
+            std::memcpy(&c, &pk[k].y, sizeof(c));
+            sg[k] = pk[k].x | (nmag == 2 && std::fabs(c) == d.mag32[1] ? 0x40000000 : 0) | (pk[k].y & (int32_t)0x80000000);
+        }
+        pool.add(&d.ell_sg32, sg.data(), sg.size());
+    } else {
+        pool.add(&d.ell_pk32, pk.data(), pk.size());
+    }
     return ED_OK;
 }
 

@@ -1,5 +1,5 @@
-"""FP32 products through the packed hop table, whose slots without a hop read zero columns behind the
-staged ones: rows of every residue mod 8 and of whole slices, strings without a hop, few and many bonds,
+"""FP32 products through the packed hop table (one word a slot where the hoppings have one or two magnitudes,
+else two), whose slots without a hop read zero columns behind the staged ones: rows of every residue mod 8 and of whole slices, strings without a hop, few and many bonds,
 each kernel that stages rows (one and four rows per CTA, batched 4, 8 and 16).
 
 Integer t, U and x keep every sum below 2^24, so the FP32 products equal the FP64 ones; a NaN of x
@@ -13,19 +13,20 @@ pytestmark = pytest.mark.gpu
 ROWS = [(12, 5, 6, 12), (12, 6, 5, 60), (13, 4, 5, 20), (13, 5, 4, 3), (17, 8, 2, 17), (17, 7, 2, 30), (17, 9, 3, 20)]
 
 
-def _t(n, bonds, rng):
+def _t(n, bonds, rng, mags):
     t = np.zeros((n, n))
     for _ in range(bonds):
         a, b = rng.choice(n, 2, replace=False)
-        t[a, b] = t[b, a] = rng.integers(1, 4)
+        t[a, b] = t[b, a] = rng.choice([-1, 1]) * rng.integers(1, mags + 1)
     return t
 
 
+@pytest.mark.parametrize("mags", [1, 2, 3])
 @pytest.mark.parametrize("n,nu,nd,bonds", ROWS)
-def test_row_products_equal_fp64(edlib, n, nu, nd, bonds):
+def test_row_products_equal_fp64(edlib, n, nu, nd, bonds, mags):
     import torch
     rng = np.random.default_rng(n + nu)
-    sec = edlib.Sector(n, nu, nd, edlib.ED_HUBBARD, t=_t(n, bonds, rng), U=rng.integers(0, 5, n).astype(float))
+    sec = edlib.Sector(n, nu, nd, edlib.ED_HUBBARD, t=_t(n, bonds, rng, mags), U=rng.integers(0, 5, n).astype(float))
     x = torch.randint(-4, 5, (sec.nsdn * sec.nsup,), device="cuda").double()
     for nan in (False, True):
         if nan:
@@ -45,8 +46,8 @@ def test_batched_products_equal_fp64(edlib, rows):
     from pyhub_gb300 import _capi
     rng = np.random.default_rng(rows)
     shapes = [(4, 0, 2), (5, 1, 2), (8, 1, 3), (6, 3, 2), (6, 2, 3), (7, 3, 3), (8, 4, 1), (8, 3, 4), (12, 5, 2), (9, 3, 3)]
-    secs = [edlib.Sector(n, nu, nd, edlib.ED_HUBBARD, t=_t(n, n, rng), U=rng.integers(0, 5, n).astype(float))
-            for n, nu, nd in shapes]
+    secs = [edlib.Sector(n, nu, nd, edlib.ED_HUBBARD, t=_t(n, n, rng, 1 + i % 3), U=rng.integers(0, 5, n).astype(float))
+            for i, (n, nu, nd) in enumerate(shapes)]
     b = _capi.Batch(secs, rows=rows)
     scratch = torch.empty(b.scratch_bytes() // 8 + 1, dtype=torch.float64, device="cuda")
     xs = [torch.randint(-4, 5, (s.nsdn * s.nsup,), device="cuda").double() for s in secs]
