@@ -106,7 +106,7 @@ __device__ __forceinline__ void row_group(const HubArgs &a, int64_t at, const T 
 // 32-string slice at a time and walks its sliced-ELL slots (coalesced,
 // four slots in flight), gathering the sources from the staged rows.
 template <typename T, int R, bool TWO>
-__global__ void __launch_bounds__(512) hub_row_kernel(const T *__restrict__ x, T *__restrict__ y,
+__global__ void __launch_bounds__(512, 2) hub_row_kernel(const T *__restrict__ x, T *__restrict__ y,
                                                       const HubArgs a, int64_t sld, int vec_ok)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
