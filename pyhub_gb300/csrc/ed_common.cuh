@@ -113,9 +113,10 @@ struct HeisStruct {
     uint32_t *col_pat = nullptr;     // A patterns, concatenated over m
     int32_t *rankA = nullptr;        // [2^nA] colex rank among the patterns of equal popcount
     double *diagA = nullptr;         // A-A zz energy per column
-    int32_t *aa_off = nullptr, *aa_src = nullptr;   // sliced ELL of the A-A flips per m
-    float *aa_cf32 = nullptr;
-    double *aa_cf64 = nullptr;
+    // sliced ELL of the A-A flips per m: FP32 (aa_pk32) with the columns in order, FP64 by number of flips
+    int32_t *aa_off = nullptr;
+    int32_t *aa64_off = nullptr, *aa64_src = nullptr, *aa64_col = nullptr;   // col: [slices*32], -1 past the last
+    double *aa64_cf = nullptr;
     uint32_t *row_pat = nullptr;     // B pattern per row (rows in offset order)
     int32_t *row_m = nullptr, *rowidx = nullptr;    // holes in A per row; [2^nB] row of a pattern or -1
     int64_t *row_off = nullptr;

@@ -71,6 +71,9 @@ int up(T **dst, const std::vector<T> &v)
 
 }  // namespace
 
+// Vectors up to this many bytes mostly meet L2 again where neighbouring rows are read out of order.
+constexpr double kL2Bytes = 1.0e9;
+
 int heis_struct_build(ed_sector *s)
 {
     const HeisTables &ht = s->heis;
@@ -115,8 +118,9 @@ int heis_struct_build(ed_sector *s)
     }
     // A-A zz energy and hop lists per column, sliced ELL per m (32 columns per slice)
     diagA.resize(col_pat.size());
-    std::vector<int32_t> aa_off(1, 0), aa_src;
-    std::vector<double> aa_cf;
+    std::vector<int32_t> aa_off(1, 0), aa64_off(1, 0), aa64_src, aa64_col;
+    std::vector<int2> aa_pk32;
+    std::vector<double> aa64_cf;
     int64_t nslices = 0;
     for (int m = 0; m <= nA; ++m) {
         hs->slice_base[m] = nslices;
@@ -137,22 +141,44 @@ int heis_struct_build(ed_sector *s)
             diagA[(size_t)(base + r)] = d;
         }
         const int64_t ns = (n + 31) / 32;
-        for (int64_t sl = 0; sl < ns; ++sl) {
-            size_t w = 0;
-            for (int64_t r = sl * 32; r < std::min(n, sl * 32 + 32); ++r) w = std::max(w, lists[(size_t)r].size());
-            for (size_t k = 0; k < w; ++k)
-                for (int l = 0; l < 32; ++l) {
-                    const int64_t r = sl * 32 + l;
-                    if (r < n && k < lists[(size_t)r].size()) {
-                        aa_src.push_back(lists[(size_t)r][k].first);
-                        aa_cf.push_back(lists[(size_t)r][k].second);
-                    } else {
-                        aa_src.push_back((int32_t)std::min(r, n - 1));   // own column, weight 0
-                        aa_cf.push_back(0.0);
+        std::vector<int32_t> order((size_t)n);
+        for (int64_t r = 0; r < n; ++r) order[(size_t)r] = (int32_t)r;
+        // slots of the class, lane l of slice s with column order[s * 32 + l]; put(column, flip or NULL)
+        auto slots = [&](std::vector<int32_t> &off, auto put) {
+            for (int64_t sl = 0; sl < ns; ++sl) {
+                size_t w = 0;
+                for (int64_t r = sl * 32; r < std::min(n, sl * 32 + 32); ++r)
+                    w = std::max(w, lists[(size_t)order[(size_t)r]].size());
+                for (size_t k = 0; k < w; ++k)
+                    for (int l = 0; l < 32; ++l) {
+                        const int32_t c = order[(size_t)std::min(n - 1, sl * 32 + l)];
+                        const auto &L = lists[(size_t)c];
+                        put(c, sl * 32 + l < n && k < L.size() ? &L[k] : nullptr);   // none: own column, weight 0
                     }
-                }
-            aa_off.push_back(aa_off.back() + (int32_t)w);
-        }
+                off.push_back(off.back() + (int32_t)w);
+            }
+        };
+        slots(aa_off, [&](int32_t c, const std::pair<int32_t, double> *flip) {
+            const float f = flip ? (float)flip->second : 0.f;
+            int32_t bits;
+            std::memcpy(&bits, &f, sizeof(bits));
+            aa_pk32.push_back(make_int2(flip ? flip->first : c, bits));
+        });
+        // FP64: columns by number of flips.  A slice has as many slots as its longest list and each costs the
+        // FP64 pipe a warp's operation (4x6: 12.9 slots for 9.4 flips in order, 9.7 by number), which
+        // outweighs the scattered sources and results (row pass 140 -> 128 us, in windows of 128 132 us;
+        // 4x7 3.41 -> 3.19 ms the whole product).  Vectors far above L2 pay for the scattering in DRAM
+        // sectors (5x6, 1.2 GB: 14.9 -> 22.9 ms; 4x8 56 -> 78): windows of 64 there (14.9, 55.7 ms)
+        const int64_t window = (double)s->dim * sizeof(double) <= kL2Bytes ? n : 64;
+        for (int64_t r = 0; r < n; r += window)
+            std::stable_sort(order.begin() + r, order.begin() + std::min(n, r + window), [&](int32_t x, int32_t y) {
+                return lists[(size_t)x].size() > lists[(size_t)y].size();
+            });
+        slots(aa64_off, [&](int32_t c, const std::pair<int32_t, double> *flip) {
+            aa64_src.push_back(flip ? flip->first : c);
+            aa64_cf.push_back(flip ? flip->second : 0.0);
+        });
+        for (int64_t q = 0; q < ns * 32; ++q) aa64_col.push_back(q < n ? order[(size_t)q] : -1);
         nslices += ns;
     }
     hs->slice_base[nA + 1] = nslices;
@@ -267,18 +293,13 @@ int heis_struct_build(ed_sector *s)
         hs->ab_zz[q] = 0.25 * ht.zz[b];
     }
     std::vector<float> ab_lut32(ab_lut.begin(), ab_lut.end());
-    std::vector<float> aa_cf32(aa_cf.begin(), aa_cf.end()), bb_cf32(bb_cf.begin(), bb_cf.end());
+    std::vector<float> bb_cf32(bb_cf.begin(), bb_cf.end());
     std::vector<float> diagA32(diagA.begin(), diagA.end()), diagB32(diagB.begin(), diagB.end());
-    std::vector<int2> aa_pk32(aa_src.size());
-    for (size_t q = 0; q < aa_src.size(); ++q) {
-        int32_t bits;
-        std::memcpy(&bits, &aa_cf32[q], sizeof(bits));
-        aa_pk32[q] = make_int2(aa_src[q], bits);
-    }
     int rc;
     if ((rc = up(&hs->col_pat, col_pat)) || (rc = up(&hs->rankA, rankA)) || (rc = up(&hs->diagA, diagA)) ||
-        (rc = up(&hs->aa_off, aa_off)) || (rc = up(&hs->aa_src, aa_src)) || (rc = up(&hs->aa_cf32, aa_cf32)) ||
-        (rc = up(&hs->aa_cf64, aa_cf)) || (rc = up(&hs->row_pat, row_pat)) || (rc = up(&hs->row_m, row_m)) ||
+        (rc = up(&hs->aa_off, aa_off)) || (rc = up(&hs->aa64_off, aa64_off)) ||
+        (rc = up(&hs->aa64_src, aa64_src)) || (rc = up(&hs->aa64_col, aa64_col)) || (rc = up(&hs->aa64_cf, aa64_cf)) ||
+        (rc = up(&hs->row_pat, row_pat)) || (rc = up(&hs->row_m, row_m)) ||
         (rc = up(&hs->row_off, row_off)) || (rc = up(&hs->rowidx, rowidx)) || (rc = up(&hs->diagB, diagB)) ||
         (rc = up(&hs->bb_ptr, bb_ptr)) || (rc = up(&hs->bb_src, bb_src)) || (rc = up(&hs->bb_cf32, bb_cf32)) ||
         (rc = up(&hs->bb_cf64, bb_cf)) || (rc = up(&hs->rows_of_m, rows_of_m)) ||
@@ -292,8 +313,8 @@ int heis_struct_build(ed_sector *s)
 void heis_struct_free(HeisStruct *hs)
 {
     if (!hs) return;
-    void *ptrs[] = {hs->col_pat, hs->rankA, hs->diagA, hs->aa_off, hs->aa_src, hs->aa_cf32,
-                    hs->aa_cf64, hs->row_pat, hs->row_m, hs->row_off, hs->rowidx, hs->diagB,
+    void *ptrs[] = {hs->col_pat, hs->rankA, hs->diagA, hs->aa_off, hs->aa64_off, hs->aa64_src,
+                    hs->aa64_col, hs->aa64_cf, hs->row_pat, hs->row_m, hs->row_off, hs->rowidx, hs->diagB,
                     hs->bb_ptr, hs->bb_src, hs->bb_cf32, hs->bb_cf64, hs->rows_of_m,
                     hs->aa_pk32, hs->col_abbits, hs->row_bbits, hs->diagA32, hs->diagB32, hs->ab_rank,
                     hs->ab_lut, hs->ab_lut32};
@@ -309,11 +330,12 @@ struct HsArgs {
     int64_t nrows;
     int64_t col_base[kMaxHalf + 2], ncol[kMaxHalf + 1], slice_base[kMaxHalf + 2], row_base[kMaxHalf + 2];
     const uint32_t *col_pat, *row_pat;
-    const int32_t *rankA, *aa_off, *aa_src, *row_m, *rowidx, *bb_ptr, *bb_src, *rows_of_m;
+    const int32_t *rankA, *aa_off, *aa64_src, *aa64_col, *row_m, *rowidx, *bb_ptr, *bb_src, *rows_of_m;
     const int64_t *row_off;
     const void *diagA, *diagB;     // float or double, like the vectors
-    const void *aa_cf, *bb_cf;     // float or double
+    const void *bb_cf;             // float or double
     const int2 *aa_pk32;           // {column, FP32 coefficient bits} of the A-A flips
+    const double *aa64_cf;
     const uint32_t *col_abbits, *row_bbits;
     const int32_t *ab_rank;        // [q][column] rank after flipping bond q's A bit (packed path)
     const void *ab_lut;            // [4][256] zz drops of eight bonds, float or double
@@ -355,7 +377,6 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
     T *ab_dsame = ab_c + a.nab;                                    // zz/4 (generic path)
     uint32_t *ab_need = reinterpret_cast<uint32_t *>(ab_dsame + a.nab);  // required A bit (1: A site down)
     T *xs = reinterpret_cast<T *>(smem_raw + heis_row_head_bytes(a.nab, sizeof(T)));
-    const T *acf = reinterpret_cast<const T *>(a.aa_cf);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = kHeisRowThreads / 32;
     const T sc = (T)a.scale;
     for (int64_t k = 0; k * gridDim.x < a.nrows; ++k) {
@@ -401,8 +422,8 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
         __syncthreads();
         const int nsl = (len + 31) / 32;
         for (int sl = warp; sl < nsl; sl += nwarps) {
-            const int c = sl * 32 + lane;
-            const bool ok = c < len;
+            const int c = sizeof(T) == 4 ? sl * 32 + lane : __ldg(a.aa64_col + (sbase + sl) * 32 + lane);
+            const bool ok = sizeof(T) == 4 ? c < len : c >= 0;
             const int cc = ok ? c : len - 1;
             const uint32_t ha = __ldg(a.col_pat + cbase + cc);
             T d = __ldg(static_cast<const T *>(a.diagA) + cbase + cc) + db;
@@ -428,7 +449,7 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
 #pragma unroll 4
                 for (int q = 0; q < ns; ++q) {
                     const int at = (s0 + q) * 32 + lane;
-                    acc += __ldg(acf + at) * xs[__ldg(a.aa_src + at)];
+                    acc += (T)__ldg(a.aa64_cf + at) * xs[__ldg(a.aa64_src + at)];
                 }
             }
             if (a.ab_fast) {
@@ -1247,12 +1268,12 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
         if (m <= kMaxHalf) a.ncol[m] = h.ncol[m];
     }
     a.col_pat = h.col_pat; a.row_pat = h.row_pat;
-    a.rankA = h.rankA; a.aa_off = h.aa_off; a.aa_src = h.aa_src; a.row_m = h.row_m;
+    a.rankA = h.rankA; a.aa_off = (sizeof(T) == 4) ? h.aa_off : h.aa64_off; a.aa64_src = h.aa64_src; a.aa64_col = h.aa64_col; a.row_m = h.row_m;
     a.rowidx = h.rowidx; a.bb_ptr = h.bb_ptr; a.bb_src = h.bb_src; a.rows_of_m = h.rows_of_m;
     a.row_off = h.row_off;
     a.diagA = (sizeof(T) == 4) ? (const void *)h.diagA32 : (const void *)h.diagA;
     a.diagB = (sizeof(T) == 4) ? (const void *)h.diagB32 : (const void *)h.diagB;
-    a.aa_cf = (sizeof(T) == 4) ? (const void *)h.aa_cf32 : (const void *)h.aa_cf64;
+    a.aa64_cf = h.aa64_cf;
     a.aa_pk32 = h.aa_pk32;
     a.col_abbits = h.col_abbits;
     a.row_bbits = h.row_bbits;
@@ -1273,7 +1294,7 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     // above L2 keep memory order, where the A-B bonds' source rows are near (4x8: 60 ms, by length 67), and
     // so do rows that have a CTA each (4x4: the row pass 5.5 us, by length 6.6: the look-up leads the chain
     // of loads)
-    a.by_length = (double)s->dim * sizeof(T) <= 1.0e9 && h.nrows > (int64_t)nsm * 4 ? 1 : 0;
+    a.by_length = (double)s->dim * sizeof(T) <= kL2Bytes && h.nrows > (int64_t)nsm * 4 ? 1 : 0;
     // ---- pass R
     const int maxsm = max_smem();
     const size_t smem4 = heis_col4_head_bytes(h.nab) + (size_t)std::max<int64_t>(h.max_len, 1) * 16;

@@ -77,3 +77,27 @@ def test_heisenberg_product(edlib, n, kind, dt):
             tol = (1e-12 if dt == "f64" else 2e-5)
             assert abs(float(dots[0]) - yx) <= tol * float((x * got).abs().sum())
             assert abs(float(dots[1]) - yy) <= tol * yy
+
+
+@pytest.mark.parametrize("norb", [8, 14, 20, 24, 30])
+def test_fp64_equals_fp32_on_integers(edlib, norb):
+    """The FP64 pass takes the columns by number of flips (in windows of 64 above 1e9 bytes: 30 sites), the
+    FP32 pass in order: with couplings that are multiples of 4 and integer x every sum is an integer below
+    2^24 and the products are equal."""
+    import torch
+    rng = np.random.default_rng(norb)
+    J = np.zeros((norb, norb))
+    for i in range(norb):
+        for j in ((i + 1) % norb, (i + norb // 4) % norb):
+            if i != j:
+                J[i, j] = J[j, i] = 4.0 * rng.integers(1, 3)
+    sec = edlib.Sector(norb, norb // 2, 0, edlib.ED_HEISENBERG, J=J)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(norb)
+    x = torch.randint(-2, 3, (sec.dim,), generator=g, device="cuda", dtype=torch.int8)
+    ys = []
+    for td in (torch.float32, torch.float64):
+        y = sec.zeros(td)
+        sec.hv(sec.from_ref(x.to(td)), y)
+        ys.append(sec.to_ref(y).to(torch.float32))
+    assert torch.equal(ys[0], ys[1])
