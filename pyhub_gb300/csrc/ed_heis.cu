@@ -812,8 +812,9 @@ __global__ void __launch_bounds__(256, kHeisSlabCtas) heis_slab_kernel(const T *
 //   * rdm_diag_tile: the Sz Sz sums with an A site, factorised through column sums.
 //   * rdm_rows: those of two B sites, from row sums.
 // The three run as one launch.  All pairs of 24 sites, FP64, whole call: 6.38 ms with every ordered
-// pair tested state by state and 31 FP64 operations per element of the diagonal sums, 0.78 ms in
-// this form; 8 sites 69 -> 68 us, 16 sites 371 -> 128 us.
+// pair tested state by state and 31 FP64 operations per element of the diagonal sums, 0.69 ms in
+// this form; 8 sites 69 -> 68 us, 16 sites 371 -> 125 us.  NB bounds the sites of the B half (the sums a
+// lane keeps), CTAS the CTAs of an SM.
 
 constexpr int kRdmTasks = kMaxSites * kMaxSites;
 constexpr int kRdmChunks = 512;
@@ -838,6 +839,10 @@ struct HsRdmArgs {
 };
 
 constexpr int kRdmThreads = 256;
+// Sectors of this many states take five CTAs per SM instead of three: the flips wait for loads most of the
+// time and more warps cover them, at the price of spilled registers, most of them in the diagonal tiles
+// (22 sites, 705,432 states: 331 -> 297 us, 24: 775 -> 690, 28: 11.6 -> 10.0 ms; 20 sites, 184,756: 205 -> 217).
+constexpr int64_t kRdmLarge = 1 << 19;
 
 __device__ __forceinline__ uint32_t insert_bit(uint32_t h, int pos, uint32_t bit)
 {
@@ -852,7 +857,7 @@ template <typename T> __device__ __forceinline__ void mul_add(double &acc, T b, 
     else acc += (double)(b * k);
 }
 
-template <typename T>
+template <typename T, int NB>
 __device__ __forceinline__ void rdm_flips(const T *__restrict__ bra, const T *__restrict__ ket, const HsRdmArgs &a,
                                           int mlo, int mhi, int task, int chunk, double *__restrict__ partials)
 {
@@ -863,9 +868,9 @@ __device__ __forceinline__ void rdm_flips(const T *__restrict__ bra, const T *__
     if (task < a.nab) {
         const int J = a.ab_site[task];
         const uint32_t bit = (uint32_t)a.ab_bit[task], mask = a.ab_mask[task];
-        double acc[kMaxHalf];
+        double acc[NB];
 #pragma unroll
-        for (int k = 0; k < kMaxHalf; ++k) acc[k] = 0.0;
+        for (int k = 0; k < NB; ++k) acc[k] = 0.0;
         for (int m = mlo; m <= mhi; ++m) {
             const int64_t ra = max(p0, a.row_base[m]), rb = min(p1, a.row_base[m + 1]);
             if (ra >= rb || m < (int)bit) continue;
@@ -880,8 +885,8 @@ __device__ __forceinline__ void rdm_flips(const T *__restrict__ bra, const T *__
                 const uint32_t need = mask & (bit ? ~hb : hb);
                 if (!need) continue;
                 const T *kr = ket + __ldg(a.row_off + row);
-                int64_t my_off = 0;
-                if ((need >> lane) & 1u) my_off = __ldg(a.row_off + __ldg(a.rowidx + (hb ^ (1u << lane))));
+                int my_off = 0;      // a sector has fewer than 2^31 states
+                if ((need >> lane) & 1u) my_off = (int)__ldg(a.row_off + __ldg(a.rowidx + (hb ^ (1u << lane))));
                 for (int64_t e0 = 0; e0 < ne; e0 += 32) {
                     const int64_t e = e0 + lane;
                     const bool ok = e < ne;
@@ -890,9 +895,9 @@ __device__ __forceinline__ void rdm_flips(const T *__restrict__ bra, const T *__
                     const int c = __ldg(a.rankA + h), c2 = __ldg(a.rankA + (h ^ (1u << J)));
                     const T kv = ok ? __ldg(kr + c) : (T)0;
 #pragma unroll
-                    for (int k = 0; k < kMaxHalf; ++k) {
+                    for (int k = 0; k < NB; ++k) {
                         if ((need >> k) & 1u) {
-                            const int64_t o2 = __shfl_sync(0xffffffffu, my_off, k);
+                            const int o2 = __shfl_sync(0xffffffffu, my_off, k);
                             mul_add<T>(acc[k], __ldg(bra + o2 + c2), kv);
                         }
                     }
@@ -900,7 +905,7 @@ __device__ __forceinline__ void rdm_flips(const T *__restrict__ bra, const T *__
             }
         }
 #pragma unroll
-        for (int k = 0; k < kMaxHalf; ++k) {
+        for (int k = 0; k < NB; ++k) {
             if (!((mask >> k) & 1u)) continue;
             const double s = warp_sum(acc[k]);
             if (lane == 0) out[2 * a.ab_pair[task][k]] = ((J + k + a.nA) & 1) ? -s : s;
@@ -1085,10 +1090,12 @@ __device__ __forceinline__ void rdm_diag_tile(const T *__restrict__ bra, const T
 }
 
 // One launch: the diagonal tiles, then the row chunks, then the flips (tasks of one chunk side by side).
-template <typename T>
-__global__ void __launch_bounds__(kRdmThreads) heis_rdm_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
-                                                               const __grid_constant__ HsRdmArgs a, int mlo, int mhi,
-                                                               int ntiles, int nch, double *__restrict__ partials)
+template <typename T, int NB, int CTAS>
+__global__ void __launch_bounds__(kRdmThreads, CTAS) heis_rdm_kernel(const T *__restrict__ bra,
+                                                                     const T *__restrict__ ket,
+                                                                     const __grid_constant__ HsRdmArgs a, int mlo,
+                                                                     int mhi, int ntiles, int nch,
+                                                                     double *__restrict__ partials)
 {
     extern __shared__ __align__(16) double smem_d[];
     int b = blockIdx.x;
@@ -1106,7 +1113,7 @@ __global__ void __launch_bounds__(kRdmThreads) heis_rdm_kernel(const T *__restri
     }
     constexpr int W = kRdmThreads / 32;
     const int ng = (a.ntask + W - 1) / W;
-    rdm_flips<T>(bra, ket, a, mlo, mhi, (b % ng) * W + (threadIdx.x >> 5), b / ng, partials);
+    rdm_flips<T, NB>(bra, ket, a, mlo, mhi, (b % ng) * W + (threadIdx.x >> 5), b / ng, partials);
 }
 
 // out[p][k] = sum over the partial rows of the distinct pair of p
@@ -1204,6 +1211,7 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
     }
     a.tile_base[h.mhi + 1] = ntiles;
     // row chunks: rows [0, nrows) of rows_of_m, cut where the states before them pass i/nch of all
+    const bool large = dim >= kRdmLarge;
     const int nch = (int)std::max<int64_t>(1, std::min<int64_t>({h.nrows, kRdmChunks, 3 * max_blocks - ntiles}));
     if (nch + ntiles > 3 * max_blocks) {
         set_error("spin-correlation pass needs %d partial rows (scratch holds %d)", nch + ntiles, 3 * max_blocks);
@@ -1227,10 +1235,13 @@ static int heis_struct_rdm_run(ed_sector *s, cudaStream_t st, const T *bra, cons
     ED_CHECK_CUDA(cudaMemsetAsync(scratch, 0, sizeof(double) * 2 * (size_t)a.npairs * (nch + ntiles), st));
     constexpr int W = kRdmThreads / 32;
     const size_t smem = sizeof(double) * std::max((size_t)(h.nB + 1) * kHdThreads, (size_t)W * a.nbb);
+    auto *kfn = h.nB > 12 ? heis_rdm_kernel<T, kMaxHalf, 5>
+                : large   ? heis_rdm_kernel<T, 12, 5>
+                : h.nB > 8 ? heis_rdm_kernel<T, 12, 3> : heis_rdm_kernel<T, 8, 3>;
     if (smem > 48 * 1024)
-        ED_CHECK_CUDA(cudaFuncSetAttribute(heis_rdm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int nblk = ntiles + (a.nbb > 0 ? nch : 0) + (a.ntask + W - 1) / W * nch;
-    heis_rdm_kernel<T><<<nblk, kRdmThreads, smem, st>>>(bra, ket, a, h.mlo, h.mhi, ntiles, nch, scratch);
+    kfn<<<nblk, kRdmThreads, smem, st>>>(bra, ket, a, h.mlo, h.mhi, ntiles, nch, scratch);
     ED_CHECK_LAUNCH();
     heis_rdm_reduce_kernel<<<(2 * npairs + 7) / 8, 256, 0, st>>>(scratch, nch + ntiles, a.npairs, map, npairs, out);
     ED_CHECK_LAUNCH();
