@@ -800,7 +800,7 @@ def main():
     # roofline of the dominant kernel of the solve, from the events of the timed solves
     dom = max(ksum, key=lambda k: ksum[k]["seconds"])
     tr = traffic_table()
-    names = {"hv": "hub_slab_kernel+hub_row_kernel", "multidot": "multidot_kernel", "update": "update_kernel"}
+    names = {"hv": "hub_slab_kernel+hub_row_col4_kernel", "multidot": "multidot32_kernel", "update": "update_kernel"}
 
     def roof(kind):
         d = ksum[kind]

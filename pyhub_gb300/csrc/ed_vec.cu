@@ -8,7 +8,7 @@
 // elements per thread, every such partial is promoted to FP64 and all further
 // accumulation is FP64, so no FP64 multiply is spent per element.  FP64
 // vectors: FP64 throughout.  (The FP32 multi-dot reduces each warp's 512
-// products in FP32 before the FP64 stage; see multidot_kernel.)
+// products in FP32 before the FP64 stage; see multidot32_kernel.)
 #include "ed_common.cuh"
 
 #include <algorithm>
