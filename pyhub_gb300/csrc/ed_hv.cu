@@ -559,7 +559,8 @@ static int launch_fused(ed_sector *s, cudaStream_t st, const T *x, T *y, HubArgs
     auto *kfn = add ? hub_fused_kernel<T, R, true> : hub_fused_kernel<T, R, false>;
     if (smem > 48 * 1024)
         ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int threads = (int)std::min<int64_t>(512, std::max<int64_t>(64, (R * s->nsup / 2 + 31) / 32 * 32));
+    // a thread a column (two to a thread keep two chains of loads in turn: 10 sites FP64 12.3 against 10.2 us)
+    const int threads = (int)std::min<int64_t>(512, std::max<int64_t>(64, (R * s->nsup + 31) / 32 * 32));
     // CTAs resident per SM: by threads (at most 1024 by registers) and by shared memory
     const int per_sm = (int)std::max<int64_t>(1, std::min<int64_t>(1024 / threads, (228 * 1024) / (int64_t)(smem + 1024)));
     const int64_t rb = (s->nsdn + R - 1) / R, resident = std::min<int64_t>((int64_t)nsm * per_sm, kMaxPartialBlocks);
