@@ -1334,8 +1334,9 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     }
     ED_CHECK_LAUNCH();
     // ---- pass S: one wave of resident CTAs walks the items (slab, eight rows).  A slab takes at most
-    // ~48 MB of L2; small sectors cut the columns further, down to one pass of 128, until every CTA
-    // has several items (a share of 3.4 items each would leave a wave 15% empty).
+    // 20 MB of L2 (FP32 4x7 832 us with 48 MB, 802 so; 4x8 15.1 and 13.3 ms; FP64 the same); small sectors
+    // cut the columns further, down to one pass of 128, until every CTA has several items (a share of 3.4
+    // items each would leave a wave 15% empty).
     SlabPlan p;
     p.nblk = 0;
     p.item_base[0] = 0;
@@ -1347,7 +1348,7 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
         const int64_t nr = h.row_base[m + 1] - h.row_base[m];
         if (nr == 0) continue;
         const int64_t len = h.ncol[m];
-        int64_t w = (int64_t)(48.0e6 / ((double)nr * sizeof(T)));
+        int64_t w = (int64_t)(20.0e6 / ((double)nr * sizeof(T)));
         w = w / 32 * 32;
         if (w < 256) w = 256;
         w = std::min(w, std::max<int64_t>(128, (len / cuts + 127) / 128 * 128));

@@ -264,24 +264,24 @@ template <typename T> struct alignas(sizeof(T) == 4 ? 8 : 16) RowHop {
 // and issues the loads of L neighbour rows back to back.
 template <typename T, int VW, int U, int L>
 __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, T *__restrict__ y,
-                                                       const HubArgs a, int64_t slab_w, int64_t ngroups,
-                                                       int64_t nitems, double *__restrict__ partials)
+                                                       const HubArgs a, int slab_w, int ngroups, int nitems,
+                                                       double *__restrict__ partials)
 {
     __shared__ RowHop<T> lists[8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RowHop<T> *hop = lists[warp];
     const T *__restrict__ cf = static_cast<const T *>(a.dcf);
-    const int64_t nsup = a.nsup, ld = a.ld;
+    const int nsup = (int)a.nsup;
+    const int64_t ld = a.ld;
     const T sc = (T)a.scale;
     double dxy = 0.0, dyy = 0.0;
-    for (int64_t item = blockIdx.x; item < nitems; item += gridDim.x) {
-        const int64_t slab = item / ngroups, g = item - slab * ngroups;
-        const int64_t d = g * 8 + warp;
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+        const int slab = item / ngroups, d = (item - slab * ngroups) * 8 + warp;
         if (d >= a.nsdn) continue;
-        const int64_t c0 = slab * slab_w, c1 = min(c0 + slab_w, nsup);
+        const int c0 = slab * slab_w, c1 = min(c0 + slab_w, nsup);
         const int e0 = __ldg(a.dptr + d), nn = __ldg(a.dptr + d + 1) - e0;
-        T *yr = y + d * ld;
-        const T *xd = x + d * ld;
+        T *yr = y + (int64_t)d * ld;
+        const T *xd = x + (int64_t)d * ld;
         float pxy = 0.f, pyy = 0.f;
         double qxy = 0.0, qyy = 0.0;
         auto dot = [&](T xv, T yv) {
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, 
             }
             __syncwarp();
             const bool last = (b0 + 32 >= nn);
-            int64_t cb = c0;
+            int cb = c0;
             // whole passes of U chunks
             for (; cb + 32 * VW * U <= c1; cb += 32 * VW * U) {
                 using V = typename std::conditional<VW == 1, T, typename std::conditional<sizeof(T) == 4, float4, double2>::type>::type;
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, 
                 }
             }
             // the rest of the slab, a column per lane
-            for (int64_t c = cb + lane; c < c1; c += 32) {
+            for (int c = cb + lane; c < c1; c += 32) {
                 T acc = yr[c];
 #pragma unroll 4
                 for (int e = 0; e < nb; ++e) acc += hop[e].cf * __ldg(x + hop[e].src * ld + c);
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, 
         }
         if (nn == 0 && partials) {
             // no down hops: the dots still need this row's y
-            for (int64_t cc = c0 + lane; cc < c1; cc += 32) {
+            for (int cc = c0 + lane; cc < c1; cc += 32) {
                 dot(__ldg(xd + cc), yr[cc]);
             }
         }
@@ -523,15 +523,16 @@ static constexpr int kMaxPartialBlocks = 1024;
 constexpr int64_t kFuseStates = 1 << 18;
 constexpr int64_t kFuseRow = 128;
 
-// L2 budget of one x slab in the slab pass: 48 MB (a third of the 129 MB
-// L2, leaving room for the y slab in flight and the tables); the
+// L2 budget of one x slab in the slab pass.  The part of L2 near an SM holds it only while it is small:
+// 4x4 FP32 (256 / 512 / 768 columns: 13 / 26 / 40 MB) 1,486 / 1,696 / 1,812 us the whole product, 16 sites
+// (7,7) 12 / 23 / 47 MB 1,170 / 1,198 / 1,418 us; FP64, bound by its pipe, is the same over that range.  The
 // environment variable PYHUB_ED_SLAB_L2_BYTES overrides it for tuning.
 static double slab_l2_bytes()
 {
     static double v = []() {
         const char *e = std::getenv("PYHUB_ED_SLAB_L2_BYTES");
         const double d = e ? std::atof(e) : 0.0;
-        return (d >= 1.0e6 && d <= 1.0e9) ? d : 48.0e6;
+        return (d >= 1.0e6 && d <= 1.0e9) ? d : 20.0e6;
     }();
     return v;
 }
@@ -666,8 +667,8 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     const int64_t ngroups = (s->nsdn + 7) / 8;
     const bool vec2 = (ld % VWS == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
                       ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
-    // chunks x rows in flight, measured (4x4 / 14 random bonds): FP32 2 x 2 1,012 us / 148 us the whole
-    // product, 1 x 4 1,070 / 154, 4 x 2 1,790 / 250 (registers); FP64 4 x 2 5.37 ms / 742 us, 2 x 4 6.26 / 743
+    // chunks x rows in flight, measured (4x4 slab pass / 14 random bonds): FP32 2 x 2 1,012 us / 148 us the
+    // whole product, 1 x 4 1,070 / 154, 4 x 2 1,790 / 250 (registers); FP64 4 x 2 5.37 ms / 742 us, 2 x 4 6.26 / 743
     auto *kfn = !vec2 ? hub_slab_kernel<T, 1, 1, 4>
                       : sizeof(T) == 4 ? hub_slab_kernel<T, VWS, 2, 2> : hub_slab_kernel<T, VWS, 4, 2>;
     // one wave of resident CTAs: each walks its share of the items, so a grid past the
@@ -686,7 +687,7 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     if (blocks2 > nitems) blocks2 = nitems;
     if (blocks2 < 1) blocks2 = 1;
     double *part = dots ? partials : nullptr;
-    kfn<<<(unsigned)blocks2, 256, 0, st>>>(x, y, a, slab_w, ngroups, nitems, part);
+    kfn<<<(unsigned)blocks2, 256, 0, st>>>(x, y, a, (int)slab_w, (int)ngroups, (int)nitems, part);
     ED_CHECK_LAUNCH();
     if (dots) return launch_reduce(partials, (int)blocks2, 2, dots, st);
     return ED_OK;
