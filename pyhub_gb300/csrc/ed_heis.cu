@@ -1334,9 +1334,11 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     }
     ED_CHECK_LAUNCH();
     // ---- pass S: one wave of resident CTAs walks the items (slab, eight rows).  A slab takes at most
-    // 20 MB of L2 (FP32 4x7 832 us with 48 MB, 802 so; 4x8 15.1 and 13.3 ms; FP64 the same); small sectors
-    // cut the columns further, down to one pass of 128, until every CTA has several items (a share of 3.4
-    // items each would leave a wave 15% empty).
+    // 20 MB of L2 in FP32 (48 / 30 / 20 / 10 MB: 4x7 864 / 821 / 811 / 828 us, 5x6 3.71 / 3.65 / 3.29 / 3.36
+    // ms, 4x8 15.3 / 15.5 / 13.5-14.2 / 13.5), 48 MB in FP64 (4x7 3.20 against 3.22 ms, 4x8 55.9 against 56.8,
+    // 5x6 15.1 against 14.9); small sectors cut the columns further, down to one pass of 128, until every CTA
+    // has several items (a share of 3.4 items each would leave a wave 15% empty).
+    const double slab_bytes = sizeof(T) == 4 ? 20.0e6 : 48.0e6;
     SlabPlan p;
     p.nblk = 0;
     p.item_base[0] = 0;
@@ -1348,7 +1350,7 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
         const int64_t nr = h.row_base[m + 1] - h.row_base[m];
         if (nr == 0) continue;
         const int64_t len = h.ncol[m];
-        int64_t w = (int64_t)(20.0e6 / ((double)nr * sizeof(T)));
+        int64_t w = (int64_t)(slab_bytes / ((double)nr * sizeof(T)));
         w = w / 32 * 32;
         if (w < 256) w = 256;
         w = std::min(w, std::max<int64_t>(128, (len / cuts + 127) / 128 * 128));
