@@ -180,7 +180,8 @@ int ed_rdm(ed_sector *s, void *stream, int dtype, int64_t ld, const void *bra, c
  * sum UL(J,K,M,N) c+_{K up} c_{J up} c+_{N down} c_{M down} (terms with
  * |UL| >= 1e-14) and the sector's on-site U is dropped (no ULDIAG term on
  * that path).  The work per element is the number of terms: meant for the
- * small clusters this interaction is used on. */
+ * small clusters this interaction is used on.  Products enqueued or captured
+ * before the call keep the on-site U they were enqueued with. */
 int ed_sector_set_uijkl(ed_sector *s, const double *ul);
 /* Device scratch bytes of ed_dbl_occ for nquads site quadruples. */
 int64_t ed_dbl_occ_scratch_bytes(const ed_sector *s, int nquads);

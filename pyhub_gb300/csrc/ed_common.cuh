@@ -205,8 +205,9 @@ struct ed_sector {
     bool u_uniform = true;
     double u_value = 0.0;
     double *u_lut = nullptr;       // [4][256]: on-site energy of the doubly occupied bits of one byte; then
-                                   // U times 0, 1, .. norb when U is uniform
+                                   // U times 0, 1, .. norb when U is uniform.  Enqueued products read it: never written again
     float *u_lut32 = nullptr;
+    double *u_zero = nullptr;      // the table of no on-site interaction (its zeros serve FP32 as well)
     ed::HeisTables heis;
     ed::HeisStruct *hs = nullptr;  // Heisenberg row tables
     ed::UijklTables *uijkl = nullptr;   // U_ijkl terms (ed_sector_set_uijkl), else NULL

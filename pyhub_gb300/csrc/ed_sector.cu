@@ -756,6 +756,8 @@ int ed_sector_create(int norb, int nup, int ndn, int kind, const double *t, cons
         TablePool pool;
         pool.add(&s->u_lut, ulut.data(), ulut.size());
         pool.add(&s->u_lut32, ulut32.data(), ulut32.size());
+        const std::vector<double> uzero(kULut, 0.0);
+        pool.add(&s->u_zero, uzero.data(), uzero.size());
         HostHop hu;
         rc = build_hop_host(norb, nup, t, hu);
         if (!rc) rc = upload_hop(hu, norb, nup, s->up, pool);

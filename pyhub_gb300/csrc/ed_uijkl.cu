@@ -205,8 +205,9 @@ extern "C" int ed_sector_set_uijkl(ed_sector *s, const double *ul)
     for (int b = 0; b < kMaxSites; ++b) s->u_site[b] = 0.0;
     s->u_uniform = true;
     s->u_value = 0.0;
-    ED_CHECK_CUDA(cudaMemset(s->u_lut, 0, sizeof(double) * kULut));
-    ED_CHECK_CUDA(cudaMemset(s->u_lut32, 0, sizeof(float) * kULut));
+    // later products are handed the table of zeros; those enqueued or captured before keep the one they were handed
+    s->u_lut = s->u_zero;
+    s->u_lut32 = reinterpret_cast<float *>(s->u_zero);
     uijkl_free(s->uijkl);
     s->uijkl = nullptr;
     if (jk.empty()) return ED_OK;
