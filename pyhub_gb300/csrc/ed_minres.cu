@@ -271,5 +271,6 @@ extern "C" int ed_minres(ed_sector *s, void *stream, int64_t ld, const double *p
     minres_scalar_kernel<<<1, 256, 0, st>>>(part, grid, 0, rtol, S);
     minres_project_kernel<<<grid, kMrThreads, 0, st>>>(n, x, psi, x, S, part);
     ED_CHECK_LAUNCH();
+    ED_CHECK_CUDA(cudaStreamSynchronize(st));      // x is final and the scratch free when the call returns
     return ED_OK;
 }

@@ -1,0 +1,34 @@
+"""ed_minres as a call: what it promises its caller about streams and buffers."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(edlib, n=8, nu=4, nd=4):
+    """A sector, a unit vector psi and a right-hand side (psi need not be an eigenvector)."""
+    import torch
+    rng = np.random.default_rng(11)
+    t = np.zeros((n, n))
+    for i in range(n):
+        t[i, (i + 1) % n] = t[(i + 1) % n, i] = -rng.uniform(0.5, 1.5)
+    sec = edlib.Sector(n, nu, nd, edlib.ED_HUBBARD, t=t, U=rng.uniform(2.0, 6.0, n))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(4)
+    psi = sec.from_ref(torch.randn(sec.dim, generator=g, dtype=torch.float64, device="cuda"))
+    psi /= torch.linalg.vector_norm(psi)
+    b = sec.from_ref(torch.randn(sec.dim, generator=g, dtype=torch.float64, device="cuda"))
+    return sec, psi, b
+
+
+@pytest.mark.parametrize("shape", [(8, 4, 4), (11, 5, 5), (12, 6, 6)])
+@pytest.mark.parametrize("maxiter", [0, 3])
+def test_the_stream_is_idle_when_the_call_returns(edlib, shape, maxiter):
+    import torch
+    sec, psi, b = _case(edlib, *shape)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for _ in range(5):
+        with torch.cuda.stream(side):
+            sec.minres(psi, -30.0, b, maxiter, 1e-10)
+            assert side.query()
