@@ -293,13 +293,19 @@ class Sector:
 
     def minres(self, psi, e0: float, b, maxiter: int, rtol: float, stream=None):
         """ed_minres: (x, iterations, relative residual) of (H - e0) x = b on the
-        complement of psi (FP64 device vectors in the internal layout)."""
+        complement of psi (FP64 device vectors in the internal layout).  A stream
+        of its own waits for the current one (where x and the scratch are
+        allocated); x is final on return."""
         import torch
         if psi.dtype != torch.float64 or b.dtype != torch.float64:
             raise TypeError("minres works in FP64")
         nb = int(lib().ed_minres_scratch_bytes(self._h, self.ld))
         scratch = torch.empty((nb + 7) // 8, dtype=torch.float64, device=psi.device)
         x = torch.zeros_like(b)
+        cur = torch.cuda.current_stream(psi.device)
+        if _stream(stream) != cur.cuda_stream:
+            own = stream if not isinstance(stream, int) else torch.cuda.ExternalStream(stream, device=psi.device)
+            own.wait_stream(cur)
         it, rr = _I(), _D()
         need = self.n if self.kind == ED_HUBBARD else self.dim
         check("ed_minres", lib().ed_minres(self._h, _stream(stream), self.ld, _ptr(psi, need, "psi"), float(e0),

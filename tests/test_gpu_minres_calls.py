@@ -32,3 +32,29 @@ def test_the_stream_is_idle_when_the_call_returns(edlib, shape, maxiter):
         with torch.cuda.stream(side):
             sec.minres(psi, -30.0, b, maxiter, 1e-10)
             assert side.query()
+
+
+@pytest.mark.parametrize("kind", ["stream", "handle"])
+def test_a_stream_of_its_own_waits_for_the_current_one(edlib, kind):
+    """The current stream is held up by a bounded spin: what Sector.minres enqueues there (x, b's last write) comes first."""
+    import torch
+    sec, psi, b = _case(edlib)
+    want, it0, rr0 = sec.minres(psi, -30.0, b, 6, 0.0)
+    late = torch.zeros_like(b)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    torch.cuda._sleep(100_000_000)      # ~50 ms
+    late.copy_(b)
+    x, it, rr = sec.minres(psi, -30.0, late, 6, 0.0, stream=side if kind == "stream" else side.cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(x, want) and (it, rr) == (it0, rr0)
+
+
+def test_the_default_streams_handle(edlib):
+    import torch
+    sec, psi, b = _case(edlib)
+    want, it0, rr0 = sec.minres(psi, -30.0, b, 6, 0.0)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        x, it, rr = sec.minres(psi, -30.0, b, 6, 0.0, stream=0)
+    assert torch.equal(x, want) and (it, rr) == (it0, rr0)
