@@ -227,6 +227,15 @@ extern "C" int ed_minres(ed_sector *s, void *stream, int64_t ld, const double *p
     *relres = 0.0;
     const int64_t n = s->kind == ED_HUBBARD ? s->nsdn * ld : s->dim, nv = minres_len(s, ld);
     if (n == 0) return ED_OK;
+    // x is cleared before b is read and written while psi and the scratch are in use
+    auto apart = [](const void *a, int64_t na, const void *c, int64_t nc) {
+        const uintptr_t pa = reinterpret_cast<uintptr_t>(a), pc = reinterpret_cast<uintptr_t>(c);
+        return pa + (uintptr_t)na <= pc || pc + (uintptr_t)nc <= pa;
+    };
+    const int64_t vb = n * (int64_t)sizeof(double), sb = ed_minres_scratch_bytes(s, ld);
+    ED_REQUIRE(apart(x, vb, b, vb) && apart(x, vb, psi, vb), "x must not alias b or psi");
+    ED_REQUIRE(apart(scratch, sb, x, vb) && apart(scratch, sb, b, vb) && apart(scratch, sb, psi, vb),
+               "the scratch must not alias x, b or psi");
     double *q = static_cast<double *>(scratch);
     double *u[2] = {q + nv, q + 2 * nv}, *w[2] = {q + 3 * nv, q + 4 * nv};
     double *S = q + 5 * nv, *part = S + kMScal;

@@ -58,3 +58,31 @@ def test_the_default_streams_handle(edlib):
     with torch.cuda.stream(torch.cuda.Stream()):
         x, it, rr = sec.minres(psi, -30.0, b, 6, 0.0, stream=0)
     assert torch.equal(x, want) and (it, rr) == (it0, rr0)
+
+
+def test_overlapping_buffers_are_refused(edlib):
+    import ctypes
+    import torch
+    sec, psi, b = _case(edlib)
+    L = edlib.lib()
+    nb = int(L.ed_minres_scratch_bytes(sec.handle, sec.ld))
+    scratch = torch.empty(nb // 8 + 1, dtype=torch.float64, device="cuda")
+    x = torch.full_like(b, 3.0)
+    wide = torch.zeros(2 * sec.n, dtype=torch.float64, device="cuda")
+    it, rr = ctypes.c_int(), ctypes.c_double()
+
+    def call(p, r, xx, sc):
+        return L.ed_minres(sec.handle, None, sec.ld, p, -30.0, r, xx, 3, 1e-10, ctypes.byref(it), ctypes.byref(rr),
+                           sc, nb)
+
+    P, B, X, S, W = (v.data_ptr() for v in (psi, b, x, scratch, wide))
+    keep = (psi.clone(), b.clone())
+    for args in ((P, B, B, S), (P, B, P, S), (P, W, W + 8 * (sec.n - 1), S), (P, W + 8 * (sec.n - 1), W, S),
+                 (P, B, S, S), (S, B, X, S), (P, S + 8, X, S)):
+        assert call(*args) == edlib.ED_ERR_ARG
+        assert "alias" in L.ed_last_error().decode()
+    torch.cuda.synchronize()
+    assert torch.equal(psi, keep[0]) and torch.equal(b, keep[1]) and bool((x == 3.0).all())
+    # side by side and b = psi are fine
+    assert call(P, W, W + 8 * sec.n, S) == edlib.ED_OK
+    assert call(P, P, X, S) == edlib.ED_OK
