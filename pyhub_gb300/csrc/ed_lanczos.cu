@@ -272,7 +272,7 @@ int ed::launch_coef(cudaStream_t st, int k, int mmax, const double *dots, int dr
                     double *state, double *coef, double *alpha, double *beta)
 {
     const size_t smem = coef_smem(k);
-    if (smem > 48 * 1024)
+    if (smem > 40 * 1024)      // the default limit of 48 KB holds the static arrays as well
         ED_CHECK_CUDA(cudaFuncSetAttribute(lanczos_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)coef_smem(kLanczosMax)));
     lanczos_coef_kernel<<<kCoefCtas, kCoefThreads, smem, st>>>(k, mmax, dots, drows, nrm, nrows, state, coef,
