@@ -53,13 +53,47 @@ __device__ __forceinline__ double dot_sum(const double *__restrict__ dots, int d
     return v[0];
 }
 
+// Part 1 of a step (below): s_k and the stop code from nrm2 = ||u_k||^2, beta_{k-1} through beta when not NULL.
+__device__ __forceinline__ void step_scale(int k, double nrm2, const double *__restrict__ state,
+                                           const double *__restrict__ alpha, double *__restrict__ beta, double &sk,
+                                           double &stop)
+{
+    stop = state[0];
+    sk = state[2 + k];
+    if (k < 1 || stop != 0.0) return;
+    const double pos = fmax(nrm2, 0.0), bk = sqrt(pos);
+    if (!isfinite(nrm2)) {
+        stop = -(double)k;
+        sk = 0.0;
+        return;
+    }
+    if (beta) beta[k - 1] = bk;
+    if (bk <= 1e-13 * fmax(1.0, fabs(alpha[k - 1]))) {
+        stop = (double)k;
+        sk = 0.0;
+    } else {
+        sk = rsqrt(pos);
+    }
+}
+
+// A closing call is part 1 alone: one warp, no cluster to bring up (k = 1 to 8,000: 2.4 us, in the kernel below 2.8).
+__global__ void __launch_bounds__(32) lanczos_close_kernel(int k, const double *__restrict__ nrm, double *state,
+                                                           const double *__restrict__ alpha, double *__restrict__ beta)
+{
+    if (threadIdx.x != 0) return;
+    double sk, stop;
+    step_scale(k, k >= 1 ? nrm[0] : 0.0, state, alpha, beta, sk, stop);
+    state[2 + k] = sk;
+    if (stop != 0.0) state[0] = stop;
+}
+
 // One cluster of kCoefCtas CTAs.  Part 1 (every call, k >= 1): beta_{k-1} and s_k from nrm, with
 // the breakdown test of the host loop (beta <= 1e-13 max(1, |alpha|)).
 // Part 1 is idempotent: a second call for the same k with the same nrm writes
 // the same beta_{k-1} and s_k.  The host's look-ahead relies on it (a run that
 // stops at a check has already enqueued the next step, whose part 1 rewrites
 // them before the Ritz vector is formed).  Part 2
-// (dots != NULL): G row k, Linv row k, coef and alpha_k; it also stops the run
+// (not in a closing call): G row k, Linv row k, coef and alpha_k; it also stops the run
 // when u_k is numerically dependent on the basis.  Once stopped, coef is
 // written as zeros (and s stays 0), so the vectors that follow are zero and
 // finite until the host sees the stop code.
@@ -83,7 +117,6 @@ __global__ void __cluster_dims__(kCoefCtas, 1, 1) __launch_bounds__(kCoefThreads
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), t = threadIdx.x, lane = t & 31;
     double *s = state + 2;
-    if (dots == nullptr && rank != 0) return;
     // ||u_k||^2, or its partial sums in the order of launch_reduce
     double nrm2 = 0.0;
     if (nrows > 64) {
@@ -97,37 +130,21 @@ __global__ void __cluster_dims__(kCoefCtas, 1, 1) __launch_bounds__(kCoefThreads
         nrm2 = nrm[0];
     }
     if (t == 0) {
-        double stop = state[0], sk = s[k];
-        if (k >= 1 && stop == 0.0) {
-            const double nb = nrm2, pos = fmax(nb, 0.0);
-            const double bk = sqrt(pos);
-            if (!isfinite(nb)) {
-                stop = -(double)k;
-                sk = 0.0;
-            } else {
-                if (rank == 0) beta[k - 1] = bk;
-                if (bk <= 1e-13 * fmax(1.0, fabs(alpha[k - 1]))) {
-                    stop = (double)k;
-                    sk = 0.0;
-                } else {
-                    sk = rsqrt(pos);
-                }
-            }
-        }
+        double sk, stop;
+        step_scale(k, nrm2, state, alpha, rank == 0 ? beta : nullptr, sk, stop);
         head[0] = sk;
         head[1] = stop;
     }
     __syncthreads();
     const double sk = head[0], stop = head[1];
-    if (dots == nullptr || stop != 0.0) {
-        if (dots != nullptr) cluster.sync();   // every CTA has read the state before rank 0 writes it
+    if (stop != 0.0) {
+        cluster.sync();      // every CTA has read the state before rank 0 writes it
         if (rank != 0) return;
         if (t == 0) {
             s[k] = sk;
-            if (stop != 0.0) state[0] = stop;
+            state[0] = stop;
         }
-        if (dots != nullptr)
-            for (int j = t; j <= k; j += kCoefThreads) coef[j] = 0.0;
+        for (int j = t; j <= k; j += kCoefThreads) coef[j] = 0.0;
         return;
     }
     double *Linv = state + lz_linv_off(mmax);
@@ -271,6 +288,11 @@ extern "C" int ed_lanczos_coef(void *stream, int k, int mmax, const double *dots
 int ed::launch_coef(cudaStream_t st, int k, int mmax, const double *dots, int drows, const double *nrm, int nrows,
                     double *state, double *coef, double *alpha, double *beta)
 {
+    if (dots == nullptr) {
+        lanczos_close_kernel<<<1, 32, 0, st>>>(k, nrm, state, alpha, beta);
+        ED_CHECK_LAUNCH();
+        return ED_OK;
+    }
     const size_t smem = coef_smem(k);
     if (smem > 40 * 1024)      // the default limit of 48 KB holds the static arrays as well
         ED_CHECK_CUDA(cudaFuncSetAttribute(lanczos_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

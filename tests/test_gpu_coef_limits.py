@@ -79,3 +79,42 @@ def test_largest_gram_entry(edlib, k):
         nxt[2 * k + 3] = 1.0
         edlib.lanczos_coef(k + 1, m, nxt, nrm, st, coef, ab[0], ab[1])
         assert float(st[0]) == 0.0 and float(st[1]) == want
+
+
+@pytest.mark.parametrize("k", [0, 1, 40])
+@pytest.mark.parametrize("case", ["healthy", "breakdown", "non-finite", "stopped"])
+def test_closing_call_is_part_one_of_the_step(edlib, k, case):
+    """A closing call writes what the step's first part writes, bit for bit, and nothing else; a step after it agrees."""
+    import torch
+    m = 48
+    nb = {"healthy": 2.3, "breakdown": 1e-28, "non-finite": float("inf"), "stopped": 2.3}[case]
+    got = []
+    for close_first in (False, True):
+        st = torch.zeros(edlib.lanczos_state_doubles(m), dtype=torch.float64, device="cuda")
+        st[2:3 + k] = 0.7
+        if case == "stopped":
+            st[0] = 3.0
+        lin = st[3 + m:3 + m + (m + 1) ** 2].view(m + 1, m + 1)
+        lin[:k, :k] = torch.eye(k, dtype=torch.float64, device="cuda")
+        nrm = torch.tensor([nb], dtype=torch.float64, device="cuda")
+        ab = torch.ones(2, m, dtype=torch.float64, device="cuda")
+        if close_first:
+            before = st.clone()
+            edlib.lanczos_coef(k, m, None, nrm, st, None, ab[0], ab[1])
+            same = torch.ones_like(st, dtype=torch.bool)
+            same[0] = same[2 + k] = False
+            assert torch.equal(st[same], before[same])
+            first = (st[0].clone(), st[2 + k].clone(), ab.clone())
+        dots = torch.zeros(2 * (k + 1), dtype=torch.float64, device="cuda")
+        dots[2 * k + 1] = 1.0 / (0.49 if k == 0 else 1.0 / 2.3)
+        coef = torch.full((k + 1,), 9.0, dtype=torch.float64, device="cuda")
+        edlib.lanczos_coef(k, m, dots, nrm, st, coef, ab[0], ab[1])
+        got.append((st.clone(), coef, ab.clone()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    st, _, ab = got[0]
+    assert torch.equal(first[0], st[0]) and torch.equal(first[1], st[2 + k])
+    if k:
+        assert torch.equal(first[2][1], ab[1])
+    want = {"healthy": 0.0, "breakdown": float(k), "non-finite": -float(k), "stopped": 3.0}[case]
+    assert float(st[0]) == (want if k else (3.0 if case == "stopped" else 0.0))
