@@ -45,6 +45,7 @@ NADD = 5
 # a block against one step: 6,720 elements 4.2 / 4.6 ms, 64,512 6.4 / 7.1, 221,760 13.7 / 13.3,
 # 633,600 34.4 / 32.5 (there the steps of the block that the run does not keep cost more than the wait).
 LOOKAHEAD_SMALL = 1 << 17
+MAX_BASIS = 1600       # vectors that one multi-dot with two right-hand sides takes (200 KB of partial sums per CTA)
 
 
 def _torch():
@@ -316,6 +317,8 @@ def lanczos_full(sec, v0, max_steps: int, dtype=None, rule=None, check_every: in
                                                -(-min_steps // check_every) * check_every))
         if pending is not None:
             k1 = min(k1, k_done + ahead)
+        if k_done < MAX_BASIS < k1:
+            k1 = MAX_BASIS     # a check in flight may end the run before the step that has no room
         sec.lanczos_steps(V, k_done, k1, m, w, state, ab[0], ab[1], sbuf)
         k_done = k1
         if pending is not None:
