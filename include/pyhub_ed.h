@@ -248,10 +248,11 @@ int ed_rdm1(ed_sector *s, void *stream, int dtype, int64_t ld, const void *psi, 
 /* MINRES for (H - e0) x = b on the complement of psi (FP64 vectors of row
  * stride ld, row padding zero): b is projected off psi, every product too, x
  * is returned off psi.  Stops at residual rtol * |b| or after maxiter
- * iterations; iters and relres (host) report the count and the residual
- * reached.  scratch: ed_minres_scratch_bytes, 16-byte aligned.  x and the
- * scratch must not overlap each other, b or psi.  Synchronises the stream.
- * No reference counterpart. */
+ * iterations (none for maxiter <= 0; a negative rtol is never met); iters
+ * and relres (host) report the count and the residual reached.  scratch:
+ * ed_minres_scratch_bytes, 16-byte aligned.  x and the scratch must not
+ * overlap each other, b or psi.  Synchronises the stream.  No reference
+ * counterpart. */
 int64_t ed_minres_scratch_bytes(const ed_sector *s, int64_t ld);
 int ed_minres(ed_sector *s, void *stream, int64_t ld, const double *psi, double e0, const double *b, double *x,
               int maxiter, double rtol, int *iters, double *relres, void *scratch, int64_t scratch_bytes);

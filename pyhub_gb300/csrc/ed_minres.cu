@@ -216,7 +216,6 @@ extern "C" int ed_minres(ed_sector *s, void *stream, int64_t ld, const double *p
     clear_error();
     ED_REQUIRE(s != nullptr, "sector is NULL");
     ED_REQUIRE(psi != nullptr && b != nullptr && x != nullptr && iters != nullptr && relres != nullptr, "NULL argument");
-    ED_REQUIRE(maxiter >= 0 && rtol >= 0.0, "maxiter=%d or rtol=%g is negative", maxiter, rtol);
     ED_REQUIRE(s->kind != ED_HUBBARD || ld >= s->nsup, "ld=%lld below nsup=%lld", (long long)ld, (long long)s->nsup);
     ED_REQUIRE(scratch != nullptr && scratch_bytes >= ed_minres_scratch_bytes(s, ld),
                "scratch of %lld bytes is below the %lld needed", (long long)scratch_bytes,

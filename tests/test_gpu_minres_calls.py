@@ -86,3 +86,22 @@ def test_overlapping_buffers_are_refused(edlib):
     # side by side and b = psi are fine
     assert call(P, W, W + 8 * sec.n, S) == edlib.ED_OK
     assert call(P, P, X, S) == edlib.ED_OK
+
+
+@pytest.mark.parametrize("maxiter,rtol", [(0, 1e-10), (-3, 1e-10), (4, -1.0), (4, float("nan"))])
+def test_odd_limits_run_as_the_torch_recurrence(edlib, maxiter, rtol):
+    """No iterations for maxiter <= 0 (x = 0, residual 1); a tolerance that cannot be met runs to maxiter."""
+    import torch
+    from pyhub_gb300.core import gradients as GR
+    sec, psi, b = _case(edlib)
+    work = torch.zeros_like(b)
+
+    def apply(v):
+        sec.hv(v, work)
+        return work + 30.0 * v
+
+    x0, it0, rr0 = GR.minres(apply, b, psi, maxiter=maxiter, rtol=rtol)
+    x, it, rr = sec.minres(psi, -30.0, b, maxiter, rtol)
+    assert it == it0 and abs(rr - rr0) <= 1e-10
+    # both recurrences agree to rounding: a few iterations of a system of condition ~10
+    assert float(torch.linalg.vector_norm(x - x0)) <= 1e-12 * float(torch.linalg.vector_norm(x0))
