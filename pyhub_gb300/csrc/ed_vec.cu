@@ -12,6 +12,7 @@
 #include "ed_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace ed {
 
@@ -106,10 +107,13 @@ __global__ void __launch_bounds__(kVecThreads, kVecResident) multidot32_kernel(i
 }
 
 // FP64, same partials.  An FP64 instruction costs 64 FP32 ones on this chip, so the pass is bound by
-// the FP64 pipe (two FMA per basis element) and spends it on nothing else: a CTA owns kJ64 vectors
-// and one range of elements, every thread keeps its 2*kJ64 sums in registers over the whole range,
+// the FP64 pipe (two FMA per basis element) and spends it on nothing else: a CTA owns up to KJ vectors
+// and one range of elements, every thread keeps its 2*KJ sums in registers over the whole range,
 // and lanes are summed once at its end (the pass that summed lanes after every 16 elements took 11
-// FP64 instructions per 8 here).  w and z are read again for every kJ64 vectors, from L2.
+// FP64 instructions per 8 here).  w and z are read again for every KJ = kJ64 vectors, from L2.
+// With few vectors (KJ < kJ64) the loads are the time: U steps of all vectors are in flight together
+// (one vector of 1.7e8: 778 us with kJ64 and one step, 375 so; of 300,000: 9.5 -> 4.9), and one wave of
+// CTAs has less to start and to sum (seven of 500,000 and z: 29.5 -> 23.6 us).
 static constexpr int kJ64 = 8;
 static constexpr int kStep64 = kVecThreads * 2;   // elements of one iteration: a 16-byte load per thread
 
@@ -140,50 +144,57 @@ __device__ __forceinline__ void warp_sum_many(double (&v)[N])
     for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
 }
 
-template <bool Z>
-__global__ void __launch_bounds__(kVecThreads, 2) multidot64_kernel(int64_t n, const double *__restrict__ V,
+// CTAs of a variant that an SM holds (registers)
+template <int KJ, int U> constexpr int multidot64_ctas() { return KJ == 1 && U == 4 ? 4 : KJ == 2 ? 3 : 2; }
+
+template <bool Z, int KJ, int U>
+__global__ void __launch_bounds__(kVecThreads, multidot64_ctas<KJ, U>()) multidot64_kernel(int64_t n, const double *__restrict__ V,
                                                                     int64_t ldv, int nvec,
                                                                     const double *__restrict__ w,
                                                                     const double *__restrict__ z,
                                                                     double *__restrict__ partials)
 {
-    constexpr int NS = Z ? 2 * kJ64 : kJ64;
+    constexpr int NS = Z ? 2 * KJ : KJ;
     __shared__ double red[kVecThreads / 32][NS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ng = gridDim.y;
     const int j0 = (int)((int64_t)nvec * blockIdx.y / ng), nj = (int)((int64_t)nvec * (blockIdx.y + 1) / ng) - j0;
-    const int64_t steps = (n + kStep64 - 1) / kStep64;
+    const int64_t steps = (n + U * kStep64 - 1) / (U * kStep64);
     const int64_t s0 = steps * blockIdx.x / gridDim.x, s1 = steps * (blockIdx.x + 1) / gridDim.x;
     double acc[NS];
 #pragma unroll
     for (int q = 0; q < NS; ++q) acc[q] = 0.0;
     const double *Vj = V + (int64_t)j0 * ldv;
     for (int64_t st = s0; st < s1; ++st) {
-        const int64_t i = st * kStep64 + threadIdx.x * 2;
-        double2 v[kJ64];
+        const int64_t i = st * (U * kStep64) + threadIdx.x * 2;
+        double2 v[U][KJ], a[U], b[U];
 #pragma unroll
-        for (int j = 0; j < kJ64; ++j)
-            if (j < nj) v[j] = load2(Vj + (int64_t)j * ldv, i, n);
-        const double2 a = load2(w, i, n);
-        double2 b;
-        if constexpr (Z) b = load2(z, i, n);
+        for (int u = 0; u < U; ++u) {
 #pragma unroll
-        for (int j = 0; j < kJ64; ++j) {
-            if (j >= nj) break;
-            acc[j] = fma(v[j].x, a.x, acc[j]);
-            if constexpr (Z) acc[kJ64 + j] = fma(v[j].x, b.x, acc[kJ64 + j]);
-            acc[j] = fma(v[j].y, a.y, acc[j]);
-            if constexpr (Z) acc[kJ64 + j] = fma(v[j].y, b.y, acc[kJ64 + j]);
+            for (int j = 0; j < KJ; ++j)
+                if (j < nj) v[u][j] = load2(Vj + (int64_t)j * ldv, i + u * kStep64, n);
+            a[u] = load2(w, i + u * kStep64, n);
+            if constexpr (Z) b[u] = load2(z, i + u * kStep64, n);
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) {
+                if (j >= nj) break;
+                acc[j] = fma(v[u][j].x, a[u].x, acc[j]);
+                if constexpr (Z) acc[KJ + j] = fma(v[u][j].x, b[u].x, acc[KJ + j]);
+                acc[j] = fma(v[u][j].y, a[u].y, acc[j]);
+                if constexpr (Z) acc[KJ + j] = fma(v[u][j].y, b[u].y, acc[KJ + j]);
+            }
     }
     warp_sum_many<NS>(acc);
     if (lane % (32 / NS) == 0) red[warp][lane / (32 / NS)] = acc[0];
     __syncthreads();
-    const int q = threadIdx.x, j = q % kJ64;
+    const int q = threadIdx.x, j = q % KJ;
     if (q < NS && j < nj) {
         double s = 0.0;
         for (int k = 0; k < kVecThreads / 32; ++k) s += red[k][q];
-        partials[(int64_t)blockIdx.x * (Z ? 2 * nvec : nvec) + (q < kJ64 ? 0 : nvec) + j0 + j] = s;
+        partials[(int64_t)blockIdx.x * (Z ? 2 * nvec : nvec) + (q < KJ ? 0 : nvec) + j0 + j] = s;
     }
 }
 
@@ -347,17 +358,34 @@ int launch_multidot(cudaStream_t st, int dtype, int64_t n, const void *V, int64_
             static_cast<const float *>(z), part);
         *rows = gx;
     } else {
-        const int64_t steps = (n + kStep64 - 1) / kStep64;
-        // groups of 5 to kJ64 vectors, as even as they come: the CTAs with the largest group end the pass
-        int ng = (nvec + kJ64 - 1) / kJ64;
-        for (int g = ng + 1; g <= (nvec + 4) / 5; ++g)
-            if ((int64_t)((nvec + g - 1) / g) * g < (int64_t)((nvec + ng - 1) / ng) * ng) ng = g;
-        const int gx = (int)std::max<int64_t>(1, std::min(steps, ctas / ng));   // whole waves: one CTA more costs a wave
-        const dim3 grid((unsigned)gx, (unsigned)ng);
         const double *Vd = static_cast<const double *>(V), *wd = static_cast<const double *>(w),
                      *zd = static_cast<const double *>(z);
-        if (z) multidot64_kernel<true><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
-        else multidot64_kernel<false><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
+        int ng = 1, gx = 0;
+        // one group: a wave of resident CTAs; several groups, of unequal sizes: two.  One CTA more than
+        // whole waves costs a wave
+        auto launch = [&](auto kj, auto un) {
+            constexpr int KJ = decltype(kj)::value, U = decltype(un)::value;
+            const int64_t steps = (n + U * kStep64 - 1) / (U * kStep64);
+            const int64_t fill = ng == 1 ? (int64_t)num_sms() * multidot64_ctas<KJ, U>() : ctas;
+            gx = (int)std::max<int64_t>(1, std::min(steps, std::min(fill, ctas) / ng));
+            const dim3 grid((unsigned)gx, (unsigned)ng);
+            if (z) multidot64_kernel<true, KJ, U><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
+            else multidot64_kernel<false, KJ, U><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
+        };
+        using std::integral_constant;
+        if (nvec == 1) {
+            launch(integral_constant<int, 1>(), integral_constant<int, 4>());
+        } else if (nvec == 2) {
+            launch(integral_constant<int, 2>(), integral_constant<int, 4>());
+        } else if (nvec <= 4) {
+            launch(integral_constant<int, 4>(), integral_constant<int, 2>());
+        } else {
+            // groups of 5 to kJ64 vectors, as even as they come: the CTAs with the largest group end the pass
+            ng = (nvec + kJ64 - 1) / kJ64;
+            for (int g = ng + 1; g <= (nvec + 4) / 5; ++g)
+                if ((int64_t)((nvec + g - 1) / g) * g < (int64_t)((nvec + ng - 1) / ng) * ng) ng = g;
+            launch(integral_constant<int, kJ64>(), integral_constant<int, 1>());
+        }
         *rows = gx;
     }
     ED_CHECK_LAUNCH();
