@@ -202,9 +202,8 @@ __global__ void __launch_bounds__(kVecThreads, multidot64_ctas<KJ, U>()) multido
 // scalar, or 1 when wscale is NULL), optional partial <out,out>.
 // Accumulation type A: FP32 for an FP32 basis with FP32 output, FP64 otherwise.
 // EPT elements per thread, NT threads: 16 x 256 streams long vectors at the HBM rate (FP64: the FP64
-// pipe's), 4 x 128 spreads shorter ones evenly over the SMs (FP64, 50 vectors of 853,872: 125 ->
-// 97 us; from about 2.5 M elements on the 16-element form is as fast or faster: FP32, 4 M: 131 us
-// against 146).
+// pipe's), 4 x 128 spreads shorter ones evenly over the SMs (FP64, 50 vectors of 853,888: 120 ->
+// 91 us; launch_update has the line between them).
 template <typename T, typename O, typename A, int EPT, int NT>
 __global__ void __launch_bounds__(NT) update_kernel(int64_t n, const T *__restrict__ V, int64_t ldv,
                                                              int nvec, const double *__restrict__ coef,
@@ -399,16 +398,26 @@ static int launch_update(cudaStream_t st, int64_t n, const T *V, int64_t ldv, in
     const int64_t ctas = vec_ctas();
     const size_t smem = sizeof(double) * (size_t)(nvec > 0 ? nvec : 1);
     const int64_t tiles = (n + kSplitTile - 1) / kSplitTile;
-    // up to four tiles per CTA of the split form; then 4 elements per thread until the 16-element
-    // chunks fill every resident CTA
-    if (tiles <= 4 * ctas) {
+    // The split form takes short vectors (up to four tiles per CTA), where a warp has vectors enough to pay
+    // for the exchange; more of them the more tiles share the loads: 16,000 elements from 4 vectors on in
+    // both types, 63,488 FP32 10: 6.6 us against 7.5 for 4 x 128, FP64 24: 11.2 against 11.7; 300,000 FP32 50:
+    // 14.7 / 15.5, FP64 64: 49 / 52.  With fewer: 300,000 and one vector FP32 8.7 against 6.0, FP64 14.1 / 7.3.
+    // 4 x 128 takes the rest up to where 16-element chunks fill every resident CTA (FP64, bound by its
+    // pipe), or (FP32, bound by the streams) while its chunks have a CTA each and there are vectors enough
+    // to outlast the CTAs' start: 853,888 elements 32 vectors 24.4 us against 28.6, 12: 11.1 / 9.6;
+    // 1.5 M, 100 vectors 126 / 99.
+    const int64_t chunks = (n + kChunk - 1) / kChunk;
+    constexpr bool f64 = sizeof(A) == 8;
+    const int64_t split_from = tiles <= 2 * num_sms() ? 4 : f64 ? std::min<int64_t>(64, tiles / 20) : tiles / 45;
+    const bool small = f64 ? chunks < ctas : (n + 511) / 512 <= kMaxNormRows && 9 * (int64_t)nvec >= chunks;
+    if (tiles <= 4 * ctas && nvec >= split_from) {
         *rows = (int)std::min(tiles, ctas);
         update_split_kernel<T, O, A><<<*rows, kVecThreads, 0, st>>>(n, V, ldv, nvec, coef, wscale, w, out, part);
-    } else if ((n + kChunk - 1) / kChunk < ctas) {
+    } else if (small) {
         *rows = (int)std::min<int64_t>((n + 511) / 512, kMaxNormRows);
         update_kernel<T, O, A, 4, 128><<<*rows, 128, smem, st>>>(n, V, ldv, nvec, coef, wscale, w, out, part);
     } else {
-        *rows = (int)std::min<int64_t>((n + kChunk - 1) / kChunk, ctas);
+        *rows = (int)std::min<int64_t>(chunks, ctas);
         update_kernel<T, O, A, kEPT, kVecThreads><<<*rows, kVecThreads, smem, st>>>(n, V, ldv, nvec, coef, wscale, w,
                                                                                     out, part);
     }

@@ -39,3 +39,40 @@ def test_multidot_few_vectors(edlib, n, nvec):
             p = V[j % nvec, :n] * (w if j < nvec else z)[:n]
             assert abs(got[j] - float(p.sum())) <= 1.05 * (n / 256 + 48) * 2.0 ** -53 * float(p.abs().sum()), (j, zz is None)
         assert np.isnan(got[m])
+
+
+# (elements, vectors) on both sides of every line between the split, the 4 x 128 and the 16 x 256 form
+UPDATE = [(38_912, 3), (38_912, 4), (38_913, 4), (38_913, 15), (63_488, 10), (63_488, 11), (63_488, 24), (63_488, 25),
+          (200_000, 5), (200_000, 34), (200_000, 63), (200_000, 64), (311_296, 1), (311_296, 9), (311_296, 54),
+          (311_297, 8), (311_297, 64), (853_888, 23), (853_888, 24), (1_048_576, 28), (1_048_576, 29),
+          (1_048_577, 100), (1_048_577, 1)]
+
+
+@pytest.mark.parametrize("n,nvec", UPDATE)
+@pytest.mark.parametrize("dt", ["f32", "f64", "f32-f64", "f64-f32"])
+def test_update_forms(edlib, n, nvec, dt):
+    """Per element (nvec + 4) u (|ws w| + sum |c v|), u that of the accumulation, and one rounding to the output's
+    type; the norm over 16 elements in FP32, then FP64: 17 u + n 2^-53 (FP64: (n / 256 + 48) 2^-53)."""
+    import torch
+    td = torch.float32 if dt.startswith("f32") else torch.float64
+    od = torch.float32 if dt in ("f32", "f64-f32") else torch.float64
+    u = 2.0 ** -24 if dt == "f32" else 2.0 ** -53
+    uo = 2.0 ** -24 if od == torch.float32 else 2.0 ** -53
+    ld, V, w, z, g = _vectors(n, nvec, td, n + nvec)
+    w = w.to(od)
+    coef = torch.randn(nvec, generator=g, dtype=torch.float64, device="cuda")
+    scratch = torch.full((edlib.scratch_bytes(n, nvec) // 8 + 1,), float("nan"), dtype=torch.float64, device="cuda")
+    V64, c = V[:, :n].double(), coef.to(torch.float32).double() if dt == "f32" else coef
+    ws = torch.tensor([0.75], dtype=torch.float64, device="cuda")
+    for start, in_place in ((w, False), (w.clone(), True), (None, False)):
+        head = 0.75 * start[:n].double() if start is not None else torch.zeros(n, dtype=torch.float64, device="cuda")
+        want, mag = head - c @ V64, head.abs() + c.abs() @ V64.abs()
+        out = start if in_place else torch.full((ld,), -7.0, dtype=od, device="cuda")
+        tail = out[n:].clone()
+        nrm = torch.zeros(2, dtype=torch.float64, device="cuda")
+        edlib.update(V, nvec, coef, start, out, norm2=nrm, scratch=scratch, n=n, wscale=None if start is None else ws)
+        assert bool(((out[:n].double() - want).abs() <= 1.05 * ((nvec + 4) * u * mag + uo * want.abs())).all())
+        assert torch.equal(out[n:], tail)
+        got = float((out[:n].double() ** 2).sum())
+        tol = 17 * uo + n * 2.0 ** -53 if od == torch.float32 else (n / 256 + 48) * 2.0 ** -53
+        assert abs(float(nrm[0]) - got) <= 1.05 * tol * got
