@@ -435,6 +435,22 @@ __global__ void __launch_bounds__(kBatchThreads) batch_hv_kernel(const BatchInst
     hv_item<T, R, false>(inst, b, i, u, y, scal[(int64_t)i * kScal + kS], part_out, smem_raw);
 }
 
+// FP64 with eight rows, four CTAs an SM (60 registers): left to itself the compiler takes 79, and clusters
+// whose rows leave room for a fourth CTA miss it (512 of 4 sites 18.1 -> 12.5 us, eight of 12 sites (4,4)
+// 148 -> 136; four of 12 sites half filled, where shared memory holds two, 243 -> 246).  A bound of one CTA on the others is
+// not the same as none: it lets the compiler take registers up to one CTA an SM.
+template <>
+__global__ void __launch_bounds__(kBatchThreads, 4)
+    batch_hv_kernel<double, 8>(const BatchInst *__restrict__ inst, const int32_t *__restrict__ blk_inst,
+                               const double *__restrict__ u, double *__restrict__ y, const double *__restrict__ scal,
+                               double *__restrict__ part_out)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int64_t b = blockIdx.x;
+    const int i = __ldg(blk_inst + b);
+    hv_item<double, 8, false>(inst, b, i, u, y, scal[(int64_t)i * kScal + kS], part_out, smem_raw);
+}
+
 // u_next = y - c_cur u_k - c_prev u_prev, written to un (which is u_prev
 // itself when only two Krylov vectors are kept, a new basis slot otherwise),
 // partial ||u_next||^2, in 16-byte vectors over the CTA's rows (padding is
