@@ -262,7 +262,7 @@ template <typename T> struct alignas(sizeof(T) == 4 ? 8 : 16) RowHop {
 // keeps its row's neighbour list in shared memory (one 8- or 16-byte broadcast
 // read per hop; two or three shuffles per hop before), walks U chunks of 32*VW columns together
 // and issues the loads of L neighbour rows back to back.
-template <typename T, int VW, int U, int L>
+template <typename T, int VW, int U, int L, bool SINGLE>
 __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, T *__restrict__ y,
                                                        const HubArgs a, int slab_w, int ngroups, int nitems,
                                                        double *__restrict__ partials)
@@ -297,18 +297,18 @@ __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, 
             }
             __syncwarp();
             const bool last = (b0 + 32 >= nn);
-            int cb = c0;
-            // whole passes of U chunks
-            for (; cb + 32 * VW * U <= c1; cb += 32 * VW * U) {
+            // UN chunks of 32*VW columns from cb on, NL neighbour rows' loads in flight
+            auto pass = [&](auto chunks, auto loads, int cb) {
+                constexpr int UN = decltype(chunks)::value, NL = decltype(loads)::value;
                 using V = typename std::conditional<VW == 1, T, typename std::conditional<sizeof(T) == 4, float4, double2>::type>::type;
                 const V *xc = reinterpret_cast<const V *>(x + cb) + lane;
                 V *yc = reinterpret_cast<V *>(yr + cb) + lane;
-                V acc[U];
+                V acc[UN];
 #pragma unroll
-                for (int u = 0; u < U; ++u) acc[u] = yc[u * 32];
+                for (int u = 0; u < UN; ++u) acc[u] = yc[u * 32];
                 auto hops = [&](auto count, int e) {
                     constexpr int N = decltype(count)::value;
-                    V v[N][U];
+                    V v[N][UN];
                     T w[N];
 #pragma unroll
                     for (int i = 0; i < N; ++i) {
@@ -316,33 +316,47 @@ __global__ void __launch_bounds__(256) hub_slab_kernel(const T *__restrict__ x, 
                         w[i] = h.cf;
                         const V *xr = reinterpret_cast<const V *>(reinterpret_cast<const T *>(xc) + h.src * ld);
 #pragma unroll
-                        for (int u = 0; u < U; ++u) v[i][u] = __ldg(xr + u * 32);
+                        for (int u = 0; u < UN; ++u) v[i][u] = __ldg(xr + u * 32);
                     }
 #pragma unroll
                     for (int i = 0; i < N; ++i)
 #pragma unroll
-                        for (int u = 0; u < U; ++u)
+                        for (int u = 0; u < UN; ++u)
 #pragma unroll
                             for (int k = 0; k < VW; ++k)
                                 reinterpret_cast<T *>(&acc[u])[k] += w[i] * reinterpret_cast<const T *>(&v[i][u])[k];
                 };
                 int e = 0;
-                for (; e + L <= nb; e += L) hops(std::integral_constant<int, L>(), e);
-                if (L > 2 && e + 2 <= nb) {
+                for (; e + NL <= nb; e += NL) hops(std::integral_constant<int, NL>(), e);
+                if (NL > 2 && e + 2 <= nb) {
                     hops(std::integral_constant<int, 2>(), e);
                     e += 2;
                 }
                 for (; e < nb; ++e) hops(std::integral_constant<int, 1>(), e);
 #pragma unroll
-                for (int u = 0; u < U; ++u) yc[u * 32] = acc[u];
+                for (int u = 0; u < UN; ++u) yc[u * 32] = acc[u];
                 if (partials && last) {
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
+                    for (int u = 0; u < UN; ++u) {
                         const V xv = __ldg(reinterpret_cast<const V *>(xd + cb) + lane + u * 32);
 #pragma unroll
                         for (int k = 0; k < VW; ++k)
                             dot(reinterpret_cast<const T *>(&xv)[k], reinterpret_cast<const T *>(&acc[u])[k]);
                     }
+                }
+            };
+            using std::integral_constant;
+            int cb = c0;
+            // whole passes of U chunks
+            for (; cb + 32 * VW * U <= c1; cb += 32 * VW * U) pass(integral_constant<int, U>(), integral_constant<int, L>(), cb);
+            if constexpr (SINGLE) {
+                // whole chunks, then a short one of lanes with VW columns (not for 32 columns or fewer in FP64, where an
+                // idle lane costs the pipe what a busy one does)
+                constexpr int kAlone = sizeof(T) == 4 ? 0 : 32;
+                for (; cb + 32 * VW <= c1; cb += 32 * VW) pass(integral_constant<int, 1>(), integral_constant<int, 4>(), cb);
+                if (c1 - cb > kAlone) {
+                    if (cb + (lane + 1) * VW <= c1) pass(integral_constant<int, 1>(), integral_constant<int, 4>(), cb);
+                    cb += (c1 - cb) / VW * VW;
                 }
             }
             // the rest of the slab, a column per lane
@@ -518,10 +532,12 @@ static constexpr int kMaxPartialBlocks = 1024;
 
 // Sectors that take the one-pass product.  Measured one pass / two: 8-site ring FP64 9.4 / 12.8 us (one launch
 // instead of two), 11 sites half filled (213,444) FP64 22.5 / 26.7, FP32 11.9 / 18.5; 16 sites (3,3)
-// (313,600) 28.7 / 26.7 and 16.4 / 13.9, 3x4 half filled 101 / 81 and 48 / 23.  Rows of at most 128
-// strings leave most of a row CTA idle: 16 sites (2,8), 1.5 M states, 115 / 125 and 41 / 68.
+// (313,600) 28.7 / 26.7 and 16.4 / 13.9, 3x4 half filled 101 / 81 and 48 / 23.  Rows of at most 112
+// strings leave most of a row CTA idle: 15 sites (2,7), 675,675 states, 38.7 / 45.7 and 22.3 / 27.4; 20 sites
+// (1,8) 149 / 573 and 89 / 302.  Between that and 128 strings: 16 sites (2,5), 524,160 states, 30.7 / 35.8 and
+// 16.3 / 20.2 with per-site U, level or less without; (2,8), 1.5 M states, 137 / 119 and 45 / 36.
 constexpr int64_t kFuseStates = 1 << 18;
-constexpr int64_t kFuseRow = 128;
+constexpr int64_t kFuseRow = 112, kFuseRowSmall = 128, kFuseRowStates = 1 << 20;
 
 // L2 budget of one x slab in the slab pass.  The part of L2 near an SM holds it only while it is small:
 // 4x4 FP32 (256 / 512 / 768 columns: 13 / 26 / 40 MB) 1,486 / 1,696 / 1,812 us the whole product, 16 sites
@@ -613,7 +629,9 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
         return ED_ERR_RANGE;
     }
     const size_t lists = (size_t)std::max(s->dn.max_row, 1) * sizeof(RowHop<T>);
-    if ((s->dim <= kFuseStates || s->nsup <= kFuseRow) && lists + (size_t)s->nsup * sizeof(T) <= (size_t)maxsm) {
+    const bool one_pass = s->dim <= kFuseStates || s->nsup <= kFuseRow ||
+                          (s->nsup <= kFuseRowSmall && s->dim <= kFuseRowStates);
+    if (one_pass && lists + (size_t)s->nsup * sizeof(T) <= (size_t)maxsm) {
         // the U_ijkl terms go into a cleared y first, so that the dots see the whole product
         const bool add = s->uijkl != nullptr;
         if (add) {
@@ -669,8 +687,14 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
                       ((reinterpret_cast<uintptr_t>(y) & 15) == 0);
     // chunks x rows in flight, measured (4x4 slab pass / 14 random bonds): FP32 2 x 2 1,012 us / 148 us the
     // whole product, 1 x 4 1,070 / 154, 4 x 2 1,790 / 250 (registers); FP64 4 x 2 5.37 ms / 742 us, 2 x 4 6.26 / 743
-    auto *kfn = !vec2 ? hub_slab_kernel<T, 1, 1, 4>
-                      : sizeof(T) == 4 ? hub_slab_kernel<T, VWS, 2, 2> : hub_slab_kernel<T, VWS, 4, 2>;
+    constexpr int U = sizeof(T) == 4 ? 2 : 4, kPass = 32 * VWS * U;
+    // A pass of U chunks is 256 columns.  Rows with a good part of their columns past the whole passes take
+    // those by single chunks: a column per lane there has one scalar load per hop and lane in flight (12 sites
+    // (4,6), 495 strings, FP32 15.6 -> 9.6 us; half filled, 924 strings, 13.9 -> 11.1).  Where that part is small
+    // (below a sixteenth) the two kernels are level.
+    const bool single = s->nsup % kPass >= 32 && 16 * (s->nsup % kPass) >= s->nsup;
+    auto *kfn = !vec2 ? hub_slab_kernel<T, 1, 1, 4, false>
+                      : single ? hub_slab_kernel<T, VWS, U, 2, true> : hub_slab_kernel<T, VWS, U, 2, false>;
     // one wave of resident CTAs: each walks its share of the items, so a grid past the
     // resident count would leave a second, partial wave running whole shares
     int per_sm = 0;
