@@ -667,8 +667,11 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
         auto *kfn = two ? hub_row_kernel<T, 2, false> : hub_row_kernel<T, 1, false>;
         if (sizeof(T) == 4 && a.ell_sg32) kfn = two ? hub_row_kernel<T, 2, sizeof(T) == 4> : hub_row_kernel<T, 1, sizeof(T) == 4>;
         ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const int64_t blocks = std::min<int64_t>((s->nsdn + R - 1) / R, (int64_t)nsm * 2);
-        kfn<<<(unsigned)blocks, threads, smem, st>>>(x, y, a, sld, vec_ok ? 1 : 0);
+        // a warp per slice of short rows, and more CTAs: idle warps hold an SM's threads (18 sites (2,7), 5
+        // slices, FP64 256 -> 199 us)
+        const int nt = (int)std::min<int64_t>(threads, std::max<int64_t>(64, s->up.nslice * 32));
+        const int64_t blocks = std::min<int64_t>((s->nsdn + R - 1) / R, (int64_t)nsm * (1024 / nt));
+        kfn<<<(unsigned)blocks, nt, smem, st>>>(x, y, a, sld, vec_ok ? 1 : 0);
     }
     ED_CHECK_LAUNCH();
     // ---- the U_ijkl terms, if any (before pass 2, whose fused dots need the whole product)
