@@ -35,7 +35,7 @@ struct HubArgs {
     float mag32[2];
     const void *u_lut;        // [4][256], then U times a count; float or double like the vectors
     int nbytes;               // bytes of a string with an on-site interaction (1 when there is none: zeros)
-    int u_uniform;
+    int u_uniform, u_few;     // few: min(nup, ndn) < nbytes
     double u_value;
     double scale;
 };
@@ -50,14 +50,28 @@ __device__ __forceinline__ T u_table(const HubArgs &a, uint32_t both)
     return e;
 }
 
-// the same; uval = U in T (uniform U, where a count is cheaper in FP32)
+// the same site by site
 template <typename T>
+__device__ __forceinline__ T u_by_site(const HubArgs &a, uint32_t both)
+{
+    const T *lut = static_cast<const T *>(a.u_lut);
+    auto site = [&](int b) { return __ldg(lut + (b >> 3) * 256 + (1 << (b & 7))); };
+    if (!both) return (T)0;
+    T e = site(__ffs(both) - 1);
+    for (both &= both - 1; both; both &= both - 1) e += site(__ffs(both) - 1);
+    return e;
+}
+
+// the same; uval = U in T (uniform U, where a count is cheaper in FP32).  FEW: with fewer doubly occupied sites
+// than bytes (u_few) a lane's sites cost the FP64 pipe less than the bytes (20 sites (2,6) 328 -> 294 us).
+template <typename T, bool FEW = false>
 __device__ __forceinline__ T u_energy(const HubArgs &a, uint32_t both, T uval)
 {
     if (a.u_uniform) {
         if constexpr (sizeof(T) == 4) return uval * (T)__popc(both);
         return __ldg(static_cast<const T *>(a.u_lut) + 4 * 256 + __popc(both));   // no FP64 operation
     }
+    if (FEW && a.u_few) return u_by_site<T>(a, both);
     return u_table<T>(a, both);
 }
 
@@ -140,7 +154,7 @@ __global__ void __launch_bounds__(512, 2) hub_row_kernel(const T *__restrict__ x
             const T eu = __ldg(ued_t + uu);
             T acc[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) acc[r] = (eu + ed[r] + u_energy<T>(a, su & sd[r], uval)) * xs[r * sld + uu];
+            for (int r = 0; r < R; ++r) acc[r] = (eu + ed[r] + u_energy<T, sizeof(T) == 8>(a, su & sd[r], uval)) * xs[r * sld + uu];
             const int s0 = __ldg(a.ell_off + sl), ns = __ldg(a.ell_off + sl + 1) - s0;
             const int64_t at0 = (int64_t)s0 * 32 + lane;
             // slots in groups: all table loads of a group are in flight before its first gather
@@ -614,6 +628,7 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     a.u_lut = (sizeof(T) == 4) ? (const void *)s->u_lut32 : (const void *)s->u_lut;
     a.nbytes = (s->u_uniform && s->u_value == 0.0) ? 1 : (s->norb + 7) / 8;
     a.u_uniform = s->u_uniform ? 1 : 0;
+    a.u_few = std::min(s->nup, s->ndn) < a.nbytes ? 1 : 0;
     a.u_value = s->u_value;
     a.scale = scale;
     const int nsm = num_sms();
