@@ -548,8 +548,8 @@ static constexpr int kMaxPartialBlocks = 1024;
 // instead of two), 11 sites half filled (213,444) FP64 22.5 / 26.7, FP32 11.9 / 18.5; 16 sites (3,3)
 // (313,600) 28.7 / 26.7 and 16.4 / 13.9, 3x4 half filled 101 / 81 and 48 / 23.  Rows of at most 112
 // strings leave most of a row CTA idle: 15 sites (2,7), 675,675 states, 38.7 / 45.7 and 22.3 / 27.4; 20 sites
-// (1,8) 149 / 573 and 89 / 302.  Between that and 128 strings: 16 sites (2,5), 524,160 states, 30.7 / 35.8 and
-// 16.3 / 20.2 with per-site U, level or less without; (2,8), 1.5 M states, 137 / 119 and 45 / 36.
+// (1,8) 149 / 573 and 89 / 302.  Between that and 128 strings only FP32: 16 sites (2,5), 524,160 states, with
+// per-site U 30.6 / 27.5 and 16.2 / 20.2, without 29.2 / 26.3 and 15.5 / 15.8; (2,8), 1.5 M states, 82 / 67 and 45 / 36.
 constexpr int64_t kFuseStates = 1 << 18;
 constexpr int64_t kFuseRow = 112, kFuseRowSmall = 128, kFuseRowStates = 1 << 20;
 
@@ -645,7 +645,7 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
     }
     const size_t lists = (size_t)std::max(s->dn.max_row, 1) * sizeof(RowHop<T>);
     const bool one_pass = s->dim <= kFuseStates || s->nsup <= kFuseRow ||
-                          (s->nsup <= kFuseRowSmall && s->dim <= kFuseRowStates);
+                          (sizeof(T) == 4 && s->nsup <= kFuseRowSmall && s->dim <= kFuseRowStates);
     if (one_pass && lists + (size_t)s->nsup * sizeof(T) <= (size_t)maxsm) {
         // the U_ijkl terms go into a cleared y first, so that the dots see the whole product
         const bool add = s->uijkl != nullptr;
