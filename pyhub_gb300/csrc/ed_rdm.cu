@@ -198,9 +198,10 @@ template <typename T, int R> __device__ __forceinline__ void load_rows(const T *
 // one row at a time -> 570 us (floor 458).
 constexpr int kUphopThreads = 512;
 
-template <typename T, int R>
+template <typename T, int R, bool PARTS>
 __global__ void __launch_bounds__(kUphopThreads) rdm_uphop_kernel(const T *__restrict__ bra, const T *__restrict__ ket,
-                                                                  const RdmArgs a, double *__restrict__ partials)
+                                                                  const RdmArgs a, int parts,
+                                                                  double *__restrict__ partials)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *acc = reinterpret_cast<double *>(smem_raw);          // [npairs], padded to 16 bytes
@@ -208,7 +209,9 @@ __global__ void __launch_bounds__(kUphopThreads) rdm_uphop_kernel(const T *__res
     double accW[NQ];                                              // row sums of pairs threadIdx.x, + kUphopThreads
 #pragma unroll
     for (int i = 0; i < NQ; ++i) accW[i] = 0.0;
-    __shared__ double W[R];
+    constexpr int kWarps = kUphopThreads / 32;
+    const int seg = PARTS ? parts : 1;
+    __shared__ double W[R][PARTS ? kWarps / R : 1];               // row sums, of seg parts each at first
     T *bs = reinterpret_cast<T *>(acc + (a.npairs + 1) / 2 * 2);  // [nsup][R]
     const bool same = (bra == ket);
     T *ks = same ? bs : bs + (int64_t)a.nsup * R;
@@ -226,15 +229,18 @@ __global__ void __launch_bounds__(kUphopThreads) rdm_uphop_kernel(const T *__res
             }
         }
         __syncthreads();
-        for (int task = warp; task < a.npairs + R; task += kUphopThreads / 32) {
-            if (task < R) {
+        for (int task = warp; task < a.npairs + R * seg; task += kWarps) {
+            if (task < R * seg) {
+                const int r = task / seg, part = task - r * seg;
+                const int i1 = (int)((int64_t)nsup * (part + 1) / seg);
                 double w = 0.0;
-                for (int i = lane; i < nsup; i += 32) w = fma((double)bs[i * R + task], (double)ks[i * R + task], w);
+                for (int i = (int)((int64_t)nsup * part / seg) + lane; i < i1; i += 32)
+                    w = fma((double)bs[i * R + r], (double)ks[i * R + r], w);
                 w = warp_sum(w);
-                if (lane == 0) W[task] = w;
+                if (lane == 0) W[r][part] = w;
                 continue;
             }
-            const int q = task - R;
+            const int q = task - R * seg;
             const int J = a.pj[q], K = a.pk[q];
             if (J == K) continue;
             const int pid = (J - 1) * a.norb + (K - 1);
@@ -253,6 +259,14 @@ __global__ void __launch_bounds__(kUphopThreads) rdm_uphop_kernel(const T *__res
             if (lane == 0) acc[q] += s;
         }
         __syncthreads();
+        if (PARTS) {
+            if (threadIdx.x < R) {
+                double w = W[threadIdx.x][0];
+                for (int part = 1; part < seg; ++part) w += W[threadIdx.x][part];
+                W[threadIdx.x][0] = w;
+            }
+            __syncthreads();
+        }
 #pragma unroll
         for (int i = 0; i < NQ; ++i) {
             const int q = threadIdx.x + i * kUphopThreads;
@@ -260,7 +274,7 @@ __global__ void __launch_bounds__(kUphopThreads) rdm_uphop_kernel(const T *__res
             const uint32_t both = bit_of(a.norb, a.pj[q]) | bit_of(a.norb, a.pk[q]);
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                if (d0 + r < a.nsdn && (__ldg(a.dstr + d0 + r) & both) == both) accW[i] += W[r];
+                if (d0 + r < a.nsdn && (__ldg(a.dstr + d0 + r) & both) == both) accW[i] += W[r][0];
         }
     }
     __syncthreads();
@@ -281,9 +295,14 @@ static int launch_uphop(cudaStream_t st, const T *bra, const T *ket, const RdmAr
                         int *rows)
 {
     const size_t smem = (size_t)(a.npairs + 1) / 2 * 16 + (size_t)(bra == ket ? 1 : 2) * R * a.nsup * sizeof(T);
-    ED_CHECK_CUDA(cudaFuncSetAttribute(rdm_uphop_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     *rows = (int)std::min<int64_t>((a.nsdn + R - 1) / R, std::min(4 * nsm, maxblk));
-    rdm_uphop_kernel<T, R><<<*rows, kUphopThreads, smem, st>>>(bra, ket, a, part);
+    // A row's sum is a warp's task beside the pairs', whose lists hold about a quarter of the row for each of R
+    // rows: with one or two rows it outlasts them and is cut into parts of 512 strings or more (18 sites (9,1),
+    // FP32, one pair: 287 -> 174 us; 16 sites (8,0), bonds: 130 -> 96; with four rows it makes no difference)
+    const int seg = R == 4 ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(kUphopThreads / 32 / R, a.nsup / 512));
+    auto *kfn = seg > 1 ? rdm_uphop_kernel<T, R, R != 4> : rdm_uphop_kernel<T, R, false>;
+    ED_CHECK_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kfn<<<*rows, kUphopThreads, smem, st>>>(bra, ket, a, seg, part);
     ED_CHECK_LAUNCH();
     return ED_OK;
 }
