@@ -170,7 +170,7 @@ int heis_struct_build(ed_sector *s)
         // 4x7 3.41 -> 3.19 ms the whole product).  Vectors far above L2 pay for the scattering in DRAM
         // sectors (5x6, 1.2 GB: 14.9 -> 22.9 ms; 4x8 56 -> 78): windows of 64 there (14.9, 55.7 ms)
         const int64_t window = (double)s->dim * sizeof(double) <= kL2Bytes ? n : 64;
-        for (int64_t r = 0; r < n; r += window)
+        for (int64_t r = 0; n > 32 && r < n; r += window)      // one slice: in order (the kernel relies on it)
             std::stable_sort(order.begin() + r, order.begin() + std::min(n, r + window), [&](int32_t x, int32_t y) {
                 return lists[(size_t)x].size() > lists[(size_t)y].size();
             });
@@ -422,8 +422,10 @@ __global__ void __launch_bounds__(kHeisRowThreads, 4) heis_row_kernel(const T *_
         __syncthreads();
         const int nsl = (len + 31) / 32;
         for (int sl = warp; sl < nsl; sl += nwarps) {
-            const int c = sizeof(T) == 4 ? sl * 32 + lane : __ldg(a.aa64_col + (sbase + sl) * 32 + lane);
-            const bool ok = sizeof(T) == 4 ? c < len : c >= 0;
+            // (a class of one slice is in order, and the look-up would lead a short row's chain of loads)
+            const bool plain = sizeof(T) == 4 || len <= 32;
+            const int c = plain ? sl * 32 + lane : __ldg(a.aa64_col + (sbase + sl) * 32 + lane);
+            const bool ok = plain ? c < len : c >= 0;
             const int cc = ok ? c : len - 1;
             const uint32_t ha = __ldg(a.col_pat + cbase + cc);
             T d = __ldg(static_cast<const T *>(a.diagA) + cbase + cc) + db;
