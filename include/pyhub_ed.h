@@ -98,6 +98,8 @@ int64_t ed_scratch_bytes(int64_t n, int nvec);
 int ed_hv(ed_sector *s, void *stream, int dtype, int64_t ld,
           const void *x, void *y, double scale,
           double *dots, void *scratch, int64_t scratch_bytes);
+/* Kernels that ed_hv without dots launches for the sector (-1: bad argument). */
+int ed_hv_launches(const ed_sector *s, int dtype);
 
 /* out[j] = <V_j, w> and, if z != NULL, out[nvec + j] = <V_j, z>, j < nvec.
  * V_j = V + j*ldv elements.  FP64 results (device pointer).  The dot

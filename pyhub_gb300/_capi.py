@@ -28,6 +28,7 @@ _SIGS = {
     "ed_rank": (_I64, [_I, _I, ctypes.c_uint32]),
     "ed_sector_create": (_I, [_I, _I, _I, _I, _P, _P, _P, ctypes.POINTER(_P)]),
     "ed_sector_destroy": (_I, [_P]),
+    "ed_hv_launches": (_I, [_P, _I]),
     "ed_lanczos_step_scratch_bytes": (_I64, [_P, _I]),
     "ed_lanczos_step": (_I, [_P, _P, _I, _I64, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _I64]),
     "ed_lanczos_steps": (_I, [_P, _P, _I, _I64, _P, _I64, _I, _I, _I, _P, _P, _P, _P, _P, _I64]),
@@ -388,6 +389,10 @@ class Sector:
         check("ed_hv", lib().ed_hv(self._h, _stream(stream), dtype_code(x.dtype), int(ld), _ptr(x, need, "x"),
                                    _ptr(y, need, "y"), float(scale), _ptr(dots, 2, "dots"), _ptr(scratch),
                                    int(sb)))
+
+    def hv_launches(self, dtype) -> int:
+        """Kernels that hv without dots launches."""
+        return int(lib().ed_hv_launches(self._h, dtype_code(dtype)))
 
     def _need(self, ld: int) -> int:
         """Elements a vector with row stride ld must hold."""

@@ -181,15 +181,17 @@ class KernelTimer:
     algorithmic bytes and kernel launches per call; read after a
     synchronize."""
 
-    # a product of two passes without dots; sums of partial rows beside multi-dot, update and Ritz sum
+    # where a call does not say: a product of two passes without dots (Sector.hv_launches knows the sector's);
+    # sums of partial rows beside multi-dot, update and Ritz sum
     LAUNCHES = {"hv": 2, "multidot": 2, "coef": 1, "update": 2, "ritz": 2}
 
     def __init__(self):
         self.ev = {}
         self.bytes = {}
         self.calls = {}
+        self.kernels = {}
 
-    def __call__(self, kind: str, nbytes: float):
+    def __call__(self, kind: str, nbytes: float, kernels: int = None):
         torch = _torch()
         a = torch.cuda.Event(enable_timing=True)
         b = torch.cuda.Event(enable_timing=True)
@@ -197,6 +199,7 @@ class KernelTimer:
         self.ev.setdefault(kind, []).append((a, b))
         self.bytes[kind] = self.bytes.get(kind, 0.0) + float(nbytes)
         self.calls[kind] = self.calls.get(kind, 0) + 1
+        self.kernels[kind] = self.kernels.get(kind, 0) + (self.LAUNCHES.get(kind, 1) if kernels is None else kernels)
         return b
 
     def summary(self):
@@ -204,11 +207,11 @@ class KernelTimer:
         for k, lst in self.ev.items():
             t = sum(a.elapsed_time(b) for a, b in lst) * 1e-3
             out[k] = {"calls": self.calls[k], "seconds": t, "bytes": self.bytes[k],
-                      "launches": self.calls[k] * self.LAUNCHES.get(k, 1)}
+                      "launches": self.kernels[k]}
         return out
 
     def launches(self):
-        return sum(self.calls[k] * self.LAUNCHES.get(k, 1) for k in self.calls)
+        return sum(self.kernels.values())
 
 
 class _Scratch:
@@ -304,6 +307,7 @@ def lanczos_full(sec, v0, max_steps: int, dtype=None, rule=None, check_every: in
             return rule(val, k, vec=vecs_t, beta_last=beta[k - 1])
         return rule(_tridiag_eigs(alpha, beta, k), k)
 
+    hv_kernels = sec.hv_launches(dtype) if timer is not None and hasattr(sec, "hv_launches") else None
     if lookahead is None:
         lookahead = check_every >= 3
     pending = None
@@ -341,7 +345,7 @@ def lanczos_full(sec, v0, max_steps: int, dtype=None, rule=None, check_every: in
                 converged = stop == 0
                 break
     for k in range(k_done, m if not native else k_done):
-        e = timer("hv", 2.0 * sec.dim * es) if timer is not None else None
+        e = timer("hv", 2.0 * sec.dim * es, hv_kernels) if timer is not None else None
         sec.hv(V[k], w)
         if e is not None:
             e.record()

@@ -604,6 +604,19 @@ static int launch_fused(ed_sector *s, cudaStream_t st, const T *x, T *y, HubArgs
     return ED_OK;
 }
 
+// Bytes of a row's down hops in the one-pass kernel, and whether the sector takes it.
+template <typename T> static size_t list_bytes(const ed_sector *s)
+{
+    return (size_t)std::max(s->dn.max_row, 1) * sizeof(RowHop<T>);
+}
+
+template <typename T> static bool one_pass(const ed_sector *s)
+{
+    const bool small = s->dim <= kFuseStates || s->nsup <= kFuseRow ||
+                       (sizeof(T) == 4 && s->nsup <= kFuseRowSmall && s->dim <= kFuseRowStates);
+    return small && list_bytes<T>(s) + (size_t)s->nsup * sizeof(T) <= (size_t)max_smem();
+}
+
 template <typename T>
 static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, double scale, double *dots,
                   double *partials)
@@ -643,10 +656,8 @@ static int hub_hv(ed_sector *s, cudaStream_t st, int64_t ld, const T *x, T *y, d
                   (long long)s->nsup, maxsm);
         return ED_ERR_RANGE;
     }
-    const size_t lists = (size_t)std::max(s->dn.max_row, 1) * sizeof(RowHop<T>);
-    const bool one_pass = s->dim <= kFuseStates || s->nsup <= kFuseRow ||
-                          (sizeof(T) == 4 && s->nsup <= kFuseRowSmall && s->dim <= kFuseRowStates);
-    if (one_pass && lists + (size_t)s->nsup * sizeof(T) <= (size_t)maxsm) {
+    const size_t lists = list_bytes<T>(s);
+    if (one_pass<T>(s)) {
         // the U_ijkl terms go into a cleared y first, so that the dots see the whole product
         const bool add = s->uijkl != nullptr;
         if (add) {
@@ -744,6 +755,15 @@ extern "C" int64_t ed_scratch_bytes(int64_t n, int nvec)
     (void)n;
     if (nvec < 1) nvec = 1;
     return (int64_t)kMaxPartialBlocks * 2 * nvec * (int64_t)sizeof(double) + 4096;
+}
+
+extern "C" int ed_hv_launches(const ed_sector *s, int dtype)
+{
+    if (!s || (dtype != ED_F32 && dtype != ED_F64)) return -1;
+    if (s->dim == 0) return 0;
+    if (s->kind != ED_HUBBARD) return 2;
+    const bool one = dtype == ED_F32 ? one_pass<float>(s) : one_pass<double>(s);
+    return (one ? 1 : 2) + (s->uijkl ? 1 : 0);
 }
 
 extern "C" int ed_hv(ed_sector *s, void *stream, int dtype, int64_t ld, const void *x, void *y, double scale,
