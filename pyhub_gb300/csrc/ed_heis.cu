@@ -71,7 +71,9 @@ int up(T **dst, const std::vector<T> &v)
 
 }  // namespace
 
-// Vectors up to this many bytes mostly meet L2 again where neighbouring rows are read out of order.
+// Vectors up to this many bytes take orders that scatter reads and writes (FP64 columns by number of flips,
+// rows by length): above it the scattered sectors come from DRAM more than once.  Several times the L2 (129 MB);
+// the line lies between measured sizes: 29 sites (620 MB) 6.47 ms sorted, 6.67 in order; 30 (1.24 GB) 20.4, 14.0.
 constexpr double kL2Bytes = 1.0e9;
 
 int heis_struct_build(ed_sector *s)
@@ -842,9 +844,10 @@ struct HsRdmArgs {
 
 constexpr int kRdmThreads = 256;
 // Sectors of this many states take five CTAs per SM instead of three: the flips wait for loads most of the
-// time and more warps cover them, at the price of spilled registers, most of them in the diagonal tiles
-// (22 sites, 705,432 states: 331 -> 297 us, 24: 775 -> 690, 28: 11.6 -> 10.0 ms; 20 sites, 184,756: 205 -> 217).
-constexpr int64_t kRdmLarge = 1 << 19;
+// time and more warps cover them, at the price of spilled registers, most of them in the diagonal tiles (all
+// pairs, FP64, three and five: 20 sites, 184,756 states, 149 and 161 us; 21, 352,716, 219 and 200; 22 272 and 240;
+// 24 709 and 627; FP32 168 and 174, 260 and 251, 343 and 330, 1,047 and 1,049).
+constexpr int64_t kRdmLarge = 1 << 18;
 
 __device__ __forceinline__ uint32_t insert_bit(uint32_t h, int pos, uint32_t bit)
 {
@@ -1303,10 +1306,11 @@ static int heis_struct_run(ed_sector *s, cudaStream_t st, const T *x, T *y, doub
     for (int m = 0; m <= h.nA; ++m) a.m_order[m] = (int8_t)m;
     std::sort(a.m_order, a.m_order + h.nA + 1, [&](int8_t x, int8_t y) { return h.ncol[x] > h.ncol[y]; });
     const int nsm = num_sms();
-    // rows by length give the CTAs even shares (FP64: 4x6 157 -> 149 us, 4x7 3.69 -> 3.51 ms); vectors far
-    // above L2 keep memory order, where the A-B bonds' source rows are near (4x8: 60 ms, by length 67), and
-    // so do rows that have a CTA each (4x4: the row pass 5.5 us, by length 6.6: the look-up leads the chain
-    // of loads)
+    // rows by length give the CTAs even shares (FP64: 4x6 157 -> 149 us, 4x7 3.69 -> 3.51 ms; FP32 here only
+    // with more than 32 A-B bonds: all couplings, 24 sites 570 -> 541 us, 26 2.40 -> 2.30 ms, but 22 148 -> 163);
+    // vectors far above L2 keep memory order, where the A-B bonds' source rows are near (4x8: 60 ms, by length
+    // 67; on a ring with next-but-three neighbours the two are level: 30 sites 14.6 and 14.0), and so do rows
+    // that have a CTA each (4x4: the row pass 5.5 us, by length 6.6: the look-up leads the chain of loads)
     a.by_length = (double)s->dim * sizeof(T) <= kL2Bytes && h.nrows > (int64_t)nsm * 4 ? 1 : 0;
     // ---- pass R
     const int maxsm = max_smem();

@@ -555,8 +555,9 @@ constexpr int64_t kFuseRow = 112, kFuseRowSmall = 128, kFuseRowStates = 1 << 20;
 
 // L2 budget of one x slab in the slab pass.  The part of L2 near an SM holds it only while it is small:
 // 4x4 FP32 (256 / 512 / 768 columns: 13 / 26 / 40 MB) 1,486 / 1,696 / 1,812 us the whole product, 16 sites
-// (7,7) 12 / 23 / 47 MB 1,170 / 1,198 / 1,418 us; FP64, bound by its pipe, is the same over that range.  The
-// environment variable PYHUB_ED_SLAB_L2_BYTES overrides it for tuning.
+// (7,7) 12 / 23 / 47 MB 1,170 / 1,198 / 1,418 us.  FP64 is bound by its pipe: at budgets of 20 and 48 MB 14 sites
+// and 4x4 are level, 15 sites (7,7) 2,485 and 2,538 us, 16 sites (7,7) 9,271 and 9,170.  The environment variable
+// PYHUB_ED_SLAB_L2_BYTES overrides it for tuning.
 static double slab_l2_bytes()
 {
     static double v = []() {

@@ -36,8 +36,8 @@ struct RdmArgs {
     int norb;
     int64_t nsup, nsdn, ld;
     const uint32_t *ustr, *dstr, *lut;
-    const int32_t *upl_off, *dpl_off;   // pair lists of the up and down strings
-    const int2 *upl_ent, *dpl_ent;
+    const int32_t *upl_off;             // pair lists of the up strings
+    const int2 *upl_ent;
     int npairs;
     int8_t pj[kMaxPairs], pk[kMaxPairs];
 };
@@ -375,7 +375,6 @@ static int rdm_hub(ed_sector *s, cudaStream_t st, int64_t ld, const T *bra, cons
     a.nsup = s->nsup; a.nsdn = s->nsdn; a.ld = ld;
     a.ustr = s->up.str; a.dstr = s->dn.str; a.lut = s->lut;
     a.upl_off = s->up.pl_off; a.upl_ent = s->up.pl_ent;
-    a.dpl_off = s->dn.pl_off; a.dpl_ent = s->dn.pl_ent;
     a.npairs = npairs;
     for (int p = 0; p < npairs; ++p) { a.pj[p] = (int8_t)pairs[2 * p]; a.pk[p] = (int8_t)pairs[2 * p + 1]; }
     int dev = 0, maxsm = 0, nsm = 1;
