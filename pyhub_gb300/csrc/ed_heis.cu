@@ -846,8 +846,9 @@ constexpr int kRdmThreads = 256;
 // Sectors of this many states take five CTAs per SM instead of three: the flips wait for loads most of the
 // time and more warps cover them, at the price of spilled registers, most of them in the diagonal tiles (all
 // pairs, FP64, three and five: 20 sites, 184,756 states, 149 and 161 us; 21, 352,716, 219 and 200; 22 272 and 240;
-// 24 709 and 627; FP32 168 and 174, 260 and 251, 343 and 330, 1,047 and 1,049).
-constexpr int64_t kRdmLarge = 1 << 18;
+// 24 709 and 627; FP32 168 and 174, 260 and 251, 343 and 330, 1,047 and 1,049; but the 21 bonds of a 21-site ring
+// 173 and 185, so that sector keeps three).
+constexpr int64_t kRdmLarge = 1 << 19;
 
 __device__ __forceinline__ uint32_t insert_bit(uint32_t h, int pos, uint32_t bit)
 {
