@@ -107,13 +107,14 @@ __global__ void __launch_bounds__(kVecThreads, kVecResident) multidot32_kernel(i
 }
 
 // FP64, same partials.  An FP64 instruction costs 64 FP32 ones on this chip, so the pass is bound by
-// the FP64 pipe (two FMA per basis element) and spends it on nothing else: a CTA owns up to KJ vectors
-// and one range of elements, every thread keeps its 2*KJ sums in registers over the whole range,
+// the FP64 pipe (two FMA per basis element) and spends it on nothing else: a CTA owns up to kJ64 vectors
+// and one range of elements, every thread keeps its 2*kJ64 sums in registers over the whole range,
 // and lanes are summed once at its end (the pass that summed lanes after every 16 elements took 11
-// FP64 instructions per 8 here).  w and z are read again for every KJ = kJ64 vectors, from L2.
-// With few vectors (KJ < kJ64) the loads are the time: U steps of all vectors are in flight together
-// (one vector of 1.7e8: 778 us with kJ64 and one step, 375 so; of 300,000: 9.5 -> 4.9), and one wave of
-// CTAs has less to start and to sum (seven of 500,000 and z: 29.5 -> 23.6 us).
+// FP64 instructions per 8 here).  w and z are read again for every kJ64 vectors, from L2.
+// NV = 0: groups of up to kJ64 vectors.  NV of 1 to 4: all nvec = NV vectors, where the loads are the time:
+// U steps of all of them are in flight together (one vector of 1.7e8: 778 us as a group, 375 so; of
+// 300,000: 9.5 -> 4.9).  One wave of CTAs has less to start and to sum than two (seven of 500,000 and z:
+// 29.5 -> 23.6 us).
 static constexpr int kJ64 = 8;
 static constexpr int kStep64 = kVecThreads * 2;   // elements of one iteration: a 16-byte load per thread
 
@@ -145,20 +146,22 @@ __device__ __forceinline__ void warp_sum_many(double (&v)[N])
 }
 
 // CTAs of a variant that an SM holds (registers)
-template <int KJ, int U> constexpr int multidot64_ctas() { return KJ == 1 && U == 4 ? 4 : KJ == 2 ? 3 : 2; }
+template <int NV> constexpr int multidot64_ctas() { return NV == 1 ? 4 : NV ? 3 : 2; }
 
-template <bool Z, int KJ, int U>
-__global__ void __launch_bounds__(kVecThreads, multidot64_ctas<KJ, U>()) multidot64_kernel(int64_t n, const double *__restrict__ V,
-                                                                    int64_t ldv, int nvec,
+template <bool Z, int NV, int U>
+__global__ void __launch_bounds__(kVecThreads, multidot64_ctas<NV>()) multidot64_kernel(int64_t n,
+                                                                    const double *__restrict__ V, int64_t ldv, int nvec,
                                                                     const double *__restrict__ w,
                                                                     const double *__restrict__ z,
                                                                     double *__restrict__ partials)
 {
+    constexpr int M = NV ? NV : kJ64, KJ = M == 3 ? 4 : M;      // vectors, and their sums (a power of two)
     constexpr int NS = Z ? 2 * KJ : KJ;
     __shared__ double red[kVecThreads / 32][NS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ng = gridDim.y;
-    const int j0 = (int)((int64_t)nvec * blockIdx.y / ng), nj = (int)((int64_t)nvec * (blockIdx.y + 1) / ng) - j0;
+    const int j0 = NV ? 0 : (int)((int64_t)nvec * blockIdx.y / ng);
+    const int nj = NV ? NV : (int)((int64_t)nvec * (blockIdx.y + 1) / ng) - j0;
     const int64_t steps = (n + U * kStep64 - 1) / (U * kStep64);
     const int64_t s0 = steps * blockIdx.x / gridDim.x, s1 = steps * (blockIdx.x + 1) / gridDim.x;
     double acc[NS];
@@ -167,11 +170,11 @@ __global__ void __launch_bounds__(kVecThreads, multidot64_ctas<KJ, U>()) multido
     const double *Vj = V + (int64_t)j0 * ldv;
     for (int64_t st = s0; st < s1; ++st) {
         const int64_t i = st * (U * kStep64) + threadIdx.x * 2;
-        double2 v[U][KJ], a[U], b[U];
+        double2 v[U][M], a[U], b[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
 #pragma unroll
-            for (int j = 0; j < KJ; ++j)
+            for (int j = 0; j < M; ++j)
                 if (j < nj) v[u][j] = load2(Vj + (int64_t)j * ldv, i + u * kStep64, n);
             a[u] = load2(w, i + u * kStep64, n);
             if constexpr (Z) b[u] = load2(z, i + u * kStep64, n);
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(kVecThreads, multidot64_ctas<KJ, U>()) multido
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int j = 0; j < KJ; ++j) {
+            for (int j = 0; j < M; ++j) {
                 if (j >= nj) break;
                 acc[j] = fma(v[u][j].x, a[u].x, acc[j]);
                 if constexpr (Z) acc[KJ + j] = fma(v[u][j].x, b[u].x, acc[KJ + j]);
@@ -362,28 +365,33 @@ int launch_multidot(cudaStream_t st, int dtype, int64_t n, const void *V, int64_
         int ng = 1, gx = 0;
         // one group: a wave of resident CTAs; several groups, of unequal sizes: two.  One CTA more than
         // whole waves costs a wave
-        auto launch = [&](auto kj, auto un) {
-            constexpr int KJ = decltype(kj)::value, U = decltype(un)::value;
+        auto launch = [&](auto count, auto un) {
+            constexpr int NV = decltype(count)::value, U = decltype(un)::value;
             const int64_t steps = (n + U * kStep64 - 1) / (U * kStep64);
-            const int64_t fill = ng == 1 ? (int64_t)num_sms() * multidot64_ctas<KJ, U>() : ctas;
+            const int64_t fill = ng == 1 ? (int64_t)num_sms() * multidot64_ctas<NV>() : ctas;
             gx = (int)std::max<int64_t>(1, std::min(steps, std::min(fill, ctas) / ng));
             const dim3 grid((unsigned)gx, (unsigned)ng);
-            if (z) multidot64_kernel<true, KJ, U><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
-            else multidot64_kernel<false, KJ, U><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
+            if (z) multidot64_kernel<true, NV, U><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
+            else multidot64_kernel<false, NV, U><<<grid, kVecThreads, 0, st>>>(n, Vd, ldv, nvec, wd, zd, part);
         };
         using std::integral_constant;
-        if (nvec == 1) {
+        // up to a step per SM there is nothing to keep in flight (4,928 elements, two vectors and z: 5.5 us, with
+        // four steps 6.5)
+        const int few = nvec <= 4 && n > (int64_t)kStep64 * num_sms() ? nvec : 0;
+        if (few == 1) {
             launch(integral_constant<int, 1>(), integral_constant<int, 4>());
-        } else if (nvec == 2) {
+        } else if (few == 2) {
             launch(integral_constant<int, 2>(), integral_constant<int, 4>());
-        } else if (nvec <= 4) {
+        } else if (few == 3) {
+            launch(integral_constant<int, 3>(), integral_constant<int, 2>());
+        } else if (few == 4) {
             launch(integral_constant<int, 4>(), integral_constant<int, 2>());
         } else {
             // groups of 5 to kJ64 vectors, as even as they come: the CTAs with the largest group end the pass
             ng = (nvec + kJ64 - 1) / kJ64;
             for (int g = ng + 1; g <= (nvec + 4) / 5; ++g)
                 if ((int64_t)((nvec + g - 1) / g) * g < (int64_t)((nvec + ng - 1) / ng) * ng) ng = g;
-            launch(integral_constant<int, kJ64>(), integral_constant<int, 1>());
+            launch(integral_constant<int, 0>(), integral_constant<int, 1>());
         }
         *rows = gx;
     }
@@ -398,18 +406,24 @@ static int launch_update(cudaStream_t st, int64_t n, const T *V, int64_t ldv, in
     const int64_t ctas = vec_ctas();
     const size_t smem = sizeof(double) * (size_t)(nvec > 0 ? nvec : 1);
     const int64_t tiles = (n + kSplitTile - 1) / kSplitTile;
-    // The split form takes short vectors (up to four tiles per CTA), where a warp has vectors enough to pay
-    // for the exchange; more of them the more tiles share the loads: 16,000 elements from 4 vectors on in
-    // both types, 63,488 FP32 10: 6.6 us against 7.5 for 4 x 128, FP64 24: 11.2 against 11.7; 300,000 FP32 50:
-    // 14.7 / 15.5, FP64 64: 49 / 52.  With fewer: 300,000 and one vector FP32 8.7 against 6.0, FP64 14.1 / 7.3.
-    // 4 x 128 takes the rest up to where 16-element chunks fill every resident CTA (FP64, bound by its
-    // pipe), or (FP32, bound by the streams) while its chunks have a CTA each and there are vectors enough
-    // to outlast the CTAs' start: 853,888 elements 32 vectors 24.4 us against 28.6, 12: 11.1 / 9.6;
-    // 1.5 M, 100 vectors 126 / 99.
-    const int64_t chunks = (n + kChunk - 1) / kChunk;
+    // The split form takes short vectors (up to four tiles per CTA) with vectors enough to pay for the exchange;
+    // where its many partial norms have to be summed as well, that pays later.  Without a norm,
+    // FP32: 63,488 elements, 7 vectors, 2.3 us against 3.3 for 4 x 128, 300,000 16 5.5 / 5.5; FP64: 20,000 2 2.7 /
+    // 2.8, 63,488 8 4.5 / 4.6, 300,000 50 38.1 / 38.8.  With, FP32: 63,488 12 6.6 / 6.5, 300,000 50 14.7 / 15.5; FP64:
+    // 63,488 24 10.8 / 11.4, 300,000 64 49 / 52; one vector of 300,000 8.7 / 6.0 and 14.1 / 7.3.
+    // 4 x 128 takes the rest up to where 16-element chunks fill every resident CTA (FP64, bound by its pipe;
+    // half of that for up to three vectors: one of 2.5 M 17 us, 16 x 256 14), or (FP32, bound by the streams)
+    // while its chunks have a CTA each: 853,888 elements, 7 vectors, 4.2 / 5.1, 1.1 M 100 119 / 82.  With a
+    // norm the fewer partial norms of 16 x 256 count: 853,888 12 11.1 / 9.6, 32 24.4 / 28.6.
+    // (The steps of one Lanczos run take one form, whoever sums the norms: their vectors are the same.)
+    const int64_t chunks = (n + kChunk - 1) / kChunk, ns = num_sms();
     constexpr bool f64 = sizeof(A) == 8;
-    const int64_t split_from = tiles <= 2 * num_sms() ? 4 : f64 ? std::min<int64_t>(64, tiles / 20) : tiles / 45;
-    const bool small = f64 ? chunks < ctas : (n + 511) / 512 <= kMaxNormRows && 9 * (int64_t)nvec >= chunks;
+    const bool norm = part != nullptr;
+    int64_t split_from;
+    if (norm) split_from = tiles <= 2 * ns ? 4 : f64 ? (tiles <= 4 * ns ? 24 : 64) : tiles / 45;
+    else split_from = f64 ? (tiles <= 2 * ns ? 2 : tiles <= 4 * ns ? 8 : 48) : (tiles <= 4 * ns ? 1 : tiles / 150);
+    const bool small = f64 ? chunks < (nvec > 3 ? ctas : ctas / 2)
+                           : (n + 511) / 512 <= kMaxNormRows && (!norm || 9 * (int64_t)nvec >= chunks);
     if (tiles <= 4 * ctas && nvec >= split_from) {
         *rows = (int)std::min(tiles, ctas);
         update_split_kernel<T, O, A><<<*rows, kVecThreads, 0, st>>>(n, V, ldv, nvec, coef, wscale, w, out, part);

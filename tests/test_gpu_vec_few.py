@@ -76,3 +76,22 @@ def test_update_forms(edlib, n, nvec, dt):
         got = float((out[:n].double() ** 2).sum())
         tol = 17 * uo + n * 2.0 ** -53 if od == torch.float32 else (n / 256 + 48) * 2.0 ** -53
         assert abs(float(nrm[0]) - got) <= 1.05 * tol * got
+
+
+@pytest.mark.parametrize("n,nvec", [(36, 1), (38_912, 1), (38_913, 2), (77_824, 7), (77_824, 8), (77_825, 1),
+                                    (131_072, 6), (131_072, 48), (200_000, 10), (311_296, 47), (311_297, 3),
+                                    (1_048_576, 3), (1_048_577, 3), (1_245_185, 3), (1_245_185, 4)])
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+def test_update_forms_without_a_norm(edlib, n, nvec, dt):
+    """The lines lie elsewhere where no norm is asked for; same bound per element."""
+    import torch
+    td = torch.float32 if dt == "f32" else torch.float64
+    u = 2.0 ** -24 if dt == "f32" else 2.0 ** -53
+    ld, V, w, z, g = _vectors(n, nvec, td, n - nvec)
+    coef = torch.randn(nvec, generator=g, dtype=torch.float64, device="cuda")
+    c = coef.to(td).double()
+    want, mag = w[:n].double() - c @ V[:, :n].double(), w[:n].double().abs() + c.abs() @ V[:, :n].double().abs()
+    out = torch.full((ld,), -7.0, dtype=td, device="cuda")
+    edlib.update(V, nvec, coef, w, out, n=n)
+    assert bool(((out[:n].double() - want).abs() <= 1.05 * (nvec + 5) * u * mag).all())
+    assert bool((out[n:] == -7.0).all())
