@@ -1,7 +1,7 @@
 """ed_multidot and ed_update with few vectors, where the number of vectors chooses
-the form: 1, 2, 3-4 and more vectors of the FP64 multi-dot at the edges of their
-steps (512 elements a step, 4 or 2 steps in flight), one group's grid where it
-strides, and the first count of a second group.
+the form: 1 to 4 and more vectors of the FP64 multi-dot at the edges of their
+steps (512 elements a step, 4 or 2 steps in flight past 77,824 elements), one
+group's grid where it strides, and the first count of a second group.
 
 Tolerances, from the order of summation (u = 2^-53): a thread's sum is at most
 n / 512 products long, then 8 lanes' and warps' additions and at most 1,024
@@ -24,7 +24,8 @@ def _vectors(n, nvec, td, seed):
     return ld, V, w, z, g
 
 
-@pytest.mark.parametrize("n", [1, 2, 511, 513, 1023, 1025, 2047, 2048, 2049, 4097, 311_297, 622_593, 1_245_185])
+@pytest.mark.parametrize("n", [1, 2, 511, 513, 1025, 2049, 77_824, 77_825, 79_871, 79_873, 80_897, 311_297, 622_593,
+                               1_245_185])
 @pytest.mark.parametrize("nvec", [1, 2, 3, 4, 5, 8, 9])
 def test_multidot_few_vectors(edlib, n, nvec):
     import torch
